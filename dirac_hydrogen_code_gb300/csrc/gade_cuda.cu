@@ -353,9 +353,12 @@ struct OpP {
     /* assembled operator (k_apply_asm): this step's coupling values
        A[pair][W][B] and the coupled block of every (block row, block) pair;
        a piece's order range is then a pair range */
-    const void *A;                 /* double, or float for the complex64 instance */
+    const void *A;                 /* fixed-point limbs (int2), or float for the complex64 instance */
+    const unsigned short *Ae;      /* [pair][Bp] biased exponent of a row's values (fixed point) */
     const int *pair_c;
-    size_t astride;                /* values per pulse of A */
+    size_t astride, aestride;      /* values per pulse of A and of Ae */
+    const int *pad, *off, *prow;   /* row positions of the fixed-point values (AsmLay) */
+    int Bp, npairs, RMA;           /* row positions; pairs; most row positions of one chunk (even) */
 };
 
 struct VecP {
@@ -387,27 +390,43 @@ __device__ __forceinline__ bool red_select(RedP &red, int pulse)
     return pred_ok(red.pred, red.pa ? red.pa : red.sc, red.pb ? red.pb : red.sc);
 }
 
-/* Block-wide deterministic sum of NV doubles; result valid in thread 0. */
-template <int NV>
-__device__ __forceinline__ void block_sum(double (&v)[NV], double *sh)
+/* Block-wide deterministic sum of NRED doubles per thread (a fixed tree for
+   a given block size); the result is valid in thread 0.  sh: 8 * NRED doubles
+   of scratch.  Within a warp the four values are split over the lanes first
+   (two exchanges, then one value per lane), so a warp spends 6 FP64 adds
+   instead of 20: on this GPU the adds of a plain tree over shared memory cost
+   more than its barriers (k_apply_asm: 7% of its FP64 pipe time). */
+__device__ __forceinline__ void block_sum(double (&v)[NRED], double *sh)
 {
-    const int tid = threadIdx.x, nt = blockDim.x;
-    for (int k = 0; k < NV; k++) sh[k * nt + tid] = v[k];
+    static_assert(NRED == 4, "the lane split below is for four values");
+    const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5, nw = (blockDim.x + 31) >> 5;
+    const unsigned all = 0xffffffffu;
+    /* lanes < 16 keep values 0, 1, the others 2, 3; then one value per 8 lanes */
+    const bool up = lane & 16, odd = lane & 8;
+    const double s0 = __shfl_xor_sync(all, up ? v[0] : v[2], 16), s1 = __shfl_xor_sync(all, up ? v[1] : v[3], 16);
+    const double a0 = (up ? v[2] : v[0]) + s0, a1 = (up ? v[3] : v[1]) + s1;
+    const double s2 = __shfl_xor_sync(all, odd ? a0 : a1, 8);
+    double w = (odd ? a1 : a0) + s2;                   /* value lane >> 3 */
+    w += __shfl_xor_sync(all, w, 4);
+    w += __shfl_xor_sync(all, w, 2);
+    w += __shfl_xor_sync(all, w, 1);
+    if ((lane & 7) == 0) sh[wid * NRED + (lane >> 3)] = w;
     __syncthreads();
-    for (int s = 1; s < nt; s <<= 1) {
-        /* pairwise in fixed order: thread tid (multiple of 2s) adds tid+s */
-        if ((tid % (2 * s)) == 0 && tid + s < nt)
-            for (int k = 0; k < NV; k++) sh[k * nt + tid] += sh[k * nt + tid + s];
-        __syncthreads();
+    if (wid == 0) {
+        /* lane 8 k + j: value k of warp j */
+        w = (lane & 7) < nw ? sh[(lane & 7) * NRED + (lane >> 3)] : 0.0;
+        w += __shfl_xor_sync(all, w, 4);
+        w += __shfl_xor_sync(all, w, 2);
+        w += __shfl_xor_sync(all, w, 1);
+        for (int k = 0; k < NRED; k++) v[k] = __shfl_sync(all, w, 8 * k);
     }
-    for (int k = 0; k < NV; k++) v[k] = sh[k * nt];
     __syncthreads();
 }
 
 /* The CTA's block sum of v into partial slot idx (written by thread 0). */
 __device__ __forceinline__ void reduce_part(RedP red, double (&v)[NRED], double *sh, unsigned idx)
 {
-    block_sum<NRED>(v, sh);
+    block_sum(v, sh);
     if (threadIdx.x == 0)
         for (int k = 0; k < NRED; k++) red.part[(size_t)idx * NRED + k] = v[k];
 }
@@ -429,7 +448,7 @@ __device__ void reduce_tail(RedP red, double *sh, unsigned narrive, unsigned npa
     double acc[NRED] = {0, 0, 0, 0};
     for (unsigned j = tid; j < npart; j += nt)
         for (int k = 0; k < NRED; k++) acc[k] += __ldcg(&red.part[(size_t)j * NRED + k]);
-    block_sum<NRED>(acc, sh);
+    block_sum(acc, sh);
     if (tid == 0) {
         DevScal *sc = red.sc;
         switch (red.kind) {
@@ -1077,295 +1096,555 @@ __global__ void __launch_bounds__(256, std::is_same<R, dd>::value ? GADE_DD_MINB
 
 
 /* ------------------------------------------------------------------ */
-/* assembled operator (one FP64 pulse, real couplings)                 */
+/* fixed-point products of FP64 values on the integer units             */
+/* ------------------------------------------------------------------ */
+/*
+ * GB300 retires 2 DFMA per clock and SM but 32 32x32+64-bit integer
+ * multiply-adds (measured: 1.6 against 24 per nominal clock), so the long
+ * real x real sums of the assembled operator run there.  A vector of FP64
+ * values that share a power of two is held as integers N, value = N 2^e:
+ *   coupling values   |N| <= 2^56, one e per (pair, row)      (FX_UPA = 3)
+ *   vector entries    |N| <  2^58, one e per staged window    (FX_UPX = 5)
+ * each in two signed limbs, N = hi 2^29 + lo, |lo| <= 2^28.  A product is
+ * hi hi 2^58 + (hi lo + lo hi) 2^29, three multiply-adds into two 64-bit
+ * sums (the lo lo term, below 2^-56 of the largest product, is left out);
+ * sums of up to 30 products stay below 2^63 and are exact.  A 53-bit
+ * mantissa is held in full down to 2^-3 (2^-5 for vector entries) of its
+ * group's largest value and rounded below that at 2^-56 (2^-58) of it, so a
+ * row's sum carries an error of about 2^-56 of its largest terms once,
+ * where FP64 rounds every product and partial sum to 2^-53 of them.
+ */
+#define FX_UPA 3
+#define FX_UPX 5
+#define FX_LB 29                       /* bits of the low limb */
+
+/* biased exponent field of a double given by its high word */
+__host__ __device__ __forceinline__ int fx_exp(unsigned hi) { return (int)((hi >> 20) & 0x7FF); }
+
+/* N of v in a group whose largest biased exponent is em (finite, em >= the
+   value's own): the mantissa shifted up by `up` bits and down by the
+   exponent difference (truncated) */
+__device__ __forceinline__ long long fx_from(double v, int em, int up)
+{
+    const unsigned long long b = (unsigned long long)__double_as_longlong(v);
+    int ev = (int)((b >> 52) & 0x7FF);
+    unsigned long long m = b & 0xFFFFFFFFFFFFFull;
+    if (ev) m |= 1ull << 52; else ev = 1;
+    const int d = em - ev;
+    m = d > 63 ? 0ull : (m << up) >> d;
+    return (long long)b < 0 ? -(long long)m : (long long)m;
+}
+/* two signed limbs of N */
+__device__ __forceinline__ int2 fx_split(long long N)
+{
+    int2 r;
+    r.x = (int)((N + (1ll << (FX_LB - 1))) >> FX_LB);
+    r.y = (int)(N - ((long long)r.x << FX_LB));
+    return r;
+}
+__device__ __forceinline__ double pow2d(int e) { return __hiloint2double((e + 1023) << 20, 0); }   /* -1022 <= e <= 1023 */
+/* acc += V 2^e; e of any size (below the normal range in two factors) */
+__device__ __forceinline__ double fx_add(double acc, long long V, int e)
+{
+    double v = (double)V;
+    if (e < -1022) { v *= pow2d(e + 900 < -1022 ? -1022 : e + 900); e = -900; }
+    return fma(v, pow2d(e > 1023 ? 1023 : e), acc);
+}
+/* the upper 16 bits of a double >= v (v >= 0): sign, exponent and 4 mantissa bits, rounded up */
+__device__ __forceinline__ unsigned short fx_bound16(double v)
+{
+    const unsigned long long b = (unsigned long long)__double_as_longlong(v);
+    return (unsigned short)((b + 0xFFFFFFFFFFFFull) >> 48);
+}
+__device__ __forceinline__ double fx_bound_to(unsigned short u) { return __hiloint2double((int)u << 16, 0); }
+
+/* ------------------------------------------------------------------ */
+/* assembled operator (real couplings)                                 */
 /* ------------------------------------------------------------------ */
 /*
  * The couplings of H(t) are linear in the six pulse factors, so for real
  * couplings every off-diagonal value is A(t) = sum_a w_a(t) K_a with K_a
  * the values for a unit factor a (built once from the matrix-free tables)
- * and w_a(t) the step's coefficient of a.  An apply then costs 2 FMAs per
- * stored value (a real value times a complex x) against ~4.4 in the
- * matrix-free form, for an assembly of 3 FMAs per value once per step (the
- * orders coupling a pair share a parity, which selects three of the six
- * factors).
- * Values are stored per (block row, coupled block) pair in the ELL slot
- * layout [pair][W][B] of the radial tables, so one slot map serves every
- * pair.
+ * and w_a(t) the step's coefficient of a.  The orders coupling a pair share
+ * a parity, which selects three of the six factors.
+ * Values are stored in the ELL slots of the radial tables, chunk by chunk:
+ * the rows of chunk q, padded to RMq = pad[q] (with a halves layout each half
+ * of the chunk's splines to an even count, so that two neighbouring rows make
+ * one aligned 16-byte load), at row positions off[q] .. off[q] + RMq - 1:
+ *   A [off[q] npairs W + (p W + slot) RMq + row], K with 3 factors per pair.
+ * K and A are fixed-point limbs (int2) with one exponent per (pair, factor,
+ * row position) and (pair, row position).  Ke holds the upper 16 bits of a
+ * bound of the row's largest |K| (its exponent field is the row's exponent),
+ * Ae the biased exponent of the step's values.
  */
+struct AsmLay {
+    const int *pad, *off;          /* [nchunk] padded rows, first row position */
+    const int *prow;               /* [Bp] row within the block of a row position (-1: padding) */
+    const int *pq;                 /* [Bp] its chunk << 16 | compact row within the chunk (0xffff: padding) */
+    int Bp, npairs, W, RMA;
+};
 
 /* K[pair][ia][slot][row] = sum over the pair's (order l, angular term e) of
    M0(l,k_r) a0[e] + M1 a0k[e] + M2 a1[e] + M3 a1k[e], from the tables of a
    unit factor a.  The orders coupling one pair share a parity (the angular
    selection rules), and order l uses the factors a = (l%2+1)%2 + 2 ia, so a
    pair stores three values per slot, ia = 0..2; the pairs of the other
-   parity are skipped.  grid (slot blocks, pairs) */
-__global__ void k_build_K(double *__restrict__ K, const R4<double>::T *__restrict__ M, int nk, int WB, int a,
-                          const int *__restrict__ pair_r, const int *__restrict__ pair_par,
-                          const int *__restrict__ row_kidx,
+   parity are skipped.  grid (row position blocks, pairs), one row per thread */
+__global__ void k_build_K(int2 *__restrict__ K, unsigned short *__restrict__ Ke, AsmLay L,
+                          const R4<double>::T *__restrict__ M, int nk, int B, int a, const int *__restrict__ pair_r,
+                          const int *__restrict__ pair_par, const int *__restrict__ row_kidx,
                           const int *__restrict__ le_ptr, const int *__restrict__ le_l, const int *__restrict__ le_e,
                           const double *__restrict__ a0, const double *__restrict__ a0k,
                           const double *__restrict__ a1, const double *__restrict__ a1k)
 {
-    const int p = blockIdx.y;
-    const int e_in = blockIdx.x * blockDim.x + threadIdx.x;
+    const int p = blockIdx.y, W = L.W;
+    const int g = blockIdx.x * blockDim.x + threadIdx.x;
     const int base = (pair_par[p] + 1) % 2;      /* the parity's first factor */
-    if (e_in >= WB || base != a % 2) return;
+    if (g >= L.Bp || base != a % 2) return;
+    const int i = L.prow[g];
+    if (i < 0) return;                           /* padding stays zero */
     const int ia = (a - base) / 2;
     const int kk = row_kidx[pair_r[p]];
-    double acc = 0.0;
-    for (int k = le_ptr[p]; k < le_ptr[p + 1]; k++) {
-        const int l = le_l[k], e = le_e[k];
-        const R4<double>::T m = M[((size_t)l * nk + kk) * WB + e_in];
-        acc = fma(m.a, a0[e], acc);
-        acc = fma(m.b, a0k[e], acc);
-        acc = fma(m.c, a1[e], acc);
-        acc = fma(m.d, a1k[e], acc);
+    double acc[30];
+    double mx = 0.0;
+    for (int t = 0; t < W; t++) {
+        double v = 0.0;
+        for (int k = le_ptr[p]; k < le_ptr[p + 1]; k++) {
+            const int l = le_l[k], e = le_e[k];
+            const R4<double>::T m = M[(((size_t)l * nk + kk) * W + t) * B + i];
+            v = fma(m.a, a0[e], v);
+            v = fma(m.b, a0k[e], v);
+            v = fma(m.c, a1[e], v);
+            v = fma(m.d, a1k[e], v);
+        }
+        acc[t] = v;
+        mx = fmax(mx, fabs(v));
     }
-    K[((size_t)p * 3 + ia) * WB + e_in] = acc;
+    const unsigned short u = fx_bound16(mx);
+    const int em = u >> 4 ? u >> 4 : 1;
+    Ke[((size_t)p * 3 + ia) * L.Bp + g] = u;
+    const int q = L.pq[g] >> 16, RMq = L.pad[q];
+    int2 *Kq = K + (size_t)L.off[q] * L.npairs * 3 * W + ((size_t)p * 3 + ia) * W * RMq + (g - L.off[q]);
+    for (int t = 0; t < W; t++) Kq[(size_t)t * RMq] = fx_split(fx_from(acc[t], em, FX_UPA));
 }
 
-/* this step's couplings A[pair] = sum_ia w_ia K[pair][ia], w_ia the
-   imaginary part of the step's coefficient of order parity par(pair) and
-   factor ia (coef[lpar * 3 + ia], lpar the first order of that parity).
-   grid (element blocks of a pair, pairs); two values per thread */
+/* complex64 copies of the step's values in the layout of k_apply_asm32
+   ([q][pair][W][RMp], compact rows) */
 struct A32Map {
     float *A32;                    /* NULL: no float copy */
-    const int *row_pos;            /* [B]: chunk << 16 | row within the chunk */
-    int B, W, RMp, npairs;
+    int RMp;
     size_t astride;                /* floats per pulse */
 };
 
-__global__ void k_assemble(double2 *__restrict__ A, A32Map F, const double2 *__restrict__ K, int WB2,
-                           const int *__restrict__ pair_par, const double2 *__restrict__ coef, int2 lpar,
-                           const int *__restrict__ plist, size_t astride2, size_t kstride2, int lmax)
+/*
+ * This step's couplings A[pair] = sum_ia w_ia K[pair][ia], w_ia the
+ * imaginary part of the step's coefficient of order parity par(pair) and
+ * factor ia (coef[lpar * 3 + ia], lpar the first order of that parity).
+ * One thread per (pair, two rows) and nsl of the W slots in sequence; grid
+ * (chunk, groups of blockDim / (RMA/2) pairs, groups of PT pulses x slot
+ * groups).  The rows' exponents are known before
+ * their values are: |A| <= sum_ia |w_ia| max|K_ia|.  Each w_ia is scaled once
+ * per row to a fixed-point factor with A = (sum_ia w_ia K_ia) >> 58, so a
+ * value costs nine integer multiply-adds and the kernel runs at the memory
+ * rate (24 bytes in per value and pulse group, 8 out per pulse): 190 us at
+ * 41.7M values, 6.9 TB/s (209 us with three FP64 DFMA per value, which bound it).  With PT > 1 the pulses of a group share the
+ * reads of K (batches whose pulses share the radial tables: 8 pulses 1.64 ms,
+ * now 0.69 ms).
+ */
+#define ASB_PF 1    /* slots prefetched ahead of the five being loaded (5: 204 us, 10: 238 us against 190 us at 41.7M values) */
+template <int PT>
+__global__ void __launch_bounds__(128) k_assemble(int2 *__restrict__ A, unsigned short *__restrict__ Ae, A32Map F,
+                                                  const int2 *__restrict__ K, const unsigned short *__restrict__ Ke,
+                                                  AsmLay L, const int *__restrict__ pair_par,
+                                                  const double2 *__restrict__ coef, int2 lpar,
+                                                  const int *__restrict__ plist, int nslot, size_t kstride,
+                                                  size_t kestride, int lmax, int nsl)
 {
-    /* F.A32 (NULL: none): the values rounded to float for mixed precision,
-       in the chunk-major layout of k_apply_asm32 ([q][pair][W][RMp]).
-       grid z: pulse slot (plist: slot -> pulse); A per pulse, K per pulse
-       (kstride2 0: shared by pulses with the same radial tables) */
     pdl_enter();
-    const int pulse = plist ? plist[blockIdx.z] : 0;
-    A += (size_t)pulse * astride2;
-    float *A32 = F.A32 ? F.A32 + (size_t)pulse * F.astride : nullptr;
-    K += (size_t)pulse * kstride2;
-    coef += (size_t)pulse * lmax * 3;
-    const int p = blockIdx.y;
-    const int par = pair_par[p];
-    const int cb = 3 * (par ? lpar.y : lpar.x);
-    const double w0 = coef[cb].y, w1 = coef[cb + 1].y, w2 = coef[cb + 2].y;
-    const double2 *Kp = K + (size_t)p * 3 * WB2;
-    double2 *Ap = A + (size_t)p * WB2;
-    for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < WB2; e += gridDim.x * blockDim.x) {
-        const double2 k0 = __ldcs(&Kp[e]), k1 = __ldcs(&Kp[WB2 + e]), k2 = __ldcs(&Kp[2 * WB2 + e]);
-        double2 v;
-        v.x = fma(w2, k2.x, fma(w1, k1.x, w0 * k0.x));
-        v.y = fma(w2, k2.y, fma(w1, k1.y, w0 * k0.y));
-        Ap[e] = v;
-        if (A32) {
-            /* values 2e and 2e+1 of the pair: slot t, rows i0 and i0 + 1 (B even) */
-            const int e2 = 2 * e, t = e2 / F.B, i0 = e2 - t * F.B;
-            const int rp0 = F.row_pos[i0], rp1 = F.row_pos[i0 + 1];
-            float *d = A32 + ((size_t)p * F.W + t) * F.RMp;
-            const size_t qs = (size_t)F.npairs * F.W * F.RMp;
-            d[(size_t)(rp0 >> 16) * qs + (rp0 & 0xffff)] = (float)v.x;
-            d[(size_t)(rp1 >> 16) * qs + (rp1 & 0xffff)] = (float)v.y;
+    const int q = blockIdx.x, W = L.W, NPR = L.RMA >> 1;
+    const int sub = threadIdx.x / NPR, rp = threadIdx.x - sub * NPR;
+    const int p = blockIdx.y * (blockDim.x / NPR) + sub;
+    const int RMq = L.pad[q], off = L.off[q], g = off + 2 * rp;
+    if (sub >= blockDim.x / NPR || p >= L.npairs || 2 * rp >= RMq) return;
+    const int nsg = (W + nsl - 1) / nsl;             /* slot groups */
+    const int s0 = blockIdx.z / nsg * PT, t0 = blockIdx.z % nsg * nsl, t1 = min(W, t0 + nsl);
+    const int cb = 3 * (pair_par[p] ? lpar.y : lpar.x);
+    const int pulse0 = plist ? plist[s0] : 0;
+    const int q0 = L.pq[g], q1 = L.pq[g + 1];
+    const size_t astride = (size_t)L.npairs * W * L.Bp, aestride = (size_t)L.npairs * L.Bp;
+    K += (size_t)pulse0 * kstride + ((size_t)off * L.npairs + (size_t)p * RMq) * 3 * W + (g - off);
+    A += ((size_t)off * L.npairs + (size_t)p * RMq) * W + (g - off);
+    Ke += (size_t)pulse0 * kestride + (size_t)p * 3 * L.Bp + g;
+    Ae += (size_t)p * L.Bp + g;
+    const size_t ks = (size_t)W * RMq;             /* K values of one factor */
+    /* slots t0 .. t1 - 1 of the pair's three factors (contiguous runs) into L2 */
+    auto prefetch = [&](int a, int b) {
+        if (b > t1) b = t1;
+        if (rp >= 3 || a >= b) return;
+        asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(K - 2 * rp + rp * ks + (size_t)a * RMq),
+                     "r"((unsigned)((b - a) * RMq * sizeof(int2))) : "memory");
+    };
+    prefetch(t0, t0 + ASB_PF);
+    ushort2 ke[3];
+#pragma unroll
+    for (int ia = 0; ia < 3; ia++) ke[ia] = *(const ushort2 *)(Ke + (size_t)ia * L.Bp);
+    int2 w[PT][3][2];
+    int pulse[PT];
+    float f0[PT][2], f1[PT][2];
+#pragma unroll
+    for (int j = 0; j < PT; j++) {
+        pulse[j] = -1;
+        if (s0 + j >= nslot) continue;
+        pulse[j] = plist ? plist[s0 + j] : 0;
+        const double2 *cp = coef + (size_t)pulse[j] * lmax * 3 + cb;
+        const double wv[3] = {cp[0].y, cp[1].y, cp[2].y};
+        unsigned short em2[2];
+#pragma unroll
+        for (int rr = 0; rr < 2; rr++) {
+            double b = 0.0;
+#pragma unroll
+            for (int ia = 0; ia < 3; ia++) b = fma(fabs(wv[ia]), fx_bound_to(rr ? ke[ia].y : ke[ia].x), b);
+            int em = fx_exp((unsigned)__double2hiint(b));     /* 2047: a coefficient is not finite */
+            if (em == 0) em = 1;
+#pragma unroll
+            for (int ia = 0; ia < 3; ia++) {
+                /* w 2^(ek - em + 58) */
+                const int u = (rr ? ke[ia].y : ke[ia].x) >> 4, ek = u ? u : 1;
+                const unsigned long long bits = (unsigned long long)__double_as_longlong(wv[ia]);
+                int ew = (int)((bits >> 52) & 0x7FF);
+                unsigned long long m = bits & 0xFFFFFFFFFFFFFull;
+                if (ew) m |= 1ull << 52; else ew = 1;
+                const int sh = ew + ek - em - 1017;
+                m = sh >= 0 ? (sh > 6 ? 0ull : m << sh) : (sh < -63 ? 0ull : m >> -sh);
+                w[j][ia][rr] = fx_split((long long)bits < 0 ? -(long long)m : (long long)m);
+            }
+            em2[rr] = (unsigned short)em;
+            if (F.A32) {
+                /* N 2^(em - 1078) as a float in two factors */
+                const int k = em - 1078, k1 = k < -126 ? -126 : (k > 127 ? 127 : k);
+                const int k2 = k - k1 < -126 ? -126 : (k - k1 > 127 ? 127 : k - k1);
+                f0[j][rr] = em == 2047 ? __int_as_float(0x7FC00000) : __int_as_float((k1 + 127) << 23);
+                f1[j][rr] = __int_as_float((k2 + 127) << 23);
+            }
+        }
+        if (t0 == 0) *(ushort2 *)(Ae + (size_t)pulse[j] * aestride) = make_ushort2(em2[0], em2[1]);
+    }
+    float *A32 = F.A32 ? F.A32 + ((size_t)q * L.npairs + p) * W * F.RMp : nullptr;
+#pragma unroll 5
+    for (int t = t0; t < t1; t++) {
+        if ((t - t0) % 5 == 0) prefetch(t + ASB_PF, t + ASB_PF + 5);
+        int4 k[3];
+#pragma unroll
+        for (int ia = 0; ia < 3; ia++) k[ia] = __ldcs((const int4 *)(K + ia * ks + (size_t)t * RMq));
+#pragma unroll
+        for (int j = 0; j < PT; j++) {
+            if (PT > 1 && pulse[j] < 0) continue;
+            long long N[2];
+#pragma unroll
+            for (int rr = 0; rr < 2; rr++) {
+                long long h = 0, m = 0;
+#pragma unroll
+                for (int ia = 0; ia < 3; ia++) {
+                    const int kh = rr ? k[ia].z : k[ia].x, kl = rr ? k[ia].w : k[ia].y;
+                    h += (long long)kh * w[j][ia][rr].x;
+                    m += (long long)kh * w[j][ia][rr].y;
+                    m += (long long)kl * w[j][ia][rr].x;
+                }
+                N[rr] = h + ((m + (1ll << (FX_LB - 1))) >> FX_LB);
+            }
+            const int2 v0 = fx_split(N[0]), v1 = fx_split(N[1]);
+            *(int4 *)(A + (size_t)pulse[j] * astride + (size_t)t * RMq) = make_int4(v0.x, v0.y, v1.x, v1.y);
+            if (F.A32) {
+                float *d = A32 + (size_t)pulse[j] * F.astride + (size_t)t * F.RMp;
+                if ((q0 & 0xffff) != 0xffff) d[q0 & 0xffff] = __ll2float_rn(N[0]) * f0[j][0] * f1[j][0];
+                if ((q1 & 0xffff) != 0xffff) d[q1 & 0xffff] = __ll2float_rn(N[1]) * f0[j][1] * f1[j][1];
+            }
         }
     }
 }
 
-#define ASM_GB 4   /* coupled blocks staged per phase */
+#define ASM_GB 16   /* coupled blocks staged per phase: two per warp */
+#ifndef ASM_UFIX
+#define ASM_UFIX 4.0
+#endif
 
-/* shared memory of k_apply_asm: x slices (x_r, x_n, delta), the staged
-   windows of ASM_GB coupled blocks, the slot map, the reduction buffer */
-__host__ __device__ __forceinline__ unsigned asm_smem(int CS, int W, int RM, int nt, unsigned elem, unsigned *o_xw,
-                                                      unsigned *o_lcs, unsigned *o_red)
+/* shared memory of k_apply_asm: x windows of the block row (x, x_n, delta;
+   FP64), the staged fixed-point windows of ASM_GB coupled blocks, the slot
+   columns (general layout only), the exchange / reduction buffer.  XS:
+   entries of a window: two halves of RM/2 + 16 columns each (halves layout)
+   or the chunk's columns and a zero column */
+__host__ __device__ __forceinline__ int asm_xs(int RM, int CM, bool halves) { return halves ? RM + 32 : (CM + 2) & ~1; }
+__host__ __device__ __forceinline__ unsigned asm_smem(int XS, int W, int RM, bool halves, int nt, unsigned *o_xw,
+                                                      unsigned *o_lc, unsigned *o_red, unsigned *o_xd)
 {
-    unsigned o = up32(3u * elem * CS);
-    *o_xw = o;  o = up32(o + elem * ASM_GB * CS);
-    *o_lcs = o; o = up32(o + 4u * W * RM);
+    unsigned o = up32(3u * 16u * XS);
+    *o_xw = o;  o = up32(o + 16u * ASM_GB * XS);
+    *o_lc = o;  o = up32(o + (halves ? 0u : 2u * W * RM));
     *o_red = o; o = up32(o + 8u * NRED * nt);
+    *o_xd = o;  o = up32(o + 3u * 16u * RM);
     return o;
 }
 
 /*
  * y = (S + H(t)) x with the assembled couplings: grid (pulse slot, segment)
  * over the same units and pieces as k_apply (a piece's range is a range of
- * (block row, coupled block) pairs).  Two threads per row, 15 ELL slots each
- * with their local columns in registers; per group of ASM_GB coupled blocks
- * the CTA stages the blocks' x windows in shared memory, then every thread
- * streams its rows' values and adds value x window[column].
+ * (block row, coupled block) pairs).  Per phase of ASM_GB coupled blocks each
+ * warp stages windows of x in shared memory as fixed-point limbs with the
+ * window's largest exponent.  Then a thread takes two neighbouring rows (one
+ * 16-byte load per slot) of every NG-th staged block, all W slots: with the
+ * halves layout the slots of a row are consecutive window entries, so the
+ * two rows share all but one of the entries they read and no column index is
+ * needed.  The products run on the integer units (see above) with one FP64
+ * addition per pair, row and component.  The NG partial sums of a row meet in
+ * shared memory, where two threads per row add the diagonal blocks in FP64 (their
+ * entries near the origin are orders of magnitude above the rest and meet
+ * entries of x that are as much smaller: products of the window's common
+ * exponent would lose them).
+ * N = 53,040 (41.7M values, 0.33 GB): 188 us with FP64 products (FP64 pipe
+ * bound), 83 us now (4.0 TB/s; each CTA's staging, exchange and epilogue do not
+ * overlap its stream); N = 244,000 (2.8 GB): 1.36 ms, now 0.51 ms (5.5 TB/s).
+ * HL: the halves layout (slot 15 h + t of a row of spline s is spline
+ * s - 7 + t of half h); otherwise the slots' columns come from a table.
  */
-template <typename R, bool SEP>
+template <bool SEP, bool HL>
 __global__ void __launch_bounds__(256, 3)
-    k_apply_asm(OpP P, const typename Cx<R>::T *__restrict__ x, int mode, VecP V, RedP red)
+    k_apply_asm(OpP P, const double2 *__restrict__ x, int mode, VecP V, RedP red)
 {
-    /* R: double (FP64 values and vectors) or float (the complex64 inner solve
-       of mixed precision, with the step's values rounded to float) */
     constexpr int HJ = 15;
-    typedef typename Cx<R>::T C;
+    typedef double2 C;
     extern __shared__ __align__(32) unsigned char smem_raw[];
-    const int CS = (P.CM + 2) & ~1;
-    unsigned oxw, olcs, ored;
-    asm_smem(CS, P.W, P.RM, blockDim.x, sizeof(C), &oxw, &olcs, &ored);
-    C *xr = (C *)smem_raw, *xs = xr + CS, *ds = xs + CS;
-    C *xw = (C *)(smem_raw + oxw);
-    int *lcs = (int *)(smem_raw + olcs);
+    const int XS = asm_xs(P.RMA, P.CM, HL);
+    unsigned oxw, olc, ored, oxd;
+    asm_smem(XS, P.W, P.RMA, HL, blockDim.x, &oxw, &olc, &ored, &oxd);
+    C *xr = (C *)smem_raw, *xs = xr + XS, *ds = xs + XS;   /* windows of the block row itself: x, x_n, delta (FP64) */
+    int4 *xw = (int4 *)(smem_raw + oxw);      /* [ASM_GB][XS] re hi, re lo, im hi, im lo */
+    unsigned short *lc = (unsigned short *)(smem_raw + olc);   /* [W][RM] window entry of a slot (general layout) */
     double *shred = (double *)(smem_raw + ored);
+    C *xd = (C *)(smem_raw + oxd);            /* [row][3] the diagonal blocks' sums: S, H (or D), S delta */
 
     pdl_enter();
     const int pulse = P.plist ? P.plist[blockIdx.x] : 0;
     if (!red_select(red, pulse)) return;
     x += (long long)pulse * P.vstride;
-    const int tid = threadIdx.x, nt = blockDim.x;
-    const int B = P.B, W = P.W, CM = P.CM;
-    if (tid == 0) {
-        const C z = mk<C>(0, 0);
-        xr[CM] = z; xs[CM] = z; ds[CM] = z;
-        for (int g = 0; g < ASM_GB; g++) xw[g * CS + CM] = z;
-    }
-    __shared__ int s_pc, s_pw;
+    const int tid = threadIdx.x, nt = blockDim.x, lane = tid & 31, wid = tid >> 5;
+    const int B = P.B, W = P.W, CM = P.CM, ns = B >> 1, HW = XS >> 1;
+    const int RMA = P.RMA, NPR = RMA >> 1, NG = nt / NPR;        /* row pairs of a chunk, thread groups */
+    const int grp = tid / NPR, rp = tid - grp * NPR;
+    const int half = tid / RMA, trow = tid - half * RMA;   /* diagonal blocks and output: two threads per row */
+    /* AX_R0V, AX_TS: D x where the caller knows it (NULL: formed here) */
+    const C *dx = !SEP && (mode == AX_R0V || mode == AX_TS) ? (const C *)V.in1 : nullptr;
+    __shared__ int s_pc, s_pw, s_ex[ASM_GB];
     for (int pc = P.seg_ptr[blockIdx.y]; pc < P.seg_ptr[blockIdx.y + 1]; pc = *(volatile int *)&s_pc + 1) {
     const int4 pd = P.pieces[pc];
     const int u = pd.x, r = u / P.nchunk, q = u - r * P.nchunk;
-    const int kk = P.row_kidx[r];
-    const int nrows = P.chunk_nrows[q], ncols = P.chunk_ncols[q];
-    const int half = tid / P.RM, trow = tid - half * P.RM;
-    const int i = (half < 2 && trow < nrows) ? P.chunk_rows[q * P.RM + trow] : -1;
-    const int jb = half == 0 ? 0 : (W + 1) / 2, je = half == 0 ? (W + 1) / 2 : W;
-    const int nj = je - jb;
+    const int RMq = P.pad[q], off = P.off[q], n0p = RMq >> 1;
+    const int ncols = HL ? XS : P.chunk_ncols[q] + 1;
     const int *cols = P.chunk_cols + (size_t)q * CM;
-    const C *xb = x + (size_t)r * B;
+    const int sp0 = q * (P.RM >> 1) - 7;             /* first spline of the windows (halves layout) */
+    const int nv = n0p + 14;                         /* valid window entries per half (padding rows read zeros) */
+    /* column of window entry c, -1: a zero */
+    auto column = [&](int c) {
+        if (HL) {
+            const int h = c >= HW, k = c - h * HW, sp = sp0 + k;
+            return k < nv && sp >= 0 && sp < ns ? h * ns + sp : -1;
+        }
+        return c < ncols - 1 ? cols[c] : -1;
+    };
     __syncthreads();                          /* the previous piece is done with shared memory */
     if (tid == 0) { s_pc = pc; s_pw = pd.w; } /* read back after the next barrier */
-    {
-        const int *gl = P.chunk_lcol + (size_t)q * W * P.RM;
-        for (int e = tid; e < W * P.RM; e += nt) { const int v = gl[e]; lcs[e] = v < 0 ? CM : v; }
-    }
-    for (int c = tid; c < ncols; c += nt) xr[c] = xb[cols[c]];
-    if (mode == AX_MIX) {
+    const bool diag = (pd.w & 0xffff) == 0 && !dx;   /* the unit's first piece has the diagonal blocks */
+    if (diag) {
         const size_t vo = (size_t)pulse * P.vstride + (size_t)r * B;
-        const C *xn = (const C *)V.in0 + vo, *dn = (const C *)V.in1 + vo;
-        for (int c = tid; c < ncols; c += nt) { xs[c] = xn[cols[c]]; ds[c] = dn[cols[c]]; }
-    }
-    __syncthreads();
-    unsigned lcp[(HJ + 1) / 2];
-#pragma unroll
-    for (int t = 0; t < HJ; t += 2) {
-        const unsigned c0 = (t < nj && trow < P.RM) ? lcs[(jb + t) * P.RM + trow] : CM;
-        const unsigned c1 = (t + 1 < HJ && t + 1 < nj && trow < P.RM) ? lcs[(jb + t + 1) * P.RM + trow] : CM;
-        lcp[t / 2] = c0 | (c1 << 16);
-    }
-#define LCO(t) ((int)(((t) & 1) ? (lcp[(t) >> 1] >> 16) : (lcp[(t) >> 1] & 0xffffu)))
-    const int jB = jb * B;
-    C accS = mk<C>(0, 0), accH = accS, accD = accS;
-    if (i >= 0 && (pd.w & 0xffff) == 0) {     /* diagonal blocks: the unit's first piece */
-        if (SEP && mode == AX_MIX) {
-            const C *Se = (const C *)P.S_ell + (size_t)kk * W * B + i + jB;
-            const C *He = (const C *)P.Hst_ell + (size_t)pulse * P.dstride + (size_t)kk * W * B + i + jB;
-#pragma unroll
-            for (int t = 0; t < HJ; t++) {
-                const int lc = LCO(t);
-                const C sv = *Se;
-                cfma(accS, sv, xs[lc]);
-                cfma(accD, sv, ds[lc]);
-                cfma(accH, *He, xr[lc]);
-                if (t + 1 < nj) { Se += B; He += B; }
-            }
-        } else if (SEP) {
-            const C *Se = (const C *)P.S_ell + (size_t)kk * W * B + i + jB;
-            const C *He = (const C *)P.Hst_ell + (size_t)pulse * P.dstride + (size_t)kk * W * B + i + jB;
-#pragma unroll
-            for (int t = 0; t < HJ; t++) {
-                const C xv = xr[LCO(t)];
-                cfma(accS, *Se, xv);
-                cfma(accH, *He, xv);
-                if (t + 1 < nj) { Se += B; He += B; }
-            }
-        } else {
-            const C *De = (const C *)P.D_ell + (size_t)pulse * P.dstride + (size_t)kk * W * B + i + jB;
-#pragma unroll
-            for (int t = 0; t < HJ; t++) {
-                cfma(accH, *De, xr[LCO(t)]);
-                if (t + 1 < nj) De += B;
+        const C *xb = x + (size_t)r * B;
+        for (int c = tid; c < ncols; c += nt) {
+            const int cc = column(c);
+            xr[c] = cc >= 0 ? xb[cc] : mk<C>(0, 0);
+            if (SEP && mode == AX_MIX) {
+                xs[c] = cc >= 0 ? ((const C *)V.in0)[vo + cc] : mk<C>(0, 0);
+                ds[c] = cc >= 0 ? ((const C *)V.in1)[vo + cc] : mk<C>(0, 0);
             }
         }
     }
-    const size_t WB = (size_t)W * B;
+    if (!HL) {
+        const int *gl = P.chunk_lcol + (size_t)q * W * P.RM;
+        for (int e = tid; e < W * RMA; e += nt) {
+            const int t = e / RMA, row = e - t * RMA, v = row < P.RM ? gl[t * P.RM + row] : -1;
+            lc[e] = (unsigned short)(v < 0 ? ncols - 1 : v);
+        }
+    }
+    const int i = (half < 2 && trow < RMq) ? P.prow[off + trow] : -1;
+    const bool act = grp < NG && 2 * rp < RMq;
+    const int hb = HL && 2 * rp >= n0p ? n0p : 0;    /* the rows' first window entry: row - hb */
+    C acc0 = mk<C>(0, 0), acc1 = acc0;
+    const int2 *Aq = (const int2 *)P.A + (size_t)pulse * P.astride + (size_t)off * P.npairs * W + 2 * rp;
+    if (diag) {
+        /* the diagonal blocks first: their FP64 work runs while the first values arrive */
+        C accS = mk<C>(0, 0), accH = accS, accD = accS;
+        __syncthreads();                      /* the own windows are staged */
+        if (i >= 0) {
+            const int kk = P.row_kidx[r];
+            const int jb = half == 0 ? 0 : (W + 1) / 2, je = half == 0 ? (W + 1) / 2 : W;
+            const int wb = HL ? half * HW + trow - (trow >= n0p ? n0p : 0) : 0;
+            const size_t eo = (size_t)kk * W * B + i + (size_t)jb * B;
+            if (SEP) {
+                const C *Se = (const C *)P.S_ell + eo;
+                const C *He = (const C *)P.Hst_ell + (size_t)pulse * P.dstride + eo;
+#pragma unroll 5
+                for (int t = 0; t < je - jb; t++) {
+                    const int w = HL ? wb + t : lc[(jb + t) * RMA + trow];
+                    const C sv = Se[(size_t)t * B], hv = He[(size_t)t * B];
+                    if (mode == AX_MIX) {
+                        /* x = w = 2 x_n + delta: S x_n, S delta and (i h dt/2 h0) w */
+                        cfma(accS, sv, xs[w]);
+                        cfma(accD, sv, ds[w]);
+                    } else {
+                        cfma(accS, sv, xr[w]);
+                    }
+                    cfma(accH, hv, xr[w]);
+                }
+            } else {
+                const C *De = (const C *)P.D_ell + (size_t)pulse * P.dstride + eo;
+#pragma unroll 15
+                for (int t = 0; t < je - jb; t++)
+                    cfma(accH, De[(size_t)t * B], xr[HL ? wb + t : lc[(jb + t) * RMA + trow]]);
+            }
+        }
+        if (half == 1 && i >= 0) {
+            xd[3 * trow + 1] = accH;
+            if (SEP) { xd[3 * trow] = accS; xd[3 * trow + 2] = accD; }
+        }
+        __syncthreads();
+        if (half == 0 && i >= 0) {
+            xd[3 * trow + 1] = cadd(accH, xd[3 * trow + 1]);
+            if (SEP) { xd[3 * trow] = cadd(accS, xd[3 * trow]); xd[3 * trow + 2] = cadd(accD, xd[3 * trow + 2]); }
+        }
+    }
     for (int pg = pd.y; pg < pd.z; pg += ASM_GB) {
         const int ng = pd.z - pg < ASM_GB ? pd.z - pg : ASM_GB;
         __syncthreads();     /* staging done / previous group's products done */
-        for (int item = tid; item < ng * ncols; item += nt) {
-            const int g = item / ncols, c = item - g * ncols;
-            xw[g * CS + c] = x[(size_t)P.pair_c[pg + g] * B + cols[c]];
+        for (int g = wid; g < ng; g += nt >> 5) {
+            /* the window of one coupled block: the largest exponent over the
+               warp, then the limbs (the second read of x hits L1) */
+            const C *xc = x + (size_t)P.pair_c[pg + g] * B;
+            int4 *win = xw + g * XS;
+            unsigned mx = 0;
+#pragma unroll 5
+            for (int c = lane; c < ncols; c += 32) {
+                const int cc = column(c);
+                const C v = cc >= 0 ? xc[cc] : mk<C>(0, 0);
+                mx = max(mx, max((unsigned)__double2hiint(v.x) & 0x7FFFFFFFu,
+                                 (unsigned)__double2hiint(v.y) & 0x7FFFFFFFu));
+            }
+            int em = fx_exp(__reduce_max_sync(0xffffffffu, mx));
+            if (em == 0) em = 1;
+            if (lane == 0) s_ex[g] = em;
+#pragma unroll 5
+            for (int c = lane; c < ncols; c += 32) {
+                const int cc = column(c);
+                const C v = cc >= 0 ? xc[cc] : mk<C>(0, 0);
+                const int2 re = fx_split(fx_from(v.x, em, FX_UPX)), im = fx_split(fx_from(v.y, em, FX_UPX));
+                win[c] = make_int4(re.x, re.y, im.x, im.y);
+            }
         }
         __syncthreads();
-        if (i >= 0) {
-            const R *A0 = (const R *)P.A + (size_t)pulse * P.astride + (size_t)pg * WB + i + jB;
-            if constexpr (sizeof(R) == 4) {
-                /* complex64: latency-bound, so the next block's values are
-                   loaded while this block's are used (two sets in flight) */
-                R cur[HJ];
-                {
-                    const R *Av = A0;
+        if (act) {
+            for (int g = grp; g < ng; g += NG) {
+                const ushort2 ea = *(const ushort2 *)(P.Ae + (size_t)pulse * P.aestride + (size_t)(pg + g) * P.Bp + off +
+                                                      2 * rp);
+                const int ex = s_ex[g];
+                const int2 *Av = Aq + (size_t)(pg + g) * W * RMq;
+                if (ex != 2047) {
+                    const int4 *xg = xw + g * XS + (HL ? 2 * rp - hb : 0);
+                    long long h0r = 0, m0r = 0, h0i = 0, m0i = 0, h1r = 0, m1r = 0, h1i = 0, m1i = 0;
 #pragma unroll
-                    for (int t = 0; t < HJ; t++) { cur[t] = __ldcs(Av); if (t + 1 < nj) Av += B; }
-                }
-                for (int g = 0; g < ng; g++) {
-                    R nxt[HJ];
-                    if (g + 1 < ng) {
-                        const R *Av = A0 + (size_t)(g + 1) * WB;
+                    for (int hh = 0; hh < 2; hh++) {
+                        int4 b1 = HL ? xg[hh * HW] : make_int4(0, 0, 0, 0);
+                        int4 av[HJ];           /* 15 loads in flight */
 #pragma unroll
-                        for (int t = 0; t < HJ; t++) { nxt[t] = __ldcs(Av); if (t + 1 < nj) Av += B; }
+                        for (int t = 0; t < HJ; t++)
+                            av[t] = HL || hh * HJ + t < W ? __ldcs((const int4 *)(Av + (size_t)(hh * HJ + t) * RMq))
+                                                          : make_int4(0, 0, 0, 0);
+#pragma unroll
+                        for (int t = 0; t < HJ; t++) {
+                            if (!HL && hh * HJ + t >= W) break;
+                            const int4 a = av[t];
+                            int4 b0 = b1;
+                            if (HL) {
+                                b1 = xg[hh * HW + t + 1];
+                            } else {
+                                b0 = xg[lc[(hh * HJ + t) * RMA + 2 * rp]];
+                                b1 = xg[lc[(hh * HJ + t) * RMA + 2 * rp + 1]];
+                            }
+                            h0r += (long long)a.x * b0.x;
+                            m0r += (long long)a.x * b0.y;
+                            m0r += (long long)a.y * b0.x;
+                            h0i += (long long)a.x * b0.z;
+                            m0i += (long long)a.x * b0.w;
+                            m0i += (long long)a.y * b0.z;
+                            h1r += (long long)a.z * b1.x;
+                            m1r += (long long)a.z * b1.y;
+                            m1r += (long long)a.w * b1.x;
+                            h1i += (long long)a.z * b1.z;
+                            m1i += (long long)a.z * b1.w;
+                            m1i += (long long)a.w * b1.z;
+                        }
                     }
-                    const C *xg = xw + g * CS;
-#pragma unroll
-                    for (int t = 0; t < HJ; t++) rfma(accH, cur[t], xg[LCO(t)]);
-#pragma unroll
-                    for (int t = 0; t < HJ; t++) cur[t] = nxt[t];
-                }
-            } else {
-                for (int g = 0; g < ng; g++) {
-                    const R *Av = A0 + (size_t)g * WB;
-                    const C *xg = xw + g * CS;
-#pragma unroll
-                    for (int t = 0; t < HJ; t++) {
-                        rfma(accH, __ldcs(Av), xg[LCO(t)]);
-                        if (t + 1 < nj) Av += B;
+                    const long long rnd = 1ll << (FX_LB - 1);
+                    if (ea.x == 2047 || ea.y == 2047) {
+                        acc0 = mk<C>(__longlong_as_double(0x7FF8000000000000ll), __longlong_as_double(0x7FF8000000000000ll));
+                        acc1 = acc0;
+                    } else {
+                        const int e0 = ea.x + ex - 2100, e1 = ea.y + ex - 2100;
+                        acc0.x = fx_add(acc0.x, h0r + ((m0r + rnd) >> FX_LB), e0);
+                        acc0.y = fx_add(acc0.y, h0i + ((m0i + rnd) >> FX_LB), e0);
+                        acc1.x = fx_add(acc1.x, h1r + ((m1r + rnd) >> FX_LB), e1);
+                        acc1.y = fx_add(acc1.y, h1i + ((m1i + rnd) >> FX_LB), e1);
+                    }
+                } else {
+                    /* an infinity or NaN in the window: products in FP64, so that it
+                       reaches the rows that hold it and no others */
+                    const C *xc = x + (size_t)P.pair_c[pg + g] * B;
+                    for (int rr = 0; rr < 2; rr++) {
+                        const int row = P.prow[off + 2 * rp + rr], e = rr ? ea.y : ea.x;
+                        if (row < 0) continue;
+                        const double sc = e == 2047 ? __longlong_as_double(0x7FF8000000000000ll)
+                                                    : pow2d(e - 1078 < -1022 ? -1022 : e - 1078);
+                        for (int t = 0; t < W; t++) {
+                            const int w = HL ? (t / HJ) * HW + 2 * rp + rr - hb + t % HJ : lc[t * RMA + 2 * rp + rr];
+                            const int cc = column(w);
+                            if (cc < 0) continue;
+                            const int2 a = Av[(size_t)t * RMq + rr];
+                            rfma(rr ? acc1 : acc0, ((double)a.x * 536870912.0 + (double)a.y) * sc, xc[cc]);
+                        }
                     }
                 }
             }
         }
     }
-#undef LCO
-    /* combine the two halves of every row */
+    /* the groups' partial sums of a row: [grp][row position] in shared memory */
     __syncthreads();
-    {
-        C *xch = (C *)shred;
-        if (SEP) {
-            if (half == 1 && i >= 0) { xch[3 * trow] = accS; xch[3 * trow + 1] = accH; xch[3 * trow + 2] = accD; }
-            __syncthreads();
-            if (half == 0 && i >= 0) {
-                accS = cadd(accS, xch[3 * trow]);
-                accH = cadd(accH, xch[3 * trow + 1]);
-                accD = cadd(accD, xch[3 * trow + 2]);
-            }
-        } else {
-            if (half == 1 && i >= 0) xch[trow] = accH;
-            __syncthreads();
-            if (half == 0 && i >= 0) accH = cadd(accH, xch[trow]);
+    C *xch = (C *)shred;
+    if (grp < NG) { xch[grp * RMA + 2 * rp] = acc0; xch[grp * RMA + 2 * rp + 1] = acc1; }
+    __syncthreads();
+    C accS = mk<C>(0, 0), accH = accS, accD = accS;
+    if (i >= 0 && half == 0) {
+        for (int k = 0; k < NG; k++) accH = cadd(accH, xch[k * RMA + trow]);
+        if (diag) {
+            accH = cadd(accH, xd[3 * trow + 1]);
+            if (SEP) { accS = xd[3 * trow]; accD = xd[3 * trow + 2]; }
         }
-        __syncthreads();
     }
+    __syncthreads();                          /* the exchange buffer is free for the reduction */
     const int pw = *(volatile int *)&s_pw;
     const int pi = pw & 0xffff, np = pw >> 16;
     if (np > 1) {
         const int pcc = *(volatile int *)&s_pc;
         __shared__ int piece_last;
         C *acc = (C *)P.piece_acc;
-        const size_t RM3 = (size_t)3 * P.RM;
+        const size_t RM3 = (size_t)3 * RMA;
         if (half == 0 && i >= 0) {
-            acc[pcc * RM3 + P.RM + trow] = accH;
-            if (SEP) { acc[pcc * RM3 + trow] = accS; acc[pcc * RM3 + 2 * P.RM + trow] = accD; }
+            acc[pcc * RM3 + RMA + trow] = accH;
+            if (SEP) { acc[pcc * RM3 + trow] = accS; acc[pcc * RM3 + 2 * RMA + trow] = accD; }
         }
         __threadfence();
         __syncthreads();
@@ -1380,10 +1659,10 @@ __global__ void __launch_bounds__(256, 3)
             accS = mk<C>(0, 0); accH = accS; accD = accS;
             for (int k = 0; k < np; k++) {
                 const size_t pk = (size_t)(pcc - pi + k) * RM3;
-                accH = cadd(accH, __ldcg(&acc[pk + P.RM + trow]));
+                accH = cadd(accH, __ldcg(&acc[pk + RMA + trow]));
                 if (SEP) {
                     accS = cadd(accS, __ldcg(&acc[pk + trow]));
-                    accD = cadd(accD, __ldcg(&acc[pk + 2 * P.RM + trow]));
+                    accD = cadd(accD, __ldcg(&acc[pk + 2 * RMA + trow]));
                 }
             }
         }
@@ -1392,6 +1671,7 @@ __global__ void __launch_bounds__(256, 3)
     double v[NRED] = {0, 0, 0, 0};
     if (half == 0 && i >= 0) {
         const size_t gi = (size_t)pulse * P.vstride + (size_t)r * B + i;
+        if (dx) accH = cadd(accH, dx[gi]);
         apply_epilogue<C, SEP>(mode, V, gi, accS, accH, accD, v);
     }
     if (red.kind != RED_NONE) reduce_part(red, v, shred, (unsigned)u);
@@ -2209,8 +2489,14 @@ struct gade_solver {
     int asm_part;               /* its partition: 0 plain, 1 balanced */
     int npairs;                 /* (block row, coupled block) pairs */
     int *d_pair_c;
-    double *d_K, *d_A;          /* [table set][pairs][3][W][B], [pulse][pairs][W][B] */
-    size_t asm_kstride;         /* doubles per pulse of K (0: one set shared by all pulses) */
+    int2 *d_K, *d_A;            /* fixed-point limbs of K (per table set) and of A (per pulse), see AsmLay */
+    unsigned short *d_Ke, *d_Ae;   /* row exponents: [table set][pairs][3][Bp], [pulse][pairs][Bp] */
+    int dsym;                   /* the diagonal blocks are symmetric to rounding: the block-LU solves invert them */
+    int halves;                 /* the ELL slots are laid out by column half and spline offset */
+    int APp, RMA;               /* row positions of the assembled layout (Bp of AsmLay), most of one chunk */
+    int *d_pad, *d_off, *d_prow, *d_pq;
+    std::vector<int> h_pad;
+    size_t asm_kstride;         /* values per pulse of K (0: one set shared by all pulses) */
     int *d_pair_par;            /* [pairs] parity of the orders coupling the pair */
     int lpar[2];                /* first order of each parity (-1: none) */
     std::vector<int> h_pair_ptr, h_pair_r, h_pair_par, h_le_ptr, h_le_l, h_le_e;   /* pairs per block row; (order, term) per pair */
@@ -2218,7 +2504,6 @@ struct gade_solver {
     int RMp;                    /* rows per chunk of that layout (RM rounded up to 4) */
     int max_row_pairs;          /* most coupled blocks of one block row */
     size_t a32_stride;          /* floats per pulse of d_A32 */
-    int *d_row_pos;             /* [B] chunk << 16 | row within the chunk */
     PartList part_asm[1];       /* plain: one piece per unit */
     PartList part_asm_bal[9];   /* balanced, by resident CTAs per SM */
     int occ_asm[2][2];          /* resident CTAs per SM [complex64][sep] */
@@ -2418,13 +2703,29 @@ static int set_chunking(gade_solver *s, const gade_setup *su)
         if ((rc = dev_upload(s, &s->d_chunk_acol, ac.data(), ac.size()))) return rc;
     }
     {
-        /* position of every row in the chunk layout (chunk << 16 | row within the chunk) */
-        std::vector<int> pos((size_t)s->B, 0);
-        for (int q = 0; q < s->nchunk; q++)
-            for (int t = 0; t < su->chunk_nrows[q]; t++)
-                pos[su->chunk_rows[(size_t)q * s->RM + t]] = (q << 16) | t;
-        dev_release(s, s->d_row_pos);
-        if ((rc = dev_upload(s, &s->d_row_pos, pos.data(), pos.size()))) return rc;
+        /* row positions of the assembled operator's values (AsmLay) */
+        s->halves = su->ell_halves;
+        std::vector<int> pad(s->nchunk), off(s->nchunk), prow, pq;
+        s->RMA = 0;
+        for (int q = 0; q < s->nchunk; q++) {
+            const int n = su->chunk_nrows[q], n0 = n / 2, n0p = (n0 + 1) & ~1;
+            pad[q] = s->halves ? 2 * n0p : (n + 1) & ~1;
+            off[q] = (int)prow.size();
+            for (int t = 0; t < pad[q]; t++) {
+                /* compact row of the position: halves padded apart */
+                int c = s->halves ? (t < n0p ? (t < n0 ? t : -1) : (t - n0p < n0 ? t - n0p + n0 : -1)) : (t < n ? t : -1);
+                prow.push_back(c < 0 ? -1 : su->chunk_rows[(size_t)q * s->RM + c]);
+                pq.push_back((q << 16) | (c < 0 ? 0xffff : c));
+            }
+            if (pad[q] > s->RMA) s->RMA = pad[q];
+        }
+        s->APp = (int)prow.size();
+        s->h_pad = pad;
+        dev_release(s, s->d_pad); dev_release(s, s->d_off); dev_release(s, s->d_prow); dev_release(s, s->d_pq);
+        if ((rc = dev_upload(s, &s->d_pad, pad.data(), pad.size()))) return rc;
+        if ((rc = dev_upload(s, &s->d_off, off.data(), off.size()))) return rc;
+        if ((rc = dev_upload(s, &s->d_prow, prow.data(), prow.size()))) return rc;
+        if ((rc = dev_upload(s, &s->d_pq, pq.data(), pq.size()))) return rc;
     }
     /* reduction partials: one slot per CTA of a pulse */
     size_t max_cta = (size_t)s->nchunk * s->nblk;
@@ -2534,6 +2835,42 @@ static void pack_factors(const gade_setup *su, int nk, int nch, int bw, int bwp,
     }
 }
 
+/* Whether the diagonal blocks S(k) and i h dt/2 h0(k) are symmetric to
+   rounding, |M_ij - M_ji| <= 8 2^-53 sqrt(|M_ii M_jj|).  The preconditioner
+   holds the exact LU of D^T (tools/superlu.c:142-152), so its solves then
+   also invert D: D (M^-1 p) is p up to the solve's rounding, which is
+   relative to p, a vector of the residual's size, and the FP64 BiCGSTAB
+   products need no diagonal blocks. */
+static int diag_symmetric(const gade_setup *su, int B)
+{
+    const size_t WB = (size_t)su->W * B;
+    std::vector<gc64> row((size_t)B * B), dg(B);
+    for (int m = 0; m < 2; m++) {
+        const gc64 *src = m ? su->Hst_ell : su->S_ell;
+        for (int k = 0; k < su->nk; k++) {
+            const gc64 *M = src + k * WB;
+            for (int i = 0; i < B; i++) dg[i] = gc64{0, 0};
+            for (int j = 0; j < su->W; j++)
+                for (int i = 0; i < B; i++) {
+                    const int c = su->ell_col[(size_t)j * B + i];
+                    if (c < 0) continue;
+                    row[(size_t)i * B + c] = M[(size_t)j * B + i];
+                    if (c == i) dg[i] = M[(size_t)j * B + i];
+                }
+            for (int j = 0; j < su->W; j++)
+                for (int i = 0; i < B; i++) {
+                    const int c = su->ell_col[(size_t)j * B + i];
+                    if (c <= i) continue;      /* every entry above the diagonal against its mirror (symmetric pattern) */
+                    const gc64 a = row[(size_t)i * B + c], b = row[(size_t)c * B + i];
+                    const double lim = 8.0 * 1.1102230246251565e-16 *
+                                       sqrt(hypot(dg[i].re, dg[i].im)) * sqrt(hypot(dg[c].re, dg[c].im));
+                    if (!(fabs(a.re - b.re) <= lim && fabs(a.im - b.im) <= lim)) return 0;
+                }
+        }
+    }
+    return 1;
+}
+
 /*
  * Shared by gade_solver_create (one pulse) and gade_batch_create (npulse
  * pulses on one set of angular tables, h0 and S).  Pulse k has its own time
@@ -2605,6 +2942,10 @@ static int solver_create(const gade_problem *p, int npulse, const double *dts, c
         cudaFuncSetAttribute(k_apply<float, false, true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim);
         cudaFuncSetAttribute(k_apply<float, false, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim);
         cudaFuncSetAttribute(k_apply_asm32, cudaFuncAttributeMaxDynamicSharedMemorySize, lim);
+        cudaFuncSetAttribute(k_apply_asm<true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim);
+        cudaFuncSetAttribute(k_apply_asm<false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim);
+        cudaFuncSetAttribute(k_apply_asm<true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim);
+        cudaFuncSetAttribute(k_apply_asm<false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim);
         cudaFuncSetAttribute(k_apply<dd, true, true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim);
         cudaFuncSetAttribute(k_apply<dd, true, true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim);
     }
@@ -2633,6 +2974,7 @@ static int solver_create(const gade_problem *p, int npulse, const double *dts, c
         for (int k = 0; k < npulse && s->zskip; k++)
             if (!gade_dkb_zero(p, (const gc64 *)(gext + 2 * per * k))) s->zskip = 0;
     }
+    s->dsym = diag_symmetric(su, p->blkdim);
     s->nsm = prop.multiProcessorCount;
     s->nsplit = 1;
     s->upd_block = 256;
@@ -3034,7 +3376,7 @@ static int part_upload(gade_solver *s, PartList &pl, const std::vector<int> &seg
         s->d_piece_acc = nullptr;
         s->piece_cap = 0;
         double2 *acc = nullptr;
-        if ((rc = dev_upload(s, &acc, (const double2 *)nullptr, (size_t)pl.npieces * 3 * s->RM))) return rc;
+        if ((rc = dev_upload(s, &acc, (const double2 *)nullptr, (size_t)pl.npieces * 3 * (s->RM + 2)))) return rc;
         s->d_piece_acc = acc;
         s->piece_cap = (size_t)pl.npieces;
     }
@@ -3186,7 +3528,9 @@ static int asm_partitions(gade_solver *s)
         if ((rc = part_upload(s, s->part_asm[0], seg, pcs))) return rc;
     }
     auto pcost = [&](int q) { return 2.0 * s->h_chunk_nrows[q] * s->W + 2.0 * s->h_chunk_ncols[q]; };
-    auto ufix = [&](int q) { return 4.0 * s->h_chunk_nrows[q] * s->W; };
+    auto ufix = [&](int q) { return ASM_UFIX * s->h_chunk_nrows[q] * s->W; };
+    /* units are cut at multiples of the pairs that k_apply_asm's thread groups take side by side */
+    const int cut = std::max(1, std::min(4, 256 / std::max(1, s->RMA / 2)));
     for (int cls = 0; cls < 4; cls++) {
         const int f = cls / 2, o = s->occ_asm[f][cls % 2];
         if (f == 1 && s->prec != GADE_PREC_MIXED) continue;
@@ -3209,9 +3553,10 @@ static int asm_partitions(gade_solver *s)
             if (a0 == a1) { pcs.push_back(make_int4(u, a0, a0, 0)); pseg.push_back(seg_of(pos + 0.5 * ufix(q))); }
             pos += ufix(q);
             int cur = -1, b0 = a0;
-            for (int a = a0; a < a1; a++) {
-                const int sg = seg_of(pos + 0.5 * pcost(q));
-                pos += pcost(q);
+            for (int a = a0; a < a1; a += cut) {
+                const double c = pcost(q) * std::min(cut, a1 - a);
+                const int sg = seg_of(pos + 0.5 * c);
+                pos += c;
                 if (sg != cur) {
                     if (cur >= 0) { pcs.push_back(make_int4(u, b0, a, 0)); pseg.push_back(cur); }
                     cur = sg;
@@ -3230,10 +3575,10 @@ static int asm_partitions(gade_solver *s)
     return GADE_OK;
 }
 
-static size_t asm_smem_bytes(const gade_solver *s, size_t elem)
+static size_t asm_smem_bytes(const gade_solver *s)
 {
-    unsigned a, b, c;
-    return asm_smem((s->CM + 2) & ~1, s->W, s->RM, 256, (unsigned)elem, &a, &b, &c);
+    unsigned a, b, c, d;
+    return asm_smem(asm_xs(s->RMA, s->CM, s->halves), s->W, s->RMA, s->halves, 256, &a, &b, &c, &d);
 }
 
 /* dynamic shared memory of k_apply_asm32 */
@@ -3241,6 +3586,20 @@ static size_t asm32_smem_bytes(const gade_solver *s)
 {
     unsigned a, b, c, d, e;
     return a32_smem(s->W, (s->RM + 3) & ~3, s->B, 256, s->max_row_pairs, &a, &b, &c, &d, &e);
+}
+
+static AsmLay asm_lay(const gade_solver *s)
+{
+    AsmLay L = {s->d_pad, s->d_off, s->d_prow, s->d_pq, s->APp, s->npairs, s->W, s->RMA};
+    return L;
+}
+
+/* the kernel instance of the assembled operator */
+typedef void (*AsmKernel)(OpP, const double2 *, int, VecP, RedP);
+static AsmKernel asm_kernel(const gade_solver *s, bool sep)
+{
+    if (s->halves) return sep ? k_apply_asm<true, true> : k_apply_asm<false, true>;
+    return sep ? k_apply_asm<true, false> : k_apply_asm<false, false>;
 }
 
 /* Builds K_a for every pulse factor a that some Bessel order uses: the
@@ -3252,8 +3611,7 @@ static int asm_build(gade_solver *s)
     if (!s->rc || s->npairs == 0 || s->asm_ok) return GADE_OK;
     for (int par : s->h_pair_par)
         if (par < 0) return GADE_OK;             /* a pair coupled by both parities: stay matrix-free */
-    const size_t WB = (size_t)s->W * s->B, per = (size_t)s->npairs * WB;
-    if (WB % 2) return GADE_OK;
+    const size_t WB = (size_t)s->W * s->B, per = (size_t)s->npairs * s->W * s->APp;
     s->lpar[0] = s->lmax > 0 ? 0 : -1;
     s->lpar[1] = s->lmax > 1 ? 1 : -1;
     /* K depends only on the radial tables: one set unless the pulses have their own */
@@ -3261,11 +3619,15 @@ static int asm_build(gade_solver *s)
     size_t fr = 0, tot = 0;
     CK(cudaMemGetInfo(&fr, &tot));
     const bool mixed = s->prec == GADE_PREC_MIXED;
-    const double need = (double)per * (24.0 * nset + (mixed ? 12.0 : 8.0) * s->npulse);
+    const size_t rows = (size_t)s->npairs * s->APp;         /* (pair, row) exponents */
+    const double need = (double)per * (24.0 * nset + (mixed ? 12.0 : 8.0) * s->npulse) +
+                        2.0 * rows * (3.0 * nset + s->npulse);
     if (need > 0.5 * (double)fr) return GADE_OK;
     int rc;
-    if ((rc = dev_upload(s, &s->d_K, (const double *)nullptr, per * 3 * nset))) return rc;
-    if ((rc = dev_upload(s, &s->d_A, (const double *)nullptr, per * s->npulse))) return rc;
+    if ((rc = dev_upload(s, &s->d_K, (const int2 *)nullptr, per * 3 * nset))) return rc;
+    if ((rc = dev_upload(s, &s->d_A, (const int2 *)nullptr, per * s->npulse))) return rc;
+    if ((rc = dev_upload(s, &s->d_Ke, (const unsigned short *)nullptr, rows * 3 * nset))) return rc;
+    if ((rc = dev_upload(s, &s->d_Ae, (const unsigned short *)nullptr, rows * s->npulse))) return rc;
     if (mixed) {
         /* chunk-major float copy; padded rows stay zero */
         s->RMp = (s->RM + 3) & ~3;
@@ -3311,10 +3673,10 @@ static int asm_build(gade_solver *s)
             k_tables<true, 1><<<dim3((unsigned)((per_l + 255) / 256), s->lmax, 1), 256, 0, s->stream>>>(T, s->d_coef);
             if (cudaGetLastError() != cudaSuccess) { rc = fail(GADE_ERR_CUDA, "assembled operator: table launch failed"); break; }
         }
-        dim3 grid((unsigned)((WB + 255) / 256), (unsigned)s->npairs);
-        k_build_K<<<grid, 256, 0, s->stream>>>(s->d_K + (size_t)ks * 3 * per,
-                                               (const R4<double>::T *)s->d_M + (size_t)ks * s->mstride, s->nk,
-                                               (int)WB, a, d_pr, s->d_pair_par, s->d_row_kidx, d_lp, d_ll, d_le,
+        dim3 grid((unsigned)((s->APp + 127) / 128), (unsigned)s->npairs);
+        k_build_K<<<grid, 128, 0, s->stream>>>(s->d_K + (size_t)ks * 3 * per, s->d_Ke + (size_t)ks * 3 * rows,
+                                               asm_lay(s), (const R4<double>::T *)s->d_M + (size_t)ks * s->mstride,
+                                               s->nk, s->B, a, d_pr, s->d_pair_par, s->d_row_kidx, d_lp, d_ll, d_le,
                                                (const double *)s->d_ang_a0, (const double *)s->d_ang_a0k,
                                                (const double *)s->d_ang_a1, (const double *)s->d_ang_a1k);
         if (cudaGetLastError() != cudaSuccess) { rc = fail(GADE_ERR_CUDA, "assembled operator: K build launch failed"); break; }
@@ -3327,22 +3689,22 @@ static int asm_build(gade_solver *s)
     for (int f = 0; f < 2; f++)
         for (int sep = 0; sep < 2; sep++) {
             int n = 0;
-            const size_t sm = asm_smem_bytes(s, f ? sizeof(float2) : sizeof(double2));
+            const size_t sm = asm_smem_bytes(s);
             cudaError_t e;
             if (f && sep) { s->occ_asm[f][sep] = 1; continue; }   /* no complex64 instance with S x apart */
             if (f) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_apply_asm32, 256, asm32_smem_bytes(s));
-            else e = sep ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_apply_asm<double, true>, 256, sm)
-                         : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_apply_asm<double, false>, 256, sm);
+            else e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, (const void *)asm_kernel(s, sep), 256, sm);
             if (e != cudaSuccess || n < 1) { cudaGetLastError(); n = 1; }
             s->occ_asm[f][sep] = n > 8 ? 8 : n;
         }
     if ((rc = asm_partitions(s))) return rc;
-    /* costs: 2 FMAs per stored value of the pairs' nonzero slots plus the
-       diagonal blocks (complex, 4 FMAs); the values stream once per apply */
+    /* costs: 2 multiply-adds per stored value of the pairs' nonzero slots
+       (fixed point on the integer units) plus the diagonal blocks (complex,
+       4 FP64 FMAs); the values stream once per apply */
     s->asm_flops = 2.0 * (2.0 * (double)s->npairs * s->blk_nnz + 4.0 * (double)s->nblk * s->blk_nnz);
-    s->asm_bytes = 8.0 * (double)per + 16.0 * (double)s->nk * WB + 4.0 * s->npairs + 48.0 * (double)s->n;
+    s->asm_bytes = 8.0 * (double)per + 2.0 * rows + 16.0 * (double)s->nk * WB + 4.0 * s->npairs + 48.0 * (double)s->n;
     s->asmb_flops = 2.0 * 3.0 * (double)per;
-    s->asmb_bytes = 8.0 * 4.0 * (double)per;
+    s->asmb_bytes = 8.0 * 4.0 * (double)per + 2.0 * 4.0 * rows;
     s->asm_ok = 1;
     return GADE_OK;
 }
@@ -3367,13 +3729,23 @@ static void launch_pdl(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t sme
 /* this step's assembled couplings from d_coef */
 static int launch_assemble(gade_solver *s, cudaStream_t st)
 {
-    const int WB2 = s->W * s->B / 2;
-    const size_t per2 = (size_t)s->npairs * WB2;
     prof_begin(s, st);
-    A32Map F = {(float *)s->d_A32, s->d_row_pos, s->B, s->W, s->RMp, s->npairs, s->a32_stride};
-    k_assemble<<<dim3((unsigned)((WB2 + 255) / 256), (unsigned)s->npairs, (unsigned)s->nslot), 256, 0, st>>>(
-        (double2 *)s->d_A, F, (const double2 *)s->d_K, WB2, s->d_pair_par, s->d_coef,
-        make_int2(s->lpar[0], s->lpar[1]), s->d_plist, per2, s->asm_kstride / 2, s->lmax);
+    A32Map F = {(float *)s->d_A32, s->RMp, s->a32_stride};
+    /* pulses that share K read it together, four to a group */
+    const int pt = s->asm_kstride == 0 && s->nslot > 1 ? 4 : 1;
+    const int ppb = 128 / (s->RMA / 2);                        /* pairs per CTA */
+    const int gy = (s->npairs + ppb - 1) / ppb, gz = (s->nslot + pt - 1) / pt;
+    /* all slots to a thread where the pairs alone give every SM its CTAs (the
+       scaled factors are formed once per row); else five slots, so that small
+       problems are not bound by one thread's chain of loads (19 us at 160
+       pairs of 210 rows with all 30) */
+    const int nsl = (long long)s->nchunk * gy * gz >= 8LL * s->nsm ? s->W : 5, nsg = (s->W + nsl - 1) / nsl;
+    dim3 grid((unsigned)s->nchunk, (unsigned)gy, (unsigned)(gz * nsg));
+#define AS(PT_) k_assemble<PT_><<<grid, 128, 0, st>>>(s->d_A, s->d_Ae, F, s->d_K, s->d_Ke, asm_lay(s), s->d_pair_par, \
+        s->d_coef, make_int2(s->lpar[0], s->lpar[1]), s->d_plist, s->nslot, s->asm_kstride, \
+        s->asm_kstride / s->W, s->lmax, nsl)
+    if (pt == 4) AS(4); else AS(1);
+#undef AS
     prof_end(s, st, 2);
     CKL();
     s->has_time = 1;
@@ -3382,35 +3754,51 @@ static int launch_assemble(gade_solver *s, cudaStream_t st)
 
 static OpP op_params32(const gade_solver *s);
 
-/* the assembled operator in FP64 (x double2) or complex64 (x float2) */
-template <typename R>
-static int launch_apply_asm(gade_solver *s, const typename Cx<R>::T *x, int mode, VecP V, RedP red, cudaStream_t st)
+/* the assembled operator's values, exponents and partition for a launch; returns the segment count */
+static int asm_op_params(const gade_solver *s, OpP &P, bool f32, bool sep, bool plain = false)
 {
-    const bool f32 = sizeof(R) == 4;
-    OpP P = f32 ? op_params32(s) : op_params(s);
     P.A = f32 ? (const void *)s->d_A32 : (const void *)s->d_A;
+    P.Ae = s->d_Ae;
     P.pair_c = s->d_pair_c;
-    P.astride = f32 ? s->a32_stride : (size_t)s->npairs * s->W * s->B;
-    const bool sep = mode == AX_RHS || mode == AX_PARTS || mode == AX_MIX;
-    if (f32 && sep) return fail(GADE_ERR_ARG, "complex64 assembled apply: mode %d has no float instance", mode);
+    P.astride = f32 ? s->a32_stride : (size_t)s->npairs * s->W * s->APp;
+    P.aestride = (size_t)s->npairs * s->APp;
+    P.pad = s->d_pad; P.off = s->d_off; P.prow = s->d_prow;
+    P.Bp = s->APp; P.npairs = s->npairs; P.RMA = s->RMA;
     /* batches run the plain partition (their pulses fill the SMs) */
-    const PartList &pl = (s->asm_part && s->nslot == 1) ? s->part_asm_bal[s->occ_asm[f32][sep]] : s->part_asm[0];
+    const PartList &pl = (s->asm_part && s->nslot == 1 && !plain) ? s->part_asm_bal[s->occ_asm[f32][sep]] : s->part_asm[0];
     P.seg_ptr = pl.d_seg_ptr;
     P.pieces = pl.d_pieces;
-    dim3 grid(s->nslot, pl.nseg);
-    const size_t smem = asm_smem_bytes(s, sizeof(typename Cx<R>::T));
+    return pl.nseg;
+}
+
+/* the assembled operator for FP64 vectors */
+static int launch_apply_asm(gade_solver *s, const double2 *x, int mode, VecP V, RedP red, cudaStream_t st)
+{
+    OpP P = op_params(s);
+    const bool sep = mode == AX_RHS || mode == AX_PARTS || mode == AX_MIX;
+    const int nseg = asm_op_params(s, P, false, sep);
+    dim3 grid(s->nslot, nseg);
+    const size_t smem = asm_smem_bytes(s);
     prof_begin(s, st);
-    /* FP64 with programmatic dependent launch; the complex64 inner solve
-       measured slower with it (4% per mixed step) and launches plainly */
-    if (!f32) {
-        if (sep) launch_pdl(k_apply_asm<R, true>, grid, dim3(256), smem, st, P, x, mode, V, red);
-        else launch_pdl(k_apply_asm<R, false>, grid, dim3(256), smem, st, P, x, mode, V, red);
-    } else {
-        /* the values stream through shared memory by cp.async.bulk */
-        k_apply_asm32<<<grid, 256, asm32_smem_bytes(s), st>>>(P, (const float2 *)x, mode, V, red, s->RMp, s->npairs,
-                                                              s->max_row_pairs);
-    }
-    prof_end(s, st, f32 ? 0 : 0);
+    launch_pdl(asm_kernel(s, sep), grid, dim3(256), smem, st, P, x, mode, V, red);
+    prof_end(s, st, 0);
+    CKL();
+    return GADE_OK;
+}
+
+/* the complex64 assembled operator (values streamed through shared memory by
+   cp.async.bulk); programmatic dependent launch measured slower here (4% per
+   mixed step), so it launches plainly */
+static int launch_apply_asm32(gade_solver *s, const float2 *x, int mode, VecP V, RedP red, cudaStream_t st)
+{
+    if (mode == AX_RHS || mode == AX_PARTS || mode == AX_MIX)
+        return fail(GADE_ERR_ARG, "complex64 assembled apply: mode %d has no float instance", mode);
+    OpP P = op_params32(s);
+    const int nseg = asm_op_params(s, P, true, false);
+    prof_begin(s, st);
+    k_apply_asm32<<<dim3(s->nslot, nseg), 256, asm32_smem_bytes(s), st>>>(P, x, mode, V, red, s->RMp, s->npairs,
+                                                                          s->max_row_pairs);
+    prof_end(s, st, 0);
     CKL();
     return GADE_OK;
 }
@@ -3418,7 +3806,7 @@ static int launch_apply_asm(gade_solver *s, const typename Cx<R>::T *x, int mode
 static int launch_apply(gade_solver *s, const double2 *x, int mode, VecP V, int redkind, cudaStream_t st,
                         int pred = PRED_NONE, DevScal *pb = nullptr)
 {
-    if (s->use_asm) return launch_apply_asm<double>(s, x, mode, V, make_red(s, s->d_sc, redkind, pred, nullptr, pb), st);
+    if (s->use_asm) return launch_apply_asm(s, x, mode, V, make_red(s, s->d_sc, redkind, pred, nullptr, pb), st);
     OpP P = op_params(s);
     RedP red = make_red(s, s->d_sc, redkind, pred, nullptr, pb);
     dim3 grid(s->nslot, op_partition(s, P, false, mode));
@@ -3647,7 +4035,7 @@ static OpP op_params32(const gade_solver *s)
 static int launch_apply32(gade_solver *s, const float2 *x, int mode, VecP V, int redkind, DevScal *sc,
                           int pred = PRED_NONE)
 {
-    if (s->use_asm) return launch_apply_asm<float>(s, x, mode, V, make_red(s, sc, redkind, pred), s->stream);
+    if (s->use_asm) return launch_apply_asm32(s, x, mode, V, make_red(s, sc, redkind, pred), s->stream);
     OpP P = op_params32(s);
     RedP red = make_red(s, sc, redkind, pred);
     dim3 grid(s->nslot, op_partition(s, P, true, mode));
@@ -4177,13 +4565,8 @@ extern "C" int gade_solver_apply_dot_noalloc(gade_solver *s, const void *x_dev, 
     V.in0 = r0_dev;
     if (s->use_asm) {
         /* the assembled operator, one piece per unit */
-        P.A = s->d_A;
-        P.pair_c = s->d_pair_c;
-        P.astride = (size_t)s->npairs * s->W * s->B;
-        P.seg_ptr = s->part_asm[0].d_seg_ptr;
-        P.pieces = s->part_asm[0].d_pieces;
-        k_apply_asm<double, false><<<dim3(1, s->part_asm[0].nseg), 256, asm_smem_bytes(s, sizeof(double2)), st>>>(
-            P, (const double2 *)x_dev, AX_R0V, V, red);
+        const int nseg = asm_op_params(s, P, false, false, true);
+        asm_kernel(s, false)<<<dim3(1, nseg), 256, asm_smem_bytes(s), st>>>(P, (const double2 *)x_dev, AX_R0V, V, red);
         CKL();
         return GADE_OK;
     }
@@ -4247,10 +4630,13 @@ static int batch_seq_iters(gade_batch *b, int K, cudaStream_t st)
     const size_t rsm = sizeof(double) * NRED * s->upd_block;
     for (int it = 0; it < K; it++) {
         if ((rc = launch_precond(s, PC_P, s->r, s->v, s->p, s->y, st, PRED_RUN))) return rc;
-        VecP A1 = {}; A1.out0 = s->v; A1.in0 = s->r0;
+        /* y = M^-1 p with M = D^T = D: the diagonal blocks' part D y of A y is p
+           itself (and D z is s) */
+        const bool dknown = s->dsym && s->use_asm;
+        VecP A1 = {}; A1.out0 = s->v; A1.in0 = s->r0; A1.in1 = dknown ? s->p : nullptr;
         if ((rc = launch_apply(s, s->y, AX_R0V, A1, RED_R0V, st, PRED_RUN))) return rc;
         if ((rc = launch_precond(s, PC_S, s->r, s->v, s->s, s->z, st, PRED_RUN))) return rc;
-        VecP A2 = {}; A2.out0 = s->t; A2.in0 = s->s;
+        VecP A2 = {}; A2.out0 = s->t; A2.in0 = s->s; A2.in1 = dknown ? s->s : nullptr;
         if ((rc = launch_apply(s, s->z, AX_TS, A2, RED_TS, st, PRED_RUN))) return rc;
         RedP red = make_red(s, s->d_sc, RED_UPDATE, PRED_RUN);
         launch_pdl(k_update<double>, dim3(s->upd_grid, s->nslot), dim3(s->upd_block), rsm, st,

@@ -206,8 +206,10 @@ int gade_solver_balanced(const gade_solver *s, int32_t *segments, int32_t *piece
 int gade_solver_set_operator(gade_solver *s, int32_t assembled);
 int gade_solver_operator(const gade_solver *s, int32_t *assembled, float *ms);
 
-/* FP64 flops (2 per FMA) executed by one operator apply and one
- * preconditioner solve, counted exactly from the set-up structure. */
+/* Flops (2 per multiply-add) of one operator apply and one preconditioner
+ * solve, counted exactly from the set-up structure.  The assembled operator
+ * forms its couplings' multiply-adds as fixed-point products on the integer
+ * units (56 x 58 bits, error below FP64's), the rest is FP64. */
 int gade_solver_flops(const gade_solver *s, double *apply_flops, double *precond_flops);
 /* Compulsory DRAM bytes of one FP64 BiCGSTAB operator apply (no reference
  * counterpart).  Matrix-free: the radial-table slabs of the distinct (order,
@@ -216,7 +218,7 @@ int gade_solver_flops(const gade_solver *s, double *apply_flops, double *precond
  * Assembled: the stored coupling values, the diagonal blocks and the
  * vectors. */
 int gade_solver_apply_bytes(const gade_solver *s, double *bytes);
-/* FP64 flops and compulsory DRAM bytes of one step's assembly of the
+/* Flops and compulsory DRAM bytes of one step's assembly of the
  * coupling values (0 with the matrix-free operator); no reference
  * counterpart.  gade_solver_flops and gade_solver_apply_bytes describe the
  * operator in use. */
