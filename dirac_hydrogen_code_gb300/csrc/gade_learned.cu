@@ -24,6 +24,8 @@
 #include <stdio.h>
 #include <math.h>
 
+#include <atomic>
+
 #include "gade.h"
 #include "gade_learned.h"
 
@@ -43,6 +45,19 @@ static int lfail(int code, const char *what, cudaError_t e)
     } while (0)
 
 typedef __nv_bfloat16 bf16;
+
+/* lets a kernel use `bytes` (a constant of the kernel) of dynamic shared
+   memory above the 48 KB default; set once per device */
+template <auto KERN> static cudaError_t l_allow_smem(int bytes)
+{
+    static std::atomic<unsigned long long> done{0};
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess || (dev < 64 && done.load() >> dev & 1ull)) return e;
+    e = cudaFuncSetAttribute(KERN, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    if (e == cudaSuccess && dev < 64) done |= 1ull << dev;
+    return e;
+}
 
 /* ------------------------------------------------------------------ */
 /* GEMM: C = epi(A B + bias) on the 5th-generation tensor cores         */
@@ -72,6 +87,9 @@ typedef __nv_bfloat16 bf16;
  * operand contiguous along K is staged K-major; one contiguous along M or N
  * is staged M/N-major with the descriptor's transpose bit, so no operand is
  * transposed by the SMs.
+ *
+ * k_gemm_cp (8-byte aligned operands with row strides of a multiple of 4):
+ * all threads fill the ring with 8-byte cp.async copies.
  *
  * k_gemm_ld (any strides): the four warps stage each K block with plain
  * loads into two K-major buffers while the tensor core multiplies the
@@ -288,6 +306,126 @@ __global__ void __launch_bounds__(128) k_gemm_tma(const __grid_constant__ CUtens
     if (warp == 0) l_tmem_free(tmem);
 }
 
+/* Copies four neighbouring elements of an operand along its contiguous
+   dimension (K, or M/N when MN; 8-byte aligned) to shared memory without
+   waiting; elements past rows or K arrive as zeros. */
+template <bool MN>
+__device__ __forceinline__ void l_copy4(unsigned dst, const bf16 *__restrict__ P, long long ld, int rows, int K, int r,
+                                        int k)
+{
+    const int o = MN ? k : r, i = MN ? r : k, left = (MN ? rows : K) - i;
+    const int bytes = o < (MN ? K : rows) && left > 0 ? (left < 4 ? 2 * left : 8) : 0;
+    const bf16 *p = bytes ? P + (long long)o * ld + i : P;
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(dst), "l"(p), "r"(bytes) : "memory");
+}
+/* the part of thread tid in vector n of a tile of R rows x 64 (K): rows r and
+   K offset k of its first element.  8 rows x 4 vectors of a row (32 bytes)
+   per warp: whole sectors from memory, two-way bank conflicts into the tile */
+template <bool MN, int R>
+__device__ __forceinline__ void l_vec_pos(int tid, int n, int &r, int &k)
+{
+    const int lane = tid & 31, blk = n * 4 + (tid >> 5);     /* blocks of 8 x 16 elements */
+    if (MN) { k = (blk / (R / 16)) * 8 + (lane >> 2); r = (blk % (R / 16)) * 16 + (lane & 3) * 4; }
+    else { r = (blk / (GTK / 16)) * 8 + (lane >> 2); k = (blk % (GTK / 16)) * 16 + (lane & 3) * 4; }
+}
+
+/*
+ * k_gemm_cp: both operands have a contiguous dimension, 8-byte aligned bases
+ * and row strides that are multiples of 4 elements (rows of K = 1036, say,
+ * which tensor copies do not take).  A ring of CST stages is filled by 8-byte
+ * cp.async copies of all threads, CST - 1 K blocks ahead of the MMAs; an
+ * operand contiguous along M/N is staged M/N-major.  (Staged element by
+ * element with the loads of one block exposed each time, the 512 x 256 x 1036
+ * product took 227 us.)
+ */
+#define CST 6
+template <bool A_MN, bool B_MN>
+__global__ void __launch_bounds__(128) k_gemm_cp(int M, int N, int K, const bf16 *__restrict__ A, long long lda,
+                                                 const bf16 *__restrict__ B, long long ldb,
+                                                 const float *__restrict__ bias, const float *__restrict__ mask,
+                                                 long long ldm, int act, float *__restrict__ C, long long ldc,
+                                                 bf16 *__restrict__ C16, long long ldc16, unsigned spin_limit)
+{
+    extern __shared__ __align__(1024) unsigned char gsm[];   /* [CST][A 128x64 | B 64x64] */
+    __shared__ __align__(8) uint64_t bar[CST];
+    __shared__ unsigned tmem_base;
+    const int tid = threadIdx.x, warp = tid >> 5;
+    const int i0 = blockIdx.y * GTM, j0 = blockIdx.x * GTN;
+    /* element (r, k): K-major (r/8) SBO + (k/8) LBO + (r%8) 16 + (k%8) 2, M/N-major
+       (r/8) SBO + (k/8) LBO + (k%8) 16 + (r%8) 2 */
+    constexpr unsigned LBO = 128, SBO = (GTK / 8) * 128;
+    constexpr int NA = GTM * GTK / 4 / 128, NB = GTN * GTK / 4 / 128;
+    if (warp == 0) l_tmem_alloc(&tmem_base);
+    if (tid == 0) {
+        for (int b = 0; b < CST; b++)
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(l_smem_u32(&bar[b])) : "memory");
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    const unsigned tmem = tmem_base, gbase = l_smem_u32(gsm);
+    const unsigned idesc = l_idesc(A_MN, B_MN);
+    const int nkb = (K + GTK - 1) / GTK;
+    auto fill = [&](int kb) {                  /* one commit group per block, empty past the last */
+        if (kb < nkb) {
+            const unsigned As = gbase + (kb % CST) * GSTAGE, Bs = As + GTM * GTK * 2;
+            int r, k;
+#pragma unroll
+            for (int n = 0; n < NA; n++) {
+                l_vec_pos<A_MN, GTM>(tid, n, r, k);
+                l_copy4<A_MN>(As + (r >> 3) * SBO + (k >> 3) * LBO +
+                                  (A_MN ? (k & 7) * 16 + (r & 7) * 2 : (r & 7) * 16 + (k & 7) * 2),
+                              A, lda, M, K, i0 + r, kb * GTK + k);
+            }
+#pragma unroll
+            for (int n = 0; n < NB; n++) {
+                l_vec_pos<B_MN, GTN>(tid, n, r, k);
+                l_copy4<B_MN>(Bs + (r >> 3) * SBO + (k >> 3) * LBO +
+                                  (B_MN ? (k & 7) * 16 + (r & 7) * 2 : (r & 7) * 16 + (k & 7) * 2),
+                              B, ldb, N, K, j0 + r, kb * GTK + k);
+            }
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    for (int kb = 0; kb < CST - 1; kb++) fill(kb);
+    bool ok = true;
+    int issued = 0;                            /* K blocks whose MMAs were committed */
+    for (int kb = 0; kb < nkb; kb++) {
+        asm volatile("cp.async.wait_group %0;" ::"n"(CST - 2) : "memory");   /* this thread's part of block kb */
+        /* the generic-proxy writes become visible to the tensor core */
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+        /* block kb - 1's MMAs are done with the stage that block kb + CST - 1 takes */
+        if (kb > 0) ok = l_wait(&bar[(kb - 1) % CST], ((kb - 1) / CST) & 1, spin_limit, nullptr);
+        if (__syncthreads_or(!ok)) { ok = false; break; }
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        if (tid == 0) {
+            const unsigned As = gbase + (kb % CST) * GSTAGE, Bs = As + GTM * GTK * 2;
+            for (int kk = 0; kk < GTK / 16; kk++)
+                l_mma(tmem, l_sdesc(As + kk * 2 * LBO, LBO, SBO), l_sdesc(Bs + kk * 2 * LBO, LBO, SBO), idesc,
+                      (kb > 0 || kk > 0) ? 1u : 0u);
+            l_commit(&bar[kb % CST]);
+        }
+        issued = kb + 1;
+        fill(kb + CST - 1);
+    }
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    /* the last commit covers every MMA issued before it */
+    if (ok && issued > 0) ok = l_wait(&bar[(issued - 1) % CST], ((issued - 1) / CST) & 1, spin_limit, nullptr);
+    ok = !__syncthreads_or(!ok);
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    if (ok) {
+        l_epilogue(tmem, issued > 0, M, N, i0, j0, bias, mask, ldm, act, C, ldc, C16, ldc16);
+    } else if (tid == 0) {
+        atomicOr(&g_learned_err, 1u);
+        if (issued > 0) l_wait(&bar[(issued - 1) % CST], ((issued - 1) / CST) & 1, GDRAIN, nullptr);
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    if (warp == 0) l_tmem_free(tmem);
+}
+
 __global__ void __launch_bounds__(128) k_gemm_ld(int M, int N, int K, const bf16 *__restrict__ A, long long sa0,
                                                  long long sa1, const bf16 *__restrict__ B, long long sb0,
                                                  long long sb1, const float *__restrict__ bias,
@@ -405,17 +543,22 @@ static cudaError_t launch_gemm_tma(dim3 grid, cudaStream_t st, const CUtensorMap
                                    int N, int K, const float *bias, const float *mask, long long ldm, int act,
                                    float *C, long long ldc, bf16 *C16, long long ldc16)
 {
-    static unsigned long long smem_set = 0;   /* per device: GST x 24 KB is above the 48 KB default */
-    int dev = 0;
-    cudaError_t e = cudaGetDevice(&dev);
+    const cudaError_t e = l_allow_smem<k_gemm_tma<A_MN, B_MN>>(GST * GSTAGE);
     if (e != cudaSuccess) return e;
-    if (dev >= 64 || !(smem_set >> dev & 1ull)) {
-        e = cudaFuncSetAttribute(k_gemm_tma<A_MN, B_MN>, cudaFuncAttributeMaxDynamicSharedMemorySize, GST * GSTAGE);
-        if (e != cudaSuccess) return e;
-        if (dev < 64) smem_set |= 1ull << dev;
-    }
     k_gemm_tma<A_MN, B_MN><<<grid, 128, GST * GSTAGE, st>>>(ma, mb, M, N, K, bias, mask, ldm, act, C, ldc, C16,
                                                            ldc16, g_gemm_spin, g_gemm_withhold);
+    return cudaGetLastError();
+}
+
+template <bool A_MN, bool B_MN>
+static cudaError_t launch_gemm_cp(dim3 grid, cudaStream_t st, int M, int N, int K, const bf16 *A, long long lda,
+                                  const bf16 *B, long long ldb, const float *bias, const float *mask, long long ldm,
+                                  int act, float *C, long long ldc, bf16 *C16, long long ldc16)
+{
+    const cudaError_t e = l_allow_smem<k_gemm_cp<A_MN, B_MN>>(CST * GSTAGE);
+    if (e != cudaSuccess) return e;
+    k_gemm_cp<A_MN, B_MN><<<grid, 128, CST * GSTAGE, st>>>(M, N, K, A, lda, B, ldb, bias, mask, ldm, act, C, ldc, C16,
+                                                          ldc16, g_gemm_spin);
     return cudaGetLastError();
 }
 
@@ -452,18 +595,26 @@ extern "C" int gade_gemm_bf16(int32_t M, int32_t N, int32_t K, const void *A, in
             return GADE_OK;
         }
     }
-    static unsigned long long smem_set = 0;   /* per device: 2 x 24 KB is above the 48 KB default */
-    int dev = 0;
-    cudaError_t e = cudaGetDevice(&dev);
-    if (e != cudaSuccess) return lfail(GADE_ERR_CUDA, "gade_gemm_bf16", e);
-    if (dev >= 64 || !(smem_set >> dev & 1ull)) {
-        e = cudaFuncSetAttribute(k_gemm_ld, cudaFuncAttributeMaxDynamicSharedMemorySize, 2 * GSTAGE);
-        if (e != cudaSuccess) return lfail(GADE_ERR_CUDA, "gade_gemm_bf16", e);
-        if (dev < 64) smem_set |= 1ull << dev;
+    cudaError_t e;
+    const bf16 *Ab = (const bf16 *)A, *Bb = (const bf16 *)B;
+    /* 8-byte asynchronous copies where both operands allow them, else plain loads */
+    auto cp_ok = [](const void *p, long long s0, long long s1) {
+        return ((uintptr_t)p & 7) == 0 && (s0 == 1 || s1 == 1) && (s1 == 1 ? s0 : s1) % 4 == 0;
+    };
+    if (K > 0 && cp_ok(A, sa0, sa1) && cp_ok(B, sb1, sb0)) {
+        const bool a_mn = sa1 != 1, b_mn = sb0 != 1;
+        const long long lda = a_mn ? sa1 : sa0, ldb = b_mn ? sb0 : sb1;
+#define GCP(A_, B_) launch_gemm_cp<A_, B_>(grid, st, M, N, K, Ab, lda, Bb, ldb, bias, mask, ldm, act, C, ldc, (bf16 *)C16, ldc16)
+        e = a_mn ? (b_mn ? GCP(true, true) : GCP(true, false)) : (b_mn ? GCP(false, true) : GCP(false, false));
+#undef GCP
+    } else {
+        if ((e = l_allow_smem<k_gemm_ld>(2 * GSTAGE)) != cudaSuccess)
+            return lfail(GADE_ERR_CUDA, "gade_gemm_bf16", e);
+        k_gemm_ld<<<grid, 128, 2 * GSTAGE, st>>>(M, N, K, Ab, sa0, sa1, Bb, sb0, sb1, bias, mask, ldm, act, C, ldc,
+                                                 (bf16 *)C16, ldc16, g_gemm_spin);
+        e = cudaGetLastError();
     }
-    k_gemm_ld<<<grid, 128, 2 * GSTAGE, st>>>(M, N, K, (const bf16 *)A, sa0, sa1, (const bf16 *)B, sb0, sb1, bias,
-                                             mask, ldm, act, C, ldc, (bf16 *)C16, ldc16, g_gemm_spin);
-    LCK("gade_gemm_bf16");
+    if (e != cudaSuccess) return lfail(GADE_ERR_CUDA, "gade_gemm_bf16", e);
     return GADE_OK;
 }
 
@@ -539,20 +690,32 @@ extern "C" int gade_mse_grad(int32_t M, int32_t N, const float *out, const float
     return GADE_OK;
 }
 
-/* db[j] = sum_i G(i, j) in fixed order */
-__global__ void k_colsum(int M, int N, const float *__restrict__ G, long long ldg, float *__restrict__ db)
+/* db[j] = sum_i G(i, j) in a fixed order: a CTA takes 32 columns, its 16 warps
+   every 16th row, and the warps' sums are added in order (one thread per
+   column walking all rows took 32 us at 512 x 256) */
+__global__ void __launch_bounds__(512) k_colsum(int M, int N, const float *__restrict__ G, long long ldg,
+                                                float *__restrict__ db)
 {
-    const int j = blockIdx.x * blockDim.x + threadIdx.x;
-    if (j >= N) return;
+    __shared__ float sh[16][32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, j = blockIdx.x * 32 + lane;
     float s = 0.f;
-    for (int i = 0; i < M; i++) s += G[(size_t)i * ldg + j];
-    db[j] = s;
+    if (j < N) {
+#pragma unroll 8
+        for (int i = warp; i < M; i += 16) s += G[(size_t)i * ldg + j];
+    }
+    sh[warp][lane] = s;
+    __syncthreads();
+    if (warp == 0 && j < N) {
+        s = sh[0][lane];
+        for (int w = 1; w < 16; w++) s += sh[w][lane];
+        db[j] = s;
+    }
 }
 
 extern "C" int gade_colsum(int32_t M, int32_t N, const float *G, int64_t ldg, float *db, void *stream)
 {
     if (M < 0 || N <= 0 || !G || !db) return gade_set_error(GADE_ERR_ARG, "gade_colsum: bad argument");
-    k_colsum<<<(N + 255) / 256, 256, 0, (cudaStream_t)stream>>>(M, N, G, ldg, db);
+    k_colsum<<<(N + 31) / 32, 512, 0, (cudaStream_t)stream>>>(M, N, G, ldg, db);
     LCK("gade_colsum");
     return GADE_OK;
 }
@@ -628,40 +791,113 @@ __device__ __forceinline__ float l_f32_bits(double v)
     return __uint_as_float(sign | ((unsigned)e8 << 23) | mant);
 }
 
-/* partial projections of one 1024-element chunk of one pulse's state: the
-   network's BF16 inputs need no more than FP32 products and per-chunk FP32
-   sums (relative error ~1e-7); chunks are added in FP64 in a fixed order */
-__global__ void __launch_bounds__(256) k_pod_partial(int n, int R, const float2 *__restrict__ U,
-                                                     const double2 *__restrict__ x, long long ldx,
-                                                     double2 *__restrict__ part, int npulse)
+/* partial projections of one 1024-element chunk of up to PJ_P pulses' states:
+   the network's BF16 inputs need no more than FP32 products and per-chunk FP32
+   sums (relative error ~1e-7); chunks are added in FP64 in a fixed order.
+   The basis is the traffic (8 n R bytes), so a CTA takes the chunk for all
+   pulses of its tile and reads each basis entry once; a warp takes four basis
+   rows at a time, so that a state value read from shared memory serves four.
+   n = 244,000, R = 128, 8 pulses: 158 us with one pulse per CTA, 92 us now
+   (2.7 TB/s of basis; FP32 and shared-memory issue bind). */
+#define PJ_P 8
+#define PJ_R 4
+#define PJ_ROWS 128    /* basis rows per CTA (32: 106 us, 64: 98 us, 128: 92 us) */
+template <int NP>
+__global__ void __launch_bounds__(256, 2) k_pod_partial(int n, int R, const float2 *__restrict__ U,
+                                                        const double2 *__restrict__ x, long long ldx,
+                                                        double2 *__restrict__ part, int npulse, int rows)
 {
-    __shared__ float2 xs[PJ_L];
-    const int p = blockIdx.x, ch = blockIdx.y;
+    extern __shared__ __align__(16) float2 xsf[];    /* [NP/2][PJ_L][2]: two pulses of an element side by side */
+    const int ch = blockIdx.x, p0 = blockIdx.y * PJ_P;
+    const int np = npulse - p0 < NP ? npulse - p0 : NP;
     const int i0 = ch * PJ_L;
     const int len = n - i0 < PJ_L ? n - i0 : PJ_L;
-    const double2 *xp = x + (size_t)p * ldx + i0;
     for (int e = threadIdx.x; e < len; e += 256) {
-        const double2 v = xp[e];
-        xs[e] = make_float2(l_f32_bits(v.x), l_f32_bits(v.y));
+        double2 v[NP];
+#pragma unroll
+        for (int p = 0; p < NP; p++)
+            v[p] = p < np ? x[(size_t)(p0 + p) * ldx + i0 + e] : make_double2(0.0, 0.0);
+#pragma unroll
+        for (int p = 0; p < NP; p++)
+            xsf[NP == 1 ? e : (p >> 1) * 2 * PJ_L + 2 * e + (p & 1)] = make_float2(l_f32_bits(v[p].x), l_f32_bits(v[p].y));
     }
     __syncthreads();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    for (int r = warp; r < R; r += 8) {
+    const int re = min(R, (int)(blockIdx.z + 1) * rows);
+    for (int r = blockIdx.z * rows + warp * PJ_R; r < re; r += 8 * PJ_R) {
         const float2 *u = U + (size_t)r * n + i0;
-        float sr = 0.f, si = 0.f;
+        const int nr = R - r < PJ_R ? R - r : PJ_R;
+        float sr[PJ_R][NP], si[PJ_R][NP];
+#pragma unroll
+        for (int a = 0; a < PJ_R; a++)
+#pragma unroll
+            for (int p = 0; p < NP; p++) { sr[a][p] = 0.f; si[a][p] = 0.f; }
+#pragma unroll 4
         for (int e = lane; e < len; e += 32) {
-            const float2 uv = u[e];
-            const float2 xv = xs[e];
-            sr = fmaf(uv.x, xv.x, fmaf(uv.y, xv.y, sr));      /* conj(u) x */
-            si = fmaf(uv.x, xv.y, fmaf(-uv.y, xv.x, si));
+            float2 uv[PJ_R], xv[NP];
+#pragma unroll
+            for (int a = 0; a < PJ_R; a++) uv[a] = a < nr ? __ldcs(&u[(size_t)a * n + e]) : make_float2(0.f, 0.f);
+            if constexpr (NP == 1) {
+                xv[0] = xsf[e];
+            } else {
+#pragma unroll
+                for (int p = 0; p < NP; p += 2) {
+                    const float4 q = *(const float4 *)(xsf + (p >> 1) * 2 * PJ_L + 2 * e);
+                    xv[p] = make_float2(q.x, q.y);
+                    xv[p + 1] = make_float2(q.z, q.w);
+                }
+            }
+#pragma unroll
+            for (int p = 0; p < NP; p++)
+#pragma unroll
+                for (int a = 0; a < PJ_R; a++) {
+                    sr[a][p] = fmaf(uv[a].x, xv[p].x, fmaf(uv[a].y, xv[p].y, sr[a][p]));      /* conj(u) x */
+                    si[a][p] = fmaf(uv[a].x, xv[p].y, fmaf(-uv[a].y, xv[p].x, si[a][p]));
+                }
         }
+        /* sums over the lanes (xor 16, 8, .. 1), the values split over the lanes
+           on the way, so that each lane ends with the (re, im) of its own
+           (pulse, row) and converts and stores only that */
+        float v[NP * PJ_R * 2];
+#pragma unroll
+        for (int p = 0; p < NP; p++)
+#pragma unroll
+            for (int a = 0; a < PJ_R; a++) { v[(p * PJ_R + a) * 2] = sr[a][p]; v[(p * PJ_R + a) * 2 + 1] = si[a][p]; }
+        int nv = NP * PJ_R * 2;
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) {
-            sr += __shfl_xor_sync(0xffffffffu, sr, o);
-            si += __shfl_xor_sync(0xffffffffu, si, o);
+            const bool up = lane & o;
+            if (nv > 2) {
+                nv >>= 1;
+#pragma unroll
+                for (int j = 0; j < NP * PJ_R; j++)
+                    if (j < nv) {
+                        const float got = __shfl_xor_sync(0xffffffffu, up ? v[j] : v[j + nv], o);
+                        v[j] = (up ? v[j + nv] : v[j]) + got;
+                    }
+            } else {
+                v[0] += __shfl_xor_sync(0xffffffffu, v[0], o);
+                v[1] += __shfl_xor_sync(0xffffffffu, v[1], o);
+            }
         }
-        if (lane == 0) part[((size_t)ch * npulse + p) * R + r] = make_double2(sr, si);
+        constexpr int LPV = 32 / (NP * PJ_R);           /* lanes that hold the same value */
+        const int q = lane / LPV, p = q / PJ_R, a = q - p * PJ_R;
+        if (lane % LPV == 0 && a < nr && p < np)
+            part[((size_t)ch * npulse + p0 + p) * R + r + a] = make_double2(v[0], v[1]);
     }
+}
+
+template <int NP>
+static cudaError_t launch_pod_partial(int n, int R, const float2 *U, const double2 *x, long long ldx, double2 *part,
+                                      int npulse, int nch, cudaStream_t st)
+{
+    const size_t smem = sizeof(float2) * PJ_L * NP;
+    cudaError_t e = l_allow_smem<k_pod_partial<NP>>((int)smem);
+    if (e != cudaSuccess) return e;
+    const int rows = PJ_ROWS;
+    k_pod_partial<NP><<<dim3(nch, (npulse + PJ_P - 1) / PJ_P, (R + rows - 1) / rows), 256, smem, st>>>(
+        n, R, U, x, ldx, part, npulse, rows);
+    return cudaGetLastError();
 }
 
 /* the same partial projections with FP64 products and sums (training
@@ -696,16 +932,28 @@ __global__ void __launch_bounds__(256) k_pod_partial64(int n, int R, const float
     }
 }
 
-__global__ void k_pod_sum(int nch, int npulse, int R, const double2 *__restrict__ part, double2 *__restrict__ coef)
+/* coef = sum of the chunks' partials in a fixed order: 32 coefficients per CTA,
+   every 8th chunk per warp, the warps' sums in order (one thread per
+   coefficient walking all chunks took 63 us at 239 chunks x 1024) */
+__global__ void __launch_bounds__(256) k_pod_sum(int nch, int total, const double2 *__restrict__ part,
+                                                 double2 *__restrict__ coef)
 {
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= npulse * R) return;
+    __shared__ double2 sh[8][32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, t = blockIdx.x * 32 + lane;
     double sr = 0, si = 0;
-    for (int c = 0; c < nch; c++) {
-        const double2 v = part[(size_t)c * npulse * R + t];
-        sr += v.x; si += v.y;
+    if (t < total) {
+#pragma unroll 8
+        for (int c = warp; c < nch; c += 8) {
+            const double2 v = part[(size_t)c * total + t];
+            sr += v.x; si += v.y;
+        }
     }
-    coef[t] = make_double2(sr, si);
+    sh[warp][lane] = make_double2(sr, si);
+    __syncthreads();
+    if (warp == 0 && t < total) {
+        for (int w = 1; w < 8; w++) { sr += sh[w][lane].x; si += sh[w][lane].y; }
+        coef[t] = make_double2(sr, si);
+    }
 }
 
 static int pod_project(bool fp64, int64_t n, int32_t R, const void *U, const void *x, int64_t ldx, int32_t npulse,
@@ -720,11 +968,18 @@ static int pod_project(bool fp64, int64_t n, int32_t R, const void *U, const voi
     if (fp64)
         k_pod_partial64<<<dim3(npulse, nch), 256, 0, st>>>((int)n, R, (const float2 *)U, (const double2 *)x, ldx,
                                                            (double2 *)scratch, npulse);
-    else
-        k_pod_partial<<<dim3(npulse, nch), 256, 0, st>>>((int)n, R, (const float2 *)U, (const double2 *)x, ldx,
-                                                         (double2 *)scratch, npulse);
+    else {
+        cudaError_t e;
+#define PPL(NP_) launch_pod_partial<NP_>((int)n, R, (const float2 *)U, (const double2 *)x, ldx, (double2 *)scratch, npulse, nch, st)
+        if (npulse == 1) e = PPL(1);
+        else if (npulse == 2) e = PPL(2);
+        else if (npulse <= 4) e = PPL(4);
+        else e = PPL(8);
+#undef PPL
+        if (e != cudaSuccess) return lfail(GADE_ERR_CUDA, "gade_pod_project", e);
+    }
     LCK("gade_pod_project");
-    k_pod_sum<<<(npulse * R + 255) / 256, 256, 0, st>>>(nch, npulse, R, (const double2 *)scratch, (double2 *)coef);
+    k_pod_sum<<<(npulse * R + 31) / 32, 256, 0, st>>>(nch, npulse * R, (const double2 *)scratch, (double2 *)coef);
     LCK("gade_pod_project");
     return GADE_OK;
 }
@@ -751,32 +1006,54 @@ extern "C" int64_t gade_pod_project_scratch(int64_t n, int32_t R, int32_t npulse
  * thread per i walks the basis rows, so U is read once per launch for all
  * the pulses of the block's tile. */
 #define EX_PT 8
-__global__ void __launch_bounds__(256) k_pod_expand(int n, int R, const float2 *__restrict__ U,
+#define EX_UR 4    /* basis rows loaded ahead (with them 71 us at n = 244,000, R = 128, 8 pulses; one at a time 198 us) */
+__global__ void __launch_bounds__(256, 4) k_pod_expand(int n, int R, const float2 *__restrict__ U,
                                                     const float2 *__restrict__ c, const float *__restrict__ scale,
                                                     int npulse, double2 *__restrict__ y, long long ldy)
 {
-    extern __shared__ float2 cs[];                   /* [EX_PT][R] */
+    extern __shared__ __align__(16) float2 cs[];     /* [R rounded up to EX_UR][EX_PT]: one entry's pulses side by side */
     const int p0 = blockIdx.y * EX_PT;
     const int np = npulse - p0 < EX_PT ? npulse - p0 : EX_PT;
-    for (int e = threadIdx.x; e < np * R; e += blockDim.x) {
-        const int pp = e / R, r = e % R;
-        const float s = scale ? scale[p0 + pp] : 1.f;
-        const float2 v = c[(size_t)(p0 + pp) * R + r];
-        cs[pp * R + r] = make_float2(s * v.x, s * v.y);
+    const int Rp = (R + EX_UR - 1) / EX_UR * EX_UR;
+    for (int e = threadIdx.x; e < Rp * EX_PT; e += blockDim.x) {
+        const int pp = e / Rp, r = e % Rp;
+        float2 v = make_float2(0.f, 0.f);
+        if (pp < np && r < R) {
+            const float s = scale ? scale[p0 + pp] : 1.f;
+            v = c[(size_t)(p0 + pp) * R + r];
+            v = make_float2(s * v.x, s * v.y);
+        }
+        cs[r * EX_PT + pp] = v;
     }
     __syncthreads();
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+    for (int i = blockIdx.x * 256 + threadIdx.x; i < n; i += gridDim.x * 256) {
         float ar[EX_PT], ai[EX_PT];
 #pragma unroll
         for (int pp = 0; pp < EX_PT; pp++) { ar[pp] = 0.f; ai[pp] = 0.f; }
-        for (int r = 0; r < R; r++) {
-            const float2 u = U[(size_t)r * n + i];
+        /* the next EX_UR basis entries are loaded while these are used; the
+           coefficients of the pulses past the tile's end are zero */
+        float2 nx[EX_UR];
+        auto load = [&](int r0) {
 #pragma unroll
-            for (int pp = 0; pp < EX_PT; pp++) {
-                if (pp < np) {
-                    const float2 cv = cs[pp * R + r];
-                    ar[pp] = fmaf(u.x, cv.x, fmaf(-u.y, cv.y, ar[pp]));
-                    ai[pp] = fmaf(u.x, cv.y, fmaf(u.y, cv.x, ai[pp]));
+            for (int a = 0; a < EX_UR; a++)
+                nx[a] = r0 + a < R ? __ldcs(&U[(size_t)(r0 + a) * n + i]) : make_float2(0.f, 0.f);
+        };
+        load(0);
+        for (int r0 = 0; r0 < R; r0 += EX_UR) {
+            float2 u[EX_UR];
+#pragma unroll
+            for (int a = 0; a < EX_UR; a++) u[a] = nx[a];
+            load(r0 + EX_UR);
+#pragma unroll
+            for (int a = 0; a < EX_UR; a++) {
+                const float4 *c4 = (const float4 *)(cs + (r0 + a) * EX_PT);
+#pragma unroll
+                for (int h = 0; h < EX_PT / 2; h++) {
+                    const float4 cv = c4[h];
+                    ar[2 * h] = fmaf(u[a].x, cv.x, fmaf(-u[a].y, cv.y, ar[2 * h]));
+                    ai[2 * h] = fmaf(u[a].x, cv.y, fmaf(u[a].y, cv.x, ai[2 * h]));
+                    ar[2 * h + 1] = fmaf(u[a].x, cv.z, fmaf(-u[a].y, cv.w, ar[2 * h + 1]));
+                    ai[2 * h + 1] = fmaf(u[a].x, cv.w, fmaf(u[a].y, cv.z, ai[2 * h + 1]));
                 }
             }
         }
@@ -793,7 +1070,9 @@ extern "C" int gade_pod_expand(int64_t n, int32_t R, const void *U, const void *
         return gade_set_error(GADE_ERR_ARG, "gade_pod_expand: bad argument");
     int gx = (int)((n + 255) / 256);
     if (gx > 1216) gx = 1216;
-    const size_t smem = sizeof(float2) * EX_PT * (size_t)R;
+    const size_t smem = sizeof(float2) * EX_PT * (size_t)((R + EX_UR - 1) / EX_UR * EX_UR);
+    cudaError_t e = l_allow_smem<k_pod_expand>(sizeof(float2) * EX_PT * 1024);
+    if (e != cudaSuccess) return lfail(GADE_ERR_CUDA, "gade_pod_expand", e);
     k_pod_expand<<<dim3(gx, (npulse + EX_PT - 1) / EX_PT), 256, smem, (cudaStream_t)stream>>>(
         (int)n, R, (const float2 *)U, (const float2 *)c, scale, npulse, (double2 *)y, ldy);
     LCK("gade_pod_expand");

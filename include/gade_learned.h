@@ -30,18 +30,19 @@ extern "C" {
  * 1 ReLU.  C (FP32, row stride ldc) and C16 (BF16, row stride ldc16) may
  * each be NULL, not both.  Operands that are 16-byte aligned, unit-stride
  * along one dimension and with a row stride of a multiple of 8 elements are
- * staged by tensor copies (TMA); others by plain loads.  Both stagings give
- * the same bits. */
+ * staged by tensor copies (TMA); others by asynchronous 8-byte copies where
+ * their alignment allows it, else by plain loads.  Every staging gives the
+ * same bits. */
 int gade_gemm_bf16(int32_t M, int32_t N, int32_t K, const void *A, int64_t sa0, int64_t sa1,
                    const void *B, int64_t sb0, int64_t sb1, const float *bias, const float *mask,
                    int64_t ldm, int32_t act, float *C, int64_t ldc, void *C16, int64_t ldc16, void *stream);
 
 /* 1 when gade_gemm_bf16 with these operands stages them by tensor copies,
- * 0 when by plain loads (host only, no GPU work). */
+ * 0 when otherwise (host only, no GPU work). */
 int gade_gemm_bf16_path(int32_t M, int32_t N, int32_t K, const void *A, int64_t sa0, int64_t sa1,
                         const void *B, int64_t sb0, int64_t sb1);
 
-/* Process-wide GEMM options (tests): path 0 automatic, 1 plain loads only;
+/* Process-wide GEMM options (tests): path 0 automatic, 1 no tensor copies;
  * wait_limit = mbarrier polls before a CTA gives up (0: the default, ~2^24);
  * withhold_copies = 1 makes the tensor-copy stager issue nothing, so that
  * the MMA thread's wait runs out and the status word is set. */

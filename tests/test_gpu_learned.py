@@ -261,3 +261,57 @@ def test_fused_guess_step_matches_separate_calls(workdirs, native_lib):
         assert np.array_equal(ca, cb)
     assert np.any(sa[-1][1] != 0)
     assert np.array_equal(xa, xb)
+
+
+# K past the copy ring's depth with a remainder, partial 8-byte vectors at the
+# end of a row, operands offset from the row stride: every transposition
+@pytest.mark.parametrize("M_,N_,K_,ld", [(130, 70, 1034, 1036), (8, 256, 1036, 1036), (17, 65, 389, 396)])
+@pytest.mark.parametrize("ta,tb", [(False, False), (True, False), (False, True), (True, True)])
+def test_gemm_async_copy_staging(native_lib, M_, N_, K_, ld, ta, tb):
+    """Operands whose row strides are multiples of 4 but not 8 elements (no
+    tensor copies): relative error <= 1e-5 against float64 products, FP32
+    accumulation of K ~ 1000 products of BF16 values rounding to ~1e-6."""
+    rng = np.random.default_rng(M_ + K_)
+    A, B = M.bf16(rng.standard_normal((M_, K_))), M.bf16(rng.standard_normal((K_, N_)))
+
+    def padded(x, stride):
+        buf = np.full((x.shape[0], stride), 7.0)
+        buf[:, :x.shape[1]] = x
+        return _bf(buf)
+    lda = (M_ + 3) // 4 * 4 + (4 if (M_ + 3) // 4 % 2 else 0) if ta else ld
+    lda += 4 if ta and lda % 8 == 0 else 0
+    ldb = ld if tb else (N_ + 3) // 4 * 4 + 4
+    Ad, Bd = padded(A.T if ta else A, lda), padded(B.T if tb else B, ldb)
+    sa, sb = ((1, lda) if ta else (lda, 1)), ((1, ldb) if tb else (ldb, 1))
+    C = torch.empty(M_, N_, device="cuda")
+    native.call("gade_gemm_bf16", M_, N_, K_, Ad.data_ptr(), *sa, Bd.data_ptr(), *sb, None, None, 0, 0,
+                C.data_ptr(), N_, None, 0, 0)
+    torch.cuda.synchronize()
+    assert _rel(C.cpu().numpy().astype(np.float64), A @ B) <= 1e-5
+    assert _status() == 0
+
+
+@pytest.mark.parametrize("n", [1, 1023, 1024, 1025, 5000])
+@pytest.mark.parametrize("R,P", [(1, 1), (5, 2), (33, 3), (128, 9), (130, 17)])
+def test_pod_tiles(native_lib, n, R, P):
+    """Projection and expansion at the edges of their chunk, row and pulse
+    tiles: projection <= 1e-6 of |U||x| (FP32 products), expansion <= 1e-6."""
+    rng = np.random.default_rng(n + R + P)
+    U = (rng.standard_normal((R, n)) + 1j * rng.standard_normal((R, n))).astype(np.complex64)
+    x = rng.standard_normal((P, n)) + 1j * rng.standard_normal((P, n))
+    Ud, xd = torch.from_numpy(U).cuda(), torch.from_numpy(x).cuda()
+    sb = native.call("gade_pod_project_scratch", n, R, P)
+    scratch = torch.empty(sb, dtype=torch.uint8, device="cuda")
+    coef = torch.empty(P, R, dtype=torch.complex128, device="cuda")
+    U64 = U.astype(np.complex128)
+    big = np.abs(x) @ np.abs(U64).T
+    for fn, tol in (("gade_pod_project", 1e-6), ("gade_pod_project_fp64", 1e-14)):
+        native.call(fn, n, R, Ud.data_ptr(), xd.data_ptr(), n, P, coef.data_ptr(), scratch.data_ptr(), sb, 0)
+        torch.cuda.synchronize()
+        assert np.all(np.abs(coef.cpu().numpy() - x @ U64.conj().T) <= tol * big)
+    c = (rng.standard_normal((P, R)) + 1j * rng.standard_normal((P, R))).astype(np.complex64)
+    y = torch.empty(P, n, dtype=torch.complex128, device="cuda")
+    native.call("gade_pod_expand", n, R, Ud.data_ptr(), torch.from_numpy(c).cuda().data_ptr(), None, P, y.data_ptr(), n, 0)
+    torch.cuda.synchronize()
+    c64 = c.astype(np.complex128)
+    assert np.all(np.abs(y.cpu().numpy() - c64 @ U64) <= 2e-6 * (np.abs(c64) @ np.abs(U64)))
