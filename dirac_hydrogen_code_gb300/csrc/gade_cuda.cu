@@ -41,6 +41,7 @@
 #include <vector>
 
 #include "gade_internal.h"
+#include "gade_fx.cuh"
 #include "../../include/gade.h"
 
 #define SOL 137.035999084
@@ -1096,69 +1097,6 @@ __global__ void __launch_bounds__(256, std::is_same<R, dd>::value ? GADE_DD_MINB
 
 
 /* ------------------------------------------------------------------ */
-/* fixed-point products of FP64 values on the integer units             */
-/* ------------------------------------------------------------------ */
-/*
- * GB300 retires 2 DFMA per clock and SM but 32 32x32+64-bit integer
- * multiply-adds (measured: 1.6 against 24 per nominal clock), so the long
- * real x real sums of the assembled operator run there.  A vector of FP64
- * values that share a power of two is held as integers N, value = N 2^e:
- *   coupling values   |N| <= 2^56, one e per (pair, row)      (FX_UPA = 3)
- *   vector entries    |N| <  2^58, one e per staged window    (FX_UPX = 5)
- * each in two signed limbs, N = hi 2^29 + lo, |lo| <= 2^28.  A product is
- * hi hi 2^58 + (hi lo + lo hi) 2^29, three multiply-adds into two 64-bit
- * sums (the lo lo term, below 2^-56 of the largest product, is left out);
- * sums of up to 30 products stay below 2^63 and are exact.  A 53-bit
- * mantissa is held in full down to 2^-3 (2^-5 for vector entries) of its
- * group's largest value and rounded below that at 2^-56 (2^-58) of it, so a
- * row's sum carries an error of about 2^-56 of its largest terms once,
- * where FP64 rounds every product and partial sum to 2^-53 of them.
- */
-#define FX_UPA 3
-#define FX_UPX 5
-#define FX_LB 29                       /* bits of the low limb */
-
-/* biased exponent field of a double given by its high word */
-__host__ __device__ __forceinline__ int fx_exp(unsigned hi) { return (int)((hi >> 20) & 0x7FF); }
-
-/* N of v in a group whose largest biased exponent is em (finite, em >= the
-   value's own): the mantissa shifted up by `up` bits and down by the
-   exponent difference (truncated) */
-__device__ __forceinline__ long long fx_from(double v, int em, int up)
-{
-    const unsigned long long b = (unsigned long long)__double_as_longlong(v);
-    int ev = (int)((b >> 52) & 0x7FF);
-    unsigned long long m = b & 0xFFFFFFFFFFFFFull;
-    if (ev) m |= 1ull << 52; else ev = 1;
-    const int d = em - ev;
-    m = d > 63 ? 0ull : (m << up) >> d;
-    return (long long)b < 0 ? -(long long)m : (long long)m;
-}
-/* two signed limbs of N */
-__device__ __forceinline__ int2 fx_split(long long N)
-{
-    int2 r;
-    r.x = (int)((N + (1ll << (FX_LB - 1))) >> FX_LB);
-    r.y = (int)(N - ((long long)r.x << FX_LB));
-    return r;
-}
-__device__ __forceinline__ double pow2d(int e) { return __hiloint2double((e + 1023) << 20, 0); }   /* -1022 <= e <= 1023 */
-/* acc += V 2^e; e of any size (below the normal range in two factors) */
-__device__ __forceinline__ double fx_add(double acc, long long V, int e)
-{
-    double v = (double)V;
-    if (e < -1022) { v *= pow2d(e + 900 < -1022 ? -1022 : e + 900); e = -900; }
-    return fma(v, pow2d(e > 1023 ? 1023 : e), acc);
-}
-/* the upper 16 bits of a double >= v (v >= 0): sign, exponent and 4 mantissa bits, rounded up */
-__device__ __forceinline__ unsigned short fx_bound16(double v)
-{
-    const unsigned long long b = (unsigned long long)__double_as_longlong(v);
-    return (unsigned short)((b + 0xFFFFFFFFFFFFull) >> 48);
-}
-__device__ __forceinline__ double fx_bound_to(unsigned short u) { return __hiloint2double((int)u << 16, 0); }
-
-/* ------------------------------------------------------------------ */
 /* assembled operator (real couplings)                                 */
 /* ------------------------------------------------------------------ */
 /*
@@ -1320,8 +1258,8 @@ __global__ void __launch_bounds__(128) k_assemble(int2 *__restrict__ A, unsigned
             }
             em2[rr] = (unsigned short)em;
             if (F.A32) {
-                /* N 2^(em - 1078) as a float in two factors */
-                const int k = em - 1078, k1 = k < -126 ? -126 : (k > 127 ? 127 : k);
+                /* N 2^(em - 1079) as a float in two factors */
+                const int k = em - 1079, k1 = k < -126 ? -126 : (k > 127 ? 127 : k);
                 const int k2 = k - k1 < -126 ? -126 : (k - k1 > 127 ? 127 : k - k1);
                 f0[j][rr] = em == 2047 ? __int_as_float(0x7FC00000) : __int_as_float((k1 + 127) << 23);
                 f1[j][rr] = __int_as_float((k2 + 127) << 23);
@@ -1594,7 +1532,7 @@ __global__ void __launch_bounds__(256, 3)
                         acc0 = mk<C>(__longlong_as_double(0x7FF8000000000000ll), __longlong_as_double(0x7FF8000000000000ll));
                         acc1 = acc0;
                     } else {
-                        const int e0 = ea.x + ex - 2100, e1 = ea.y + ex - 2100;
+                        const int e0 = ea.x + ex - 2101, e1 = ea.y + ex - 2101;
                         acc0.x = fx_add(acc0.x, h0r + ((m0r + rnd) >> FX_LB), e0);
                         acc0.y = fx_add(acc0.y, h0i + ((m0i + rnd) >> FX_LB), e0);
                         acc1.x = fx_add(acc1.x, h1r + ((m1r + rnd) >> FX_LB), e1);
@@ -1608,7 +1546,7 @@ __global__ void __launch_bounds__(256, 3)
                         const int row = P.prow[off + 2 * rp + rr], e = rr ? ea.y : ea.x;
                         if (row < 0) continue;
                         const double sc = e == 2047 ? __longlong_as_double(0x7FF8000000000000ll)
-                                                    : pow2d(e - 1078 < -1022 ? -1022 : e - 1078);
+                                                    : pow2d(e - 1079 < -1022 ? -1022 : e - 1079);
                         for (int t = 0; t < W; t++) {
                             const int w = HL ? (t / HJ) * HW + 2 * rp + rr - hb + t % HJ : lc[t * RMA + 2 * rp + rr];
                             const int cc = column(w);

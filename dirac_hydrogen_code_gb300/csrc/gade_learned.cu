@@ -28,6 +28,7 @@
 
 #include "gade.h"
 #include "gade_learned.h"
+#include "gade_fx.cuh"
 
 extern "C" int gade_set_error(int code, const char *msg);
 
@@ -900,36 +901,159 @@ static cudaError_t launch_pod_partial(int n, int R, const float2 *U, const doubl
     return cudaGetLastError();
 }
 
-/* the same partial projections with FP64 products and sums (training
-   targets are second differences of projections, which cancel) */
-__global__ void __launch_bounds__(256) k_pod_partial64(int n, int R, const float2 *__restrict__ U,
-                                                       const double2 *__restrict__ x, long long ldx,
-                                                       double2 *__restrict__ part, int npulse)
+/* Stages NP vectors of len complex values as fixed-point limbs (re hi, re lo,
+   im hi, im lo), x_p = x + p ldx into q[p][stride]; every RL entries share an
+   exponent, s_ex[p][nrun].  Warps take runs; ends with a barrier. */
+template <int NP, int RL>
+__device__ __forceinline__ void l_stage_fx(const double2 *__restrict__ x, long long ldx, int np, int len, int stride,
+                                           int4 *q, int *s_ex, int nrun)
 {
-    __shared__ double2 xs[PJ_L];
-    const int p = blockIdx.x, ch = blockIdx.y;
+    const int lane = threadIdx.x & 31;
+    for (int t = threadIdx.x >> 5; t < NP * nrun; t += 8) {
+        const int p = t / nrun, e0 = (t - p * nrun) * RL, e1 = min(len, e0 + RL);
+        unsigned mx = 0;
+#pragma unroll 8
+        for (int e = e0 + lane; e < e1; e += 32) {
+            const double2 v = p < np ? x[(size_t)p * ldx + e] : make_double2(0.0, 0.0);
+            mx = max(mx, max((unsigned)__double2hiint(v.x) & 0x7FFFFFFFu, (unsigned)__double2hiint(v.y) & 0x7FFFFFFFu));
+        }
+        const int em = max(fx_exp(__reduce_max_sync(0xffffffffu, mx)), 1);
+        if (lane == 0) s_ex[t] = em;
+#pragma unroll 4
+        for (int e = e0 + lane; e < e1; e += 32) {
+            const double2 v = p < np ? x[(size_t)p * ldx + e] : make_double2(0.0, 0.0);
+            const int2 re = fx_split(fx_from(v.x, em, FX_UPX)), im = fx_split(fx_from(v.y, em, FX_UPX));
+            q[p * stride + e] = make_int4(re.x, re.y, im.x, im.y);
+        }
+    }
+    __syncthreads();
+}
+
+/* sums NV (a power of two up to 32) doubles per lane over the warp, the values
+   split over the lanes on the way: lane l returns the sum of value
+   l / (32 / NV) (NV - 1 + log2(32 / NV) FP64 adds instead of 5 NV) */
+template <int NV>
+__device__ __forceinline__ double l_warp_split_sum(double (&v)[NV])
+{
+    const int lane = threadIdx.x & 31;
+    int nv = NV;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        const bool up = lane & o;
+        if (nv > 1) {
+            nv >>= 1;
+#pragma unroll
+            for (int j = 0; j < NV / 2; j++)
+                if (j < nv) {
+                    const double got = __shfl_xor_sync(0xffffffffu, up ? v[j] : v[j + nv], o);
+                    v[j] = (up ? v[j + nv] : v[j]) + got;
+                }
+        } else {
+            v[0] += __shfl_xor_sync(0xffffffffu, v[0], o);
+        }
+    }
+    return v[0];
+}
+
+/* the same partial projections to FP64 accuracy (training targets are second
+   differences of projections, which cancel).  The 8 n R npulse flops would be
+   bound by the FP64 pipe (1.83 ms at n = 53,040, R = 128, 16 pulses, float to
+   double conversions included), so the products run in fixed point: 512
+   entries of a state share an exponent and so do a lane's 16 basis entries
+   among them, 32 real products are summed exactly, one FP64 addition per sum. */
+#define PD_B 16
+template <int NP>
+__global__ void __launch_bounds__(256, 2) k_pod_partial64(int n, int R, const float2 *__restrict__ U,
+                                                          const double2 *__restrict__ x, long long ldx,
+                                                          double2 *__restrict__ part, int npulse, int rows)
+{
+    extern __shared__ __align__(16) int4 xq[];       /* [NP][PJ_L] */
+    constexpr int RL = 32 * PD_B, NR = PJ_L / RL;
+    __shared__ int s_ex[NP * NR];
+    const int ch = blockIdx.x, p0 = blockIdx.y * NP;
+    const int np = npulse - p0 < NP ? npulse - p0 : NP;
     const int i0 = ch * PJ_L;
     const int len = n - i0 < PJ_L ? n - i0 : PJ_L;
-    const double2 *xp = x + (size_t)p * ldx + i0;
-    for (int e = threadIdx.x; e < len; e += 256) xs[e] = xp[e];
-    __syncthreads();
+    const double2 *xc = x + (size_t)p0 * ldx + i0;
+    l_stage_fx<NP, RL>(xc, ldx, np, len, PJ_L, xq, s_ex, NR);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    for (int r = warp; r < R; r += 8) {
+    const int re = min(R, (int)(blockIdx.z + 1) * rows);
+    for (int r = blockIdx.z * rows + warp; r < re; r += 8) {
         const float2 *u = U + (size_t)r * n + i0;
-        double sr = 0, si = 0;
-        for (int e = lane; e < len; e += 32) {
-            const float2 uv = u[e];
-            const double2 xv = xs[e];
-            sr += (double)uv.x * xv.x + (double)uv.y * xv.y;
-            si += (double)uv.x * xv.y - (double)uv.y * xv.x;
-        }
+        double v[2 * NP];
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            sr += __shfl_xor_sync(0xffffffffu, sr, o);
-            si += __shfl_xor_sync(0xffffffffu, si, o);
+        for (int j = 0; j < 2 * NP; j++) v[j] = 0.0;
+        for (int e0 = lane; e0 < len; e0 += 32 * PD_B) {
+            float2 uv[PD_B];
+            unsigned mx = 0;
+#pragma unroll
+            for (int k = 0; k < PD_B; k++) {
+                uv[k] = e0 + 32 * k < len ? __ldcs(&u[e0 + 32 * k]) : make_float2(0.f, 0.f);
+                mx = max(mx, max(__float_as_uint(uv[k].x) & 0x7FFFFFFFu, __float_as_uint(uv[k].y) & 0x7FFFFFFFu));
+            }
+            const int em = max((int)(mx >> 23), 1);
+            int4 uq[PD_B];
+#pragma unroll
+            for (int k = 0; k < PD_B; k++) {
+                const int2 a = fx_split(fx_from_float(uv[k].x, em)), b = fx_split(fx_from_float(uv[k].y, em));
+                uq[k] = make_int4(a.x, a.y, b.x, b.y);
+            }
+#pragma unroll
+            for (int p = 0; p < NP; p++) {
+                const int ex = s_ex[p * NR + e0 / RL];
+                if (em != 255 && ex != 2047) {
+                    const int4 *xp = xq + p * PJ_L + e0;
+                    long long hr = 0, mr = 0, hi = 0, mi = 0;
+#pragma unroll
+                    for (int k = 0; k < PD_B; k++) {
+                        /* past the chunk: u = 0 (the entry read belongs to this CTA's buffer) */
+                        const int4 b = xp[e0 + 32 * k < len ? 32 * k : 0];
+                        const int4 a = uq[k];
+                        hr += (long long)a.x * b.x;      /* conj(u) x */
+                        hr += (long long)a.z * b.z;
+                        mr += (long long)a.x * b.y;
+                        mr += (long long)a.y * b.x;
+                        mr += (long long)a.z * b.w;
+                        mr += (long long)a.w * b.z;
+                        hi += (long long)a.x * b.z;
+                        hi -= (long long)a.z * b.x;
+                        mi += (long long)a.x * b.w;
+                        mi += (long long)a.y * b.z;
+                        mi -= (long long)a.z * b.y;
+                        mi -= (long long)a.w * b.x;
+                    }
+                    const long long rnd = 1ll << (FX_LB - 1);
+                    v[2 * p] = fx_add(v[2 * p], hr + ((mr + rnd) >> FX_LB), em + ex - 1205);
+                    v[2 * p + 1] = fx_add(v[2 * p + 1], hi + ((mi + rnd) >> FX_LB), em + ex - 1205);
+                } else if (p < np) {
+                    /* an infinity or NaN: FP64 products */
+                    for (int e = e0; e < len && e < e0 + 32 * PD_B; e += 32) {
+                        const float2 a = u[e];
+                        const double2 b = xc[(size_t)p * ldx + e];
+                        v[2 * p] += (double)a.x * b.x + (double)a.y * b.y;
+                        v[2 * p + 1] += (double)a.x * b.y - (double)a.y * b.x;
+                    }
+                }
+            }
         }
-        if (lane == 0) part[((size_t)ch * npulse + p) * R + r] = make_double2(sr, si);
+        const double sum = l_warp_split_sum<2 * NP>(v);
+        constexpr int LPV = 32 / (2 * NP);
+        const int q = lane / LPV;                        /* pulse q / 2, component q % 2 */
+        if (lane % LPV == 0 && (q >> 1) < np)
+            ((double *)part)[2 * (((size_t)ch * npulse + p0 + (q >> 1)) * R + r) + (q & 1)] = sum;
     }
+}
+
+template <int NP>
+static cudaError_t launch_pod_partial64(int n, int R, const float2 *U, const double2 *x, long long ldx, double2 *part,
+                                        int npulse, int nch, cudaStream_t st)
+{
+    const int smem = (int)sizeof(int4) * PJ_L * NP, rows = 32;
+    cudaError_t e = l_allow_smem<k_pod_partial64<NP>>(smem);
+    if (e != cudaSuccess) return e;
+    k_pod_partial64<NP><<<dim3(nch, (npulse + NP - 1) / NP, (R + rows - 1) / rows), 256, smem, st>>>(
+        n, R, U, x, ldx, part, npulse, rows);
+    return cudaGetLastError();
 }
 
 /* coef = sum of the chunks' partials in a fixed order: 32 coefficients per CTA,
@@ -965,11 +1089,13 @@ static int pod_project(bool fp64, int64_t n, int32_t R, const void *U, const voi
     const int64_t need = (int64_t)nch * npulse * R * (int64_t)sizeof(double2);
     if (scratch_bytes < need) return gade_set_error(GADE_ERR_ARG, "gade_pod_project: scratch too small");
     cudaStream_t st = (cudaStream_t)stream;
-    if (fp64)
-        k_pod_partial64<<<dim3(npulse, nch), 256, 0, st>>>((int)n, R, (const float2 *)U, (const double2 *)x, ldx,
-                                                           (double2 *)scratch, npulse);
-    else {
-        cudaError_t e;
+    cudaError_t e;
+    if (fp64) {
+#define PPD(NP_) launch_pod_partial64<NP_>((int)n, R, (const float2 *)U, (const double2 *)x, ldx, (double2 *)scratch, npulse, nch, st)
+        e = npulse == 1 ? PPD(1) : npulse == 2 ? PPD(2) : PPD(4);
+#undef PPD
+        if (e != cudaSuccess) return lfail(GADE_ERR_CUDA, "gade_pod_project_fp64", e);
+    } else {
 #define PPL(NP_) launch_pod_partial<NP_>((int)n, R, (const float2 *)U, (const double2 *)x, ldx, (double2 *)scratch, npulse, nch, st)
         if (npulse == 1) e = PPL(1);
         else if (npulse == 2) e = PPL(2);

@@ -8,7 +8,7 @@ from fractions import Fraction
 import numpy as np
 import pytest
 
-LB, UPA, UPX = 29, 3, 5
+LB, UPA, UPX = 29, 4, 5
 I64 = 1 << 63
 
 
@@ -20,7 +20,8 @@ def _fx(v, em, up):
     b = int(np.float64(v).view(np.uint64))
     ev, m = (b >> 52) & 0x7FF, b & ((1 << 52) - 1)
     m, ev = (m | 1 << 52, ev) if ev else (m, 1)
-    n = (m << up) >> (em - ev)
+    d = em - ev
+    n = ((m << up >> (d - 1)) + 1) >> 1 if d else m << up
     return -n if b >> 63 else n
 
 
@@ -42,7 +43,7 @@ def _row(a, x):
         assert abs(h) < I64 and abs(m) < I64
     v = h + ((m + (1 << (LB - 1))) >> LB)
     assert abs(v) < I64
-    return Fraction(v) * Fraction(2) ** (ea + ex - 2100)
+    return Fraction(v) * Fraction(2) ** (ea + ex - 2101)
 
 
 @pytest.mark.parametrize("spread", [0, 8, 40, 300])

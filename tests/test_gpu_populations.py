@@ -98,3 +98,42 @@ def test_restart_continues_the_run(workdirs, native_lib, tmp_path):
     xa = formats.out_read(os.path.join(full, f"x{nfull}.out"))
     xb = formats.out_read(os.path.join(half, f"x{nfull}.out"))
     assert np.linalg.norm(xa - xb) / np.linalg.norm(xa) < 1e-10
+
+
+@pytest.mark.parametrize("B", [1, 29, 30, 31, 256, 257, 610])
+@pytest.mark.parametrize("P", [1, 2, 3, 6])
+def test_eigproj_tiles(native_lib, B, P):
+    """Coefficients and class sums at odd sizes and pulse counts, entries spread
+    over orders of magnitude: coefficients <= 1e-14 of sum |x_i W_ij|'s
+    largest, sums <= 1e-13; a NaN in one block reaches that block and pulse
+    only."""
+    import torch
+    from dirac_hydrogen_code_gb300 import native
+    rng = np.random.default_rng(B + P)
+    nblk, nk = 5, 3
+    W = rng.standard_normal((nk, B, B)) * 10.0 ** rng.uniform(-6, 0, (nk, B, 1))
+    E = np.sort(rng.uniform(-3, 1, (nk, B)), axis=1)
+    kidx = rng.integers(0, nk, nblk).astype(np.int32)
+    x = (rng.standard_normal((P, nblk, B)) + 1j * rng.standard_normal((P, nblk, B))) * 10.0 ** rng.uniform(-8, 0, (P, nblk, B))
+    xb = x.copy()
+    xb[P - 1, 2, B // 2] = np.nan
+    dev = [torch.from_numpy(a).cuda() for a in (kidx, W, E)]
+    for state, bad in ((x, False), (xb, True)):
+        xd = torch.from_numpy(state.reshape(P, -1)).cuda()
+        coef = torch.empty(P, nblk, B, dtype=torch.complex128, device="cuda")
+        cls = torch.empty(P, nblk, 4, dtype=torch.float64, device="cuda")
+        native.call("gade_eigproj", P, nblk, B, dev[0].data_ptr(), dev[1].data_ptr(), dev[2].data_ptr(), -2.0,
+                    xd.data_ptr(), xd.shape[1], coef.data_ptr(), cls.data_ptr(), 0)
+        torch.cuda.synchronize()
+        c, s = coef.cpu().numpy(), cls.cpu().numpy()
+        for p in range(P):
+            for r in range(nblk):
+                if bad and (p, r) == (P - 1, 2):
+                    assert np.isnan(c[p, r]).all() and np.isnan(s[p, r, 3])
+                    continue
+                Wk, Ek = W[kidx[r]], E[kidx[r]]
+                ref = state[p, r].conj() @ Wk
+                assert np.all(np.abs(c[p, r] - ref) <= 1e-14 * (np.abs(state[p, r]) @ np.abs(Wk)).max())
+                q = np.abs(ref) ** 2
+                want = [q[Ek < -2].sum(), q[(Ek >= -2) & (Ek < 0)].sum(), q[Ek >= 0].sum(), q.sum()]
+                assert np.allclose(s[p, r], want, rtol=0, atol=1e-13 * q.sum())
