@@ -114,9 +114,18 @@ template <typename C, typename R> __device__ __forceinline__ void rfma(C &acc, R
 }
 __device__ __forceinline__ double2 cdiv(double2 a, double2 b)
 {
-    /* Smith's algorithm (robust complex division) */
+    /* a conj(b') / |b'|^2 2^-e with b' = b 2^-e of size 1: one division (its
+       dependent chain takes over 1,000 cycles here); Smith's form, with three,
+       where b has no normal exponent */
+    const unsigned h = max((unsigned)__double2hiint(b.x) & 0x7FFFFFFFu, (unsigned)__double2hiint(b.y) & 0x7FFFFFFFu);
+    const int e = (int)(h >> 20);
     double2 q;
-    if (fabs(b.x) >= fabs(b.y)) {
+    if (e >= 2 && e <= 2044) {
+        const double sc = __hiloint2double((2046 - e) << 20, 0), bx = b.x * sc, by = b.y * sc;
+        const double inv = 1.0 / fma(bx, bx, by * by);
+        q.x = fma(a.x, bx, a.y * by) * inv * sc;
+        q.y = fma(a.y, bx, -(a.x * by)) * inv * sc;
+    } else if (fabs(b.x) >= fabs(b.y)) {
         double r = b.y / b.x, d = b.x + b.y * r;
         q.x = (a.x + a.y * r) / d; q.y = (a.y - a.x * r) / d;
     } else {
@@ -1667,6 +1676,7 @@ struct PcT {
     int pred;                      /* PRED_* */
     unsigned spin_limit;           /* polls of a stage wait before the kernel gives up */
     int withhold;                  /* failure injection: stage whose copy is not issued (-1: none) */
+    const int *ex, *scale;         /* fixed point: [pulse][nk][2][2][nch] exponents, [pulse][nk][Bp] row scales */
 };
 
 __device__ __forceinline__ unsigned smem_u32(const void *p)
@@ -1952,6 +1962,467 @@ __global__ void __launch_bounds__(NW * 32) k_precond_tma(PcT Q, int mode, const 
         return;
     }
     for (int o = tid; o < B; o += NT) out[off + Q.ord[o]] = buf[o];
+}
+
+/* ------------------------------------------------------------------ */
+/* block-LU preconditioner in fixed point                               */
+/* ------------------------------------------------------------------ */
+/*
+ * The FP64 solves above need 129k DFMA per block row of 510 and were bound by
+ * the FP64 pipe of the SM that holds the row (58 us at N = 53,040).  Here the
+ * same sweeps run on the integer units (gade_fx.cuh).  D^T is scaled to a
+ * unit diagonal first, E D^T E with E = diag(2^-s), s_i = round(log2 |D_ii| /
+ * 2), so that the factors' entries and the vectors are of one size within a
+ * chunk: L' = E L E^-1, U' = E U E, b' = E b, x' = L'^-1 b', y = E U'^-1 x'.
+ * Factor entries are 57-bit integers with one exponent per chunk (triangle
+ * and chain block apart), vector entries 57-bit integers with one exponent
+ * per chunk; sums are exact 64-bit integers, rescaled once per chunk and
+ * sweep step.  An entry's error is ~2^-57 of the chunk's largest, where the
+ * FP64 sweeps round 33 products and sums to 2^-53 of theirs; measured against
+ * 64-bit-mantissa solves, rms over block rows, both are the same to 1% (the
+ * factors' own rounding): 4.0e-14 for a state, 2.3e-14 for random entries.
+ * What bounds it at 16 chunks: the chains' 32 dependent steps (34,000 of some
+ * 62,000 cycles), then the triangles' integer multiply-adds (21,000).  31.8 us
+ * for 104 block rows of 510 (FP64: 58), 118 us for 832 (330).
+ * An infinity or NaN in a block row or its factors makes its whole result NaN.
+ */
+#define PF_BW 16                       /* band padding it is written for (the B-spline bases' half-width is 15) */
+#define PF_PPS 2                       /* triangle pairs per stage */
+#define PF_GCH 4                       /* chain blocks per stage */
+#define PF_NAN 1000000                 /* exponent of a factor chunk that is not finite */
+#define PF_STAGE (PF_PPS * PC_TP > PF_GCH * 32 * PF_BW ? PF_PPS * PC_TP : PF_GCH * 32 * PF_BW)
+/* dynamic shared memory: two stages, x (int64 re, im) and its limbs per row,
+   partial sums, exponents (triangles and chains of both sweeps, vector) */
+__host__ __device__ __forceinline__ size_t pf_smem(int Bp, int nch)
+{
+    return (size_t)16 * (2 * PF_STAGE + 2 * Bp) + 8 * 1024 + 4 * (size_t)(7 * nch);
+}
+
+/* v 2^-sh to nearest, sh >= 1, |v| < 2^62 */
+__device__ __forceinline__ long long fx_rshift(long long v, int sh) { return ((v >> (min(sh, 63) - 1)) + 1) >> 1; }
+/* N = X 2^-sh with |N| <= 2^57 for a group whose largest |X| has high word mh; returns sh */
+__device__ __forceinline__ int fx_norm_shift(unsigned mh) { return 7 - __clz((int)mh); }
+__device__ __forceinline__ long long fx_norm(long long X, int sh) { return sh > 0 ? fx_rshift(X, sh) : X << -sh; }
+__device__ __forceinline__ unsigned fx_abs_hi(long long X)
+{
+    const int h = (int)(X >> 32);
+    return (unsigned)(h ^ (h >> 31));
+}
+
+/* scales and converts the factors of one (pulse, kappa): grid (triangle pairs
+   then chunks, sweep, pulse x kappa), one warp */
+__global__ void k_fix_factors(const double2 *__restrict__ FL, const double2 *__restrict__ FU, int4 *__restrict__ XL,
+                              int4 *__restrict__ XU, const int *__restrict__ scale, int *__restrict__ ex, int nch,
+                              int bwp, int Bp, size_t per)
+{
+    const int npair = (nch + 1) / 2, lane = threadIdx.x, up = blockIdx.y, pk = blockIdx.z;
+    const double2 *F = (up ? FU : FL) + (size_t)pk * per;
+    int4 *X = (up ? XU : XL) + (size_t)pk * per;
+    const int *s = scale + (size_t)pk * Bp;
+    int *eT = ex + ((size_t)pk * 2 + up) * 2 * nch, *eG = eT + nch;
+    /* value of an entry (row r, column c) after scaling */
+    auto scaled = [&](double2 v, int r, int c) {
+        const int k = up ? s[r] + s[c] : s[c] - s[r];
+        return make_double2(scalbn(v.x, k), scalbn(v.y, k));
+    };
+    auto gscaled = [&](double2 v, int r, int c) {
+        const int k = up ? s[r] - s[c] : s[c] - s[r];
+        return make_double2(scalbn(v.x, k), scalbn(v.y, k));
+    };
+    /* value = N 2^(em - 1075 - FX_UPA); PF_NAN where a factor is not finite */
+    auto exponent = [](int em) { return em == 2047 ? PF_NAN : em - 1075 - FX_UPA; };
+    auto hi = [](double2 v) {
+        return max((unsigned)__double2hiint(v.x) & 0x7FFFFFFFu, (unsigned)__double2hiint(v.y) & 0x7FFFFFFFu);
+    };
+    auto put = [](double2 v, int em) {
+        const int2 a = fx_split(fx_from(v.x, em, FX_UPA)), b = fx_split(fx_from(v.y, em, FX_UPA));
+        return make_int4(a.x, a.y, b.x, b.y);
+    };
+    if (blockIdx.x < npair) {
+        const int p = blockIdx.x, c0 = 2 * p, c1 = 2 * p + 1;
+        const bool has1 = c1 < nch;
+        const int sw = up ? 31 - lane : lane;
+        unsigned m0 = 0, m1 = 0;
+        for (int pass = 0; pass < 2; pass++) {
+            const int e0 = max(fx_exp(__reduce_max_sync(0xffffffffu, m0)), 1),
+                      e1 = max(fx_exp(__reduce_max_sync(0xffffffffu, m1)), 1);
+            for (int q = 0; q < 33; q++) {
+                const size_t o = (size_t)p * PC_TP + q * 32 + lane;
+                const bool first = q <= sw;
+                if (!first && !has1) { if (pass) X[o] = make_int4(0, 0, 0, 0); continue; }
+                const int r = first ? 32 * c0 + lane : 32 * c1 + 31 - lane;
+                const int c = up ? (first ? 32 * c0 + lane + q : 32 * c1 + q - 1)
+                                 : (first ? 32 * c0 + q : 32 * c1 + q - lane - 1);
+                const double2 v = scaled(F[o], r, c);
+                if (!pass) { if (first) m0 = max(m0, hi(v)); else m1 = max(m1, hi(v)); }
+                else X[o] = put(v, first ? e0 : e1);
+            }
+            if (pass && lane == 0) {
+                eT[c0] = exponent(e0);
+                if (has1) eT[c1] = exponent(e1);
+            }
+        }
+    } else {
+        const int c = blockIdx.x - npair;
+        const size_t o0 = (size_t)npair * PC_TP + (size_t)c * 32 * bwp;
+        unsigned m = 0;
+        for (int pass = 0; pass < 2; pass++) {
+            const int em = max(fx_exp(__reduce_max_sync(0xffffffffu, m)), 1);
+            for (int col = 0; col < bwp; col++) {
+                const int r = 32 * c + lane, cc = up ? 32 * (c + 1) + col : 32 * c - bwp + col;
+                double2 v = make_double2(0.0, 0.0);
+                if (cc >= 0 && cc < Bp) v = gscaled(F[o0 + col * 32 + lane], r, cc);
+                if (!pass) m = max(m, hi(v));
+                else X[o0 + col * 32 + lane] = put(v, em);
+            }
+            if (pass && lane == 0) eG[c] = exponent(em);
+        }
+    }
+}
+
+/*
+ * grid (pulse slot, block row), 8 warps; stages as in k_precond_tma (L
+ * triangles, L chain, U triangles, U chain) with two triangle pairs or four
+ * chain blocks each, so that two CTAs fit an SM.
+ * Triangle stage: a pair's 33 products per lane are split over four warps,
+ * whose sums (rows of chunk c0 and of chunk c1 apart) meet in shared memory.
+ * Chain: the next step needs only 16 of a chunk's rows, so four warps walk the
+ * chain on those alone (lane = row and component, four of the 16 columns per
+ * warp) and leave each chunk's normalised limbs in shared memory; another warp
+ * forms the chunk's other 16 rows from them as soon as they are there.
+ */
+__global__ void __launch_bounds__(256, 2) k_precond_fx(PcT Q, int mode, const double2 *__restrict__ in0,
+                                                       const double2 *__restrict__ in1, double2 *io,
+                                                       double2 *__restrict__ out, DevScal *sc)
+{
+    constexpr int BWP = PF_BW, GC = 32 * BWP, GCH = PF_GCH, SB = PF_STAGE;
+    extern __shared__ __align__(128) unsigned char smem_tma[];
+    int4 *stg = (int4 *)smem_tma;                          /* [2][SB] */
+    longlong2 *tx = (longlong2 *)(stg + 2 * SB);           /* [Bp] x as integers (re, im) */
+    int4 *xq = (int4 *)(tx + Q.Bp);                        /* [Bp] limbs */
+    long long *pt = (long long *)(xq + Q.Bp);              /* [2][4][4][32] partial sums of a triangle stage */
+    int *sexp = (int *)(pt + 1024);
+    const int nch = Q.nch;
+    int *sE = sexp + 4 * nch, *sEt = sE + nch, *sX = sEt + nch;   /* [4 nch] factors; x, triangle result, limbs */
+    __shared__ __align__(8) uint64_t bar[2];
+    __shared__ int all_ok, bad, s_prog;                    /* s_prog: chunks the chain has passed in this sweep */
+    __shared__ double2 s_c[2];                             /* beta, -w (PC_P) or -alpha (PC_S) */
+    pdl_enter();
+    const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+    const int r = blockIdx.y;
+    const int pulse = Q.plist ? Q.plist[blockIdx.x] : 0;
+    sc += pulse;
+    if (Q.pred != PRED_NONE) {
+        const int st = *(volatile const int *)&sc->state;
+        if (Q.pred == PRED_RUN ? st != ST_RUN : st != ST_RESTART) return;
+    }
+    {
+        const long long vo = (long long)pulse * Q.vstride;
+        in0 += vo;
+        if (in1) in1 += vo;
+        if (io) io += vo;
+        out += vo;
+    }
+    const int B = Q.B, Bp = Q.Bp;
+    const int npair = (nch + 1) / 2;
+    const int nsa = (npair + PF_PPS - 1) / PF_PPS, nsg = (nch + GCH - 1) / GCH, nps = nsa + nsg;
+    const int ns = 2 * nps;                 /* stages: L triangles, L chain, U triangles, U chain */
+    const int kk = Q.row_kidx[r];
+    const size_t off = (size_t)r * B;
+    const size_t per = pc_sweep_elems(nch, BWP);
+    const size_t pk = (size_t)pulse * Q.fstride / per + kk;    /* (pulse, kappa) */
+    const int4 *FL = (const int4 *)Q.FL + pk * per, *FU = (const int4 *)Q.FU + pk * per;
+    const int *scale = Q.scale + pk * Bp;
+    auto stage = [&](int k, const int4 **src, int *cnt) {
+        const int4 *F = k < nps ? FL : FU;
+        const int j = k < nps ? k : k - nps;
+        if (j < nsa) {
+            *cnt = min(PF_PPS, npair - PF_PPS * j);
+            *src = F + (size_t)PF_PPS * j * PC_TP;
+            return (unsigned)(*cnt * PC_TP * sizeof(int4));
+        }
+        const int g = k < nps ? j - nsa : nsg - 1 - (j - nsa);
+        *cnt = min(GCH, nch - g * GCH);
+        *src = F + (size_t)npair * PC_TP + (size_t)g * GCH * GC;
+        return (unsigned)(*cnt * GC * sizeof(int4));
+    };
+    if (tid == 0) {
+        mbar_init(&bar[0], 1);
+        mbar_init(&bar[1], 1);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        const int4 *src;
+        int cnt;
+        const unsigned bytes = stage(0, &src, &cnt);
+        if (Q.withhold != 0) tma_bulk_load(stg, src, bytes, &bar[0]);
+        all_ok = 1;
+        bad = 0;
+        s_prog = 0;
+    }
+    /* the vectors' entries are fetched while one thread forms the scalars (the
+       divisions of eight warps took 11,000 of the kernel's 90,000 cycles) */
+    constexpr int NL = 3;
+    double2 f0[NL], f1[NL], f2[NL];
+    int fs[NL], fg[NL];
+    auto fetch = [&](int n, int o) {
+        fs[n] = 0;
+        f0[n] = f1[n] = f2[n] = make_double2(0, 0);
+        if (o >= B) return;
+        fg[n] = Q.ord[o];
+        fs[n] = scale[o];
+        const size_t gi = off + fg[n];
+        f0[n] = in0[gi];
+        if (mode != PC_PLAIN) f1[n] = in1[gi];
+        if (mode == PC_P) f2[n] = io[gi];
+    };
+#pragma unroll
+    for (int n = 0; n < NL; n++) fetch(n, tid + 256 * n);
+    if (tid == 64) {
+        if (mode == PC_P) {
+            s_c[0] = cdiv(cmul(sc->rho, sc->alpha), cmul(sc->rho_prev, sc->w));
+            s_c[1] = make_double2(-sc->w.x, -sc->w.y);
+        } else if (mode == PC_S) {
+            s_c[1] = make_double2(-sc->alpha.x, -sc->alpha.y);
+        }
+    }
+    for (int e = tid; e < 4 * nch; e += 256) sexp[e] = Q.ex[pk * 4 * nch + e];
+    __syncthreads();
+    {
+        const double2 beta = s_c[0], negw = s_c[1], nega = s_c[1];
+        /* a warp's 32 entries are one chunk */
+        auto enter = [&](int n, int o) {
+            double2 val = f0[n];
+            const int so = fs[n];
+            if (o < B && mode != PC_PLAIN) {
+                if (mode == PC_P) {
+                    double2 t = f2[n];
+                    cfma(t, negw, f1[n]);
+                    cfma(val, beta, t);
+                } else {
+                    cfma(val, nega, f1[n]);
+                }
+                io[off + fg[n]] = val;
+            }
+            /* the largest |b'|'s exponent: the entries' less the row scales */
+            const unsigned h = max((unsigned)__double2hiint(val.x) & 0x7FFFFFFFu, (unsigned)__double2hiint(val.y) & 0x7FFFFFFFu);
+            const int e = fx_exp(h), es = e ? e - so : -5000;
+            const int em = __reduce_max_sync(0xffffffffu, es);
+            if (e == 2047) bad = 1;
+            /* N = b' 2^-(em - 1079): the mantissa with 4 bits more, down by em - (e - so) */
+            long long N[2];
+#pragma unroll
+            for (int c = 0; c < 2; c++) {
+                const unsigned long long b = (unsigned long long)__double_as_longlong(c ? val.y : val.x);
+                const int ev = (int)((b >> 52) & 0x7FF);
+                unsigned long long m = ev ? (b & 0xFFFFFFFFFFFFFull) | 1ull << 52 : 0ull;
+                m = fx_shift(m << 4, ev ? min(64, em - (ev - so)) : 0);
+                N[c] = (long long)b < 0 ? -(long long)m : (long long)m;
+            }
+            const int2 re = fx_split(N[0]), im = fx_split(N[1]);
+            xq[o] = make_int4(re.x, re.y, im.x, im.y);
+            /* a chunk of zeros: an exponent below all others, so that it moves no sum */
+            if (lane == 0) sX[o >> 5] = em - 1079;
+        };
+#pragma unroll
+        for (int n = 0; n < NL; n++)
+            if (tid + 256 * n < Bp) enter(n, tid + 256 * n);
+        for (int o = tid + 256 * NL; o < Bp; o += 256) { fetch(0, o); enter(0, o); }
+    }
+    __syncthreads();
+    for (int c = tid; c < nch; c += 256) sEt[c] = sexp[c] + sX[c] + 2 * FX_LB;
+    for (int e = tid; e < 4 * nch; e += 256)
+        if (sexp[e] == PF_NAN) bad = 1;
+
+    const long long rnd = 1ll << (FX_LB - 1);
+    int k = 0;
+    for (; k < ns; k++) {
+        if (tid == 0 && k + 1 < ns && k + 1 != Q.withhold) {
+            const int4 *src;
+            int cnt;
+            const unsigned bytes = stage(k + 1, &src, &cnt);
+            tma_bulk_load(stg + ((k + 1) & 1) * SB, src, bytes, &bar[(k + 1) & 1]);
+        }
+        unsigned spins = 0;
+        bool ok = true;
+        while (!mbar_try_wait(&bar[k & 1], (k >> 1) & 1)) {
+            if (++spins > Q.spin_limit) { ok = false; break; }
+        }
+        if (!ok) all_ok = 0;
+        __syncthreads();
+        if (!all_ok) break;
+        const int4 *S = stg + (k & 1) * SB;
+        const int up = k >= nps;                   /* U sweep */
+        const int j = up ? k - nps : k;
+        if (k == nps) {
+            /* x of the L sweep as limbs, normalised per chunk (a warp per chunk) */
+            for (int c = wid; c < nch; c += 8) {
+                const longlong2 X = tx[32 * c + lane];
+                const int sh = fx_norm_shift(__reduce_max_sync(0xffffffffu, max(fx_abs_hi(X.x), fx_abs_hi(X.y))));
+                const int2 re = fx_split(fx_norm(X.x, sh)), im = fx_split(fx_norm(X.y, sh));
+                xq[32 * c + lane] = make_int4(re.x, re.y, im.x, im.y);
+                if (lane == 0) sEt[c] = sexp[2 * nch + c] + sE[c] + sh + 2 * FX_LB;
+            }
+            __syncthreads();
+        }
+        if (j < nsa) {
+            /* triangle pair PF_PPS j + wid / 4: chunks c0 = 2p, c1 = 2p + 1; products
+               part 8 + (part > 0) .. part 8 + 8 of the 33 */
+            const int pr = wid >> 2, part = wid & 3;
+            const int p = PF_PPS * j + pr;
+            const int c0 = 2 * p, c1 = 2 * p + 1;
+            const bool act = p < npair, has1 = c1 < nch;
+            const int sw = up ? 31 - lane : lane;      /* last product of the first row */
+            const int Q0 = part * 8 + (part > 0), Q1 = part * 8 + 9;
+            if (act) {
+                const int4 *T = S + pr * PC_TP + lane;
+                /* entry of x: q + b0 up to the switch, q + b1 after it (no chunk c1: any entry, T is zero) */
+                const int b0 = up ? 32 * c0 + lane : 32 * c0, b1 = !has1 ? -1 : (up ? 32 * c1 - 1 : 32 * c1 - lane - 1);
+                long long hr = 0, mr = 0, hi = 0, mi = 0, hr0 = 0, mr0 = 0, hi0 = 0, mi0 = 0;
+#pragma unroll
+                for (int n = 0; n < 9; n++) {
+                    /* only the first part has a ninth product (the others' is made zero) */
+                    const int q = n == 8 ? min(Q0 + 8, 32) : Q0 + n;
+                    int4 d = T[q * 32];
+                    const int4 b = xq[q + (q <= sw ? b0 : b1)];
+                    if (n == 8 && part > 0) d = make_int4(0, 0, 0, 0);
+                    const int nz = -b.z, nw = -b.w;
+                    hr += (long long)d.x * b.x;
+                    hr += (long long)d.z * nz;
+                    mr += (long long)d.x * b.y;
+                    mr += (long long)d.y * b.x;
+                    mr += (long long)d.z * nw;
+                    mr += (long long)d.w * nz;
+                    hi += (long long)d.x * b.z;
+                    hi += (long long)d.z * b.x;
+                    mi += (long long)d.x * b.w;
+                    mi += (long long)d.y * b.z;
+                    mi += (long long)d.z * b.y;
+                    mi += (long long)d.w * b.x;
+                    /* the products up to sw belong to the row of c0 */
+                    const bool last = q == sw && (n < 8 || part == 0);
+                    hr0 = last ? hr : hr0; mr0 = last ? mr : mr0;
+                    hi0 = last ? hi : hi0; mi0 = last ? mi : mi0;
+                }
+                if (sw >= Q1) { hr0 = hr; mr0 = mr; hi0 = hi; mi0 = mi; }
+                long long *d = pt + (size_t)wid * 4 * 32 + lane;
+                d[0] = hr0 + ((mr0 + rnd) >> FX_LB);
+                d[32] = hi0 + ((mi0 + rnd) >> FX_LB);
+                d[64] = (hr - hr0) + ((mr - mr0 + rnd) >> FX_LB);
+                d[96] = (hi - hi0) + ((mi - mi0 + rnd) >> FX_LB);
+            }
+            __syncthreads();
+            if (act) {
+                /* warp (pair, component): re, im of the row lane of c0, then of the row 31 - lane of c1 */
+                const long long *d = pt + ((size_t)pr * 16 + part) * 32 + lane;
+                const long long v = d[0] + d[4 * 32] + d[8 * 32] + d[12 * 32];
+                const int row = part < 2 ? 32 * c0 + lane : 32 * c1 + 31 - lane;
+                if (part < 2 || has1) ((long long *)tx)[2 * row + (part & 1)] = v;
+            }
+            __syncthreads();
+        } else {
+            const int g = up ? nsg - 1 - (j - nsa) : j - nsa;
+            const int cnt = min(GCH, nch - g * GCH);
+            /* lane: row lane / 2 of the 16 rows, component lane % 2.  Limbs of a chunk's
+               16 chain entries are kept twice, as the real and as the imaginary
+               part's sums use them: (re, -im) and (im, re) */
+            const int row16 = lane >> 1, comp = lane & 1;
+            auto put_limbs = [&](int4 *xl, int2 l) {
+                int2 *la = (int2 *)(xl + row16), *lb = (int2 *)(xl + 16 + row16);
+                la[comp] = comp ? make_int2(-l.x, -l.y) : l;
+                lb[comp ^ 1] = l;
+            };
+            auto products = [&](const int4 *G, const int4 *xl, int n) {
+                long long h = 0, h2 = 0, m = 0, m2 = 0;
+#pragma unroll
+                for (int q = 0; q < n; q++) {
+                    const int4 d = G[q * 32], b = xl[q];
+                    h += (long long)d.x * b.x;
+                    m += (long long)d.x * b.y;
+                    m2 += (long long)d.y * b.x;
+                    h2 += (long long)d.z * b.z;
+                    m += (long long)d.z * b.w;
+                    m2 += (long long)d.w * b.z;
+                }
+                return h + h2 + ((m + m2 + rnd) >> FX_LB);
+            };
+            /* aligned sum of the triangle result t and the chain part v of chunk c */
+            auto join = [&](long long t, long long v, int c, int cp, int &E) {
+                const int Et = sEt[c], Eg = sexp[(2 * up + 1) * nch + c] + sX[cp] + 2 * FX_LB;
+                E = max(Et, Eg) + 1;
+                return fx_rshift(t, E - Et) + fx_rshift(v, E - Eg);
+            };
+            if (wid < 4) {
+                /* four columns per warp; the four sums of a row meet in shared memory
+                   (two buffers, one barrier of these warps per step) and every warp
+                   carries the whole x on, so that nothing is handed back */
+                for (int e = 0; e < cnt; e++) {
+                    const int ci = up ? cnt - 1 - e : e;     /* U: last chunk first */
+                    const int c = g * GCH + ci, cp = up ? c + 1 : c - 1;
+                    const int rr = up ? row16 : 16 + row16;
+                    long long *tp = (long long *)tx + 2 * (32 * c + rr) + comp;
+                    const long long t = *tp;
+                    long long X = t;
+                    int E = sEt[c];
+                    if (cp >= 0 && cp < nch) {               /* the first chunk has no neighbour: the triangle result stands */
+                        long long *ps = pt + (c & 1) * 128;
+                        ps[wid * 32 + lane] = products(S + ci * GC + rr + 4 * wid * 32, xq + 32 * cp + 16 * comp + 4 * wid, 4);
+                        asm volatile("bar.sync 1, 128;" ::: "memory");
+                        X = join(t, (ps[lane] + ps[32 + lane]) + (ps[64 + lane] + ps[96 + lane]), c, cp, E);
+                    }
+                    const int sh = fx_norm_shift(__reduce_max_sync(0xffffffffu, fx_abs_hi(X)));
+                    const int2 l = fx_split(fx_norm(X, sh));
+                    /* every warp writes the same values: the next step reads what its own warp wrote */
+                    put_limbs(xq + 32 * c, l);
+                    if (lane == 0) sX[c] = E + sh;
+                    __syncwarp();
+                    if (wid == 0) {
+                        *tp = X;
+                        if (lane == 0) sE[c] = E;
+                        __threadfence_block();
+                        if (lane == 0) *(volatile int *)&s_prog = (up ? nch - 1 - c : c) + 1;
+                    }
+                }
+            } else if (wid - 4 < cnt) {
+                const int ci = wid - 4, c = g * GCH + ci, cp = up ? c + 1 : c - 1;
+                const int need = up ? nch - 1 - c : c;       /* chunks passed when cp's limbs are there */
+                if (need > 0) {
+                    unsigned spins = 0;
+                    while (*(volatile int *)&s_prog < need && ++spins < MBAR_SPIN_LIMIT) {
+                    }
+                    if (spins >= MBAR_SPIN_LIMIT) all_ok = 0;
+                    __threadfence_block();
+                    const int rr = up ? 16 + row16 : row16;
+                    long long *tp = (long long *)tx + 2 * (32 * c + rr) + comp;
+                    int E;
+                    *tp = join(*tp, products(S + ci * GC + rr, xq + 32 * cp + 16 * comp, BWP), c, cp, E);
+                }
+            }
+            __syncthreads();
+            if (k == nps - 1 && tid == 0) s_prog = 0;        /* the U sweep counts anew */
+        }
+    }
+    if (!all_ok) {
+        if (tid == 0) {
+            atomicOr(&sc->err, 1u);
+            /* drain the copies still in flight (bounded) before exiting: the
+               stage that timed out and the next one, both issued unless withheld */
+            for (int k2 = k; k2 < k + 2 && k2 < ns; k2++) {
+                if (k2 == Q.withhold) continue;
+                unsigned spins = 0;
+                while (!mbar_try_wait(&bar[k2 & 1], (k2 >> 1) & 1) && ++spins < MBAR_SPIN_LIMIT) {
+                }
+            }
+        }
+        __syncthreads();
+        return;
+    }
+    const bool nan = bad != 0;
+    for (int o = tid; o < B; o += 256) {
+        const longlong2 X = tx[o];
+        const int e = sE[o >> 5] - scale[o];
+        double2 y = make_double2(fx_add(0.0, X.x, e), fx_add(0.0, X.y, e));
+        if (nan) y.x = y.y = __longlong_as_double(0x7FF8000000000000ll);
+        out[off + Q.ord[o]] = y;
+    }
 }
 
 /* ------------------------------------------------------------------ */
@@ -2394,6 +2865,8 @@ struct gade_solver {
     int *d_ord;
     double2 *d_FL, *d_FU;       /* chunk-packed factors for the TMA kernel */
     int bwp;
+    int4 *d_XL, *d_XU;          /* the factors in fixed point (NULL: not used) */
+    int *d_pex, *d_pscale;      /* their exponents and the row scales (PcT) */
     /* vectors */
     double2 *x, *rhs, *r, *r0, *p, *v, *y, *z, *s, *t, *tmp0, *tmp1;
     /* reductions */
@@ -2482,7 +2955,7 @@ struct gade_solver {
     void *d_ang_dd[4], *d_Sdd, *d_Hdd, *d_Mdd;
     cdd *xdd, *ddd, *wdd;
     int pc_withhold;            /* failure injection: preconditioner stage whose copy is withheld (-1: none) */
-    int pc_nw;                  /* warps per block row of the FP64 preconditioner solves (4 or 8) */
+    int pc_nw;                  /* warps per block row of the complex128 preconditioner solves (4: FP64; 8: fixed point, or FP64 without d_XL) */
 };
 
 /* dynamic shared memory of k_precond_tma: two stage buffers, the block
@@ -3059,6 +3532,17 @@ static int solver_create(const gade_problem *p, int npulse, const double *dts, c
         cudaFuncSetAttribute(k_precond_tma<double, 32, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm64);
         cudaFuncSetAttribute(k_precond_tma<double, 16, 8>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm64);
         cudaFuncSetAttribute(k_precond_tma<double, 32, 8>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm64);
+        /* k_precond_fx is written for 16 chain columns (half-bandwidth <= 16,
+           both bases' own ordering) and must fit an SM (Bp <= 4,500); wider
+           bands and larger blocks keep the FP64 kernel */
+        const size_t smx = pf_smem(s->Bp, s->nch);
+        if (s->bwp == PF_BW && smx <= 220 * 1024) {
+            cudaFuncSetAttribute(k_precond_fx, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smx);
+            UP(s->d_XL, (const int4 *)nullptr, NP * s->fstride);
+            UP(s->d_XU, (const int4 *)nullptr, NP * s->fstride);
+            UP(s->d_pex, (const int *)nullptr, NP * s->nk * 4 * s->nch);
+            UP(s->d_pscale, (const int *)nullptr, NP * s->nk * s->Bp);
+        }
         cudaFuncSetAttribute(k_precond_tma<float, 16, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm32);
         cudaFuncSetAttribute(k_precond_tma<float, 32, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm32);
     }
@@ -3113,6 +3597,27 @@ static int solver_create(const gade_problem *p, int npulse, const double *dts, c
                 if (ce == cudaSuccess) ce = cudaMemcpy((float2 *)s->d_D32 + k * s->dstride, Df.data(), sizeof(float2) * s->dstride, cudaMemcpyHostToDevice);
                 if (ce == cudaSuccess) ce = cudaMemcpy((float2 *)s->d_FL32 + k * s->fstride, FLf.data(), sizeof(float2) * s->fstride, cudaMemcpyHostToDevice);
                 if (ce == cudaSuccess) ce = cudaMemcpy((float2 *)s->d_FU32 + k * s->fstride, FUf.data(), sizeof(float2) * s->fstride, cudaMemcpyHostToDevice);
+            }
+            if (ce == cudaSuccess && s->d_XL) {
+                /* row scales: half the binary exponent of the diagonal, in the factors' ordering */
+                std::vector<int> sc((size_t)s->nk * s->Bp, 0);
+                for (int kk = 0; kk < s->nk; kk++)
+                    for (int o = 0; o < s->B; o++) {
+                        const int i = su->ord[o];
+                        for (int t = 0; t < s->W; t++)
+                            if (su->ell_col[(size_t)t * s->B + i] == i) {
+                                const double2 d = D[((size_t)kk * s->W + t) * s->B + i];
+                                const double m = hypot(d.x, d.y);
+                                if (m > 0 && std::isfinite(m)) sc[(size_t)kk * s->Bp + o] = (int)lrint(0.5 * log2(m));
+                            }
+                    }
+                ce = cudaMemcpy(s->d_pscale + (size_t)k * s->nk * s->Bp, sc.data(), sizeof(int) * sc.size(), cudaMemcpyHostToDevice);
+                k_fix_factors<<<dim3((s->nch + 1) / 2 + s->nch, 2, s->nk), 32>>>(
+                    s->d_FL + k * s->fstride, s->d_FU + k * s->fstride, s->d_XL + k * s->fstride, s->d_XU + k * s->fstride,
+                    s->d_pscale + (size_t)k * s->nk * s->Bp, s->d_pex + (size_t)k * s->nk * 4 * s->nch, s->nch, s->bwp, s->Bp,
+                    pc_sweep_elems(s->nch, s->bwp));
+                if (ce == cudaSuccess) ce = cudaGetLastError();
+                if (ce == cudaSuccess) ce = cudaDeviceSynchronize();
             }
             if (sk != su) gade_setup_release(sk);
             /* radial tables of the three pulse components used by each l */
@@ -3792,12 +4297,25 @@ static PcT pc_params(const gade_solver *s, const void *FL, const void *FU, int p
     Q.plist = s->d_plist; Q.vstride = s->n; Q.fstride = s->fstride; Q.pred = pred;
     Q.spin_limit = s->pc_wait ? s->pc_wait : MBAR_SPIN_LIMIT;
     Q.withhold = s->pc_withhold;
+    Q.ex = s->d_pex; Q.scale = s->d_pscale;
     return Q;
 }
 
 static int launch_precond(gade_solver *s, int mode, const double2 *in0, const double2 *in1, double2 *io,
                           double2 *out, cudaStream_t st, int pred = PRED_NONE)
 {
+    /* 8 warps: fixed point where the factors have that form (see solver_create):
+       31.8 us a solve at N = 53,040 and 118 us for 8 pulses, where
+       k_precond_tma's 8 FP64 warps take 58 and 330 */
+    if (s->pc_nw == 8 && s->d_XL) {
+        PcT Q = pc_params(s, s->d_XL, s->d_XU, pred);
+        const dim3 grid(s->nslot, s->nblk);
+        prof_begin(s, st);
+        launch_pdl(k_precond_fx, grid, dim3(256), pf_smem(s->Bp, s->nch), st, Q, mode, in0, in1, io, out, s->d_sc);
+        prof_end(s, st, 1);
+        CKL();
+        return GADE_OK;
+    }
     PcT Q = pc_params(s, s->d_FL, s->d_FU, pred);
     const size_t smem = pc_smem_bytes(s, sizeof(double2));
     dim3 grid(s->nslot, s->nblk), block(32 * s->pc_nw);
