@@ -38,6 +38,7 @@
 #include <type_traits>
 #include <algorithm>
 #include <utility>
+#include <queue>
 #include <vector>
 
 #include "gade_internal.h"
@@ -1331,8 +1332,13 @@ __global__ void __launch_bounds__(128) k_assemble(int2 *__restrict__ A, unsigned
 }
 
 #define ASM_GB 16   /* coupled blocks staged per phase: two per warp */
+/* what a piece costs beyond its pairs, in pairs: staging, exchange, the arrival
+   count and the next piece's descriptor, 8-12 us of latencies under load where a
+   pair takes 1.4 us.  4: 6,437 us for 8 steps at N = 53,040 and 9,166 us for 2
+   at N = 244,000, 6: 6,411 and 9,158, 8: 6,429 and 9,136; charged once per unit
+   instead of per piece, as 4: 6,469 and 9,240. */
 #ifndef ASM_UFIX
-#define ASM_UFIX 4.0
+#define ASM_UFIX 6.0
 #endif
 
 /* shared memory of k_apply_asm: x windows of the block row (x, x_n, delta;
@@ -2920,6 +2926,7 @@ struct gade_solver {
     int asm_ok;                 /* K_a built */
     int use_asm;                /* applies and steps use it */
     int asm_part;               /* its partition: 0 plain, 1 balanced */
+    double asm_bal_gain;        /* modelled time of the plain partition over the balanced one's */
     int npairs;                 /* (block row, coupled block) pairs */
     int *d_pair_c;
     int2 *d_K, *d_A;            /* fixed-point limbs of K (per table set) and of A (per pulse), see AsmLay */
@@ -3996,8 +4003,9 @@ static int asm_partitions(gade_solver *s)
         }
         if ((rc = part_upload(s, s->part_asm[0], seg, pcs))) return rc;
     }
+    /* a pair's and a piece's cost */
     auto pcost = [&](int q) { return 2.0 * s->h_chunk_nrows[q] * s->W + 2.0 * s->h_chunk_ncols[q]; };
-    auto ufix = [&](int q) { return ASM_UFIX * s->h_chunk_nrows[q] * s->W; };
+    auto ufix = [&](int q) { return ASM_UFIX * pcost(q); };
     /* units are cut at multiples of the pairs that k_apply_asm's thread groups take side by side */
     const int cut = std::max(1, std::min(4, 256 / std::max(1, s->RMA / 2)));
     for (int cls = 0; cls < 4; cls++) {
@@ -4005,36 +4013,67 @@ static int asm_partitions(gade_solver *s)
         if (f == 1 && s->prec != GADE_PREC_MIXED) continue;
         if (s->part_asm_bal[o].nseg) continue;
         const int nseg = o * s->nsm;
-        double total = 0;
-        for (int u = 0; u < nunit; u++) {
-            const int r = u / s->nchunk, q = u - r * s->nchunk;
-            total += ufix(q) + pcost(q) * (s->h_pair_ptr[r + 1] - s->h_pair_ptr[r]);
-        }
-        const double T = total / nseg;
-        auto seg_of = [&](double mid) { int k = (int)(mid / T); return k < 0 ? 0 : (k >= nseg ? nseg - 1 : k); };
         std::vector<int4> pcs;
         std::vector<int> pseg;
-        double pos = 0;
+        /* units in order, cut where a segment's cost reaches T; false when
+           more than nseg segments come out */
+        auto cut_at = [&](double T) {
+            pcs.clear();
+            pseg.clear();
+            int sg = 0;
+            double left = T;
+            for (int u = 0; u < nunit; u++) {
+                const int r = u / s->nchunk, q = u - r * s->nchunk;
+                const int a1 = s->h_pair_ptr[r + 1];
+                const size_t first = pcs.size();
+                int a = s->h_pair_ptr[r];
+                do {
+                    /* a new segment where this one has no room for a worthwhile piece */
+                    const int rest = std::min(cut, a1 - a);
+                    if (left < T && left < ufix(q) + pcost(q) * rest) {
+                        if (++sg == nseg) return false;
+                        left = T;
+                    }
+                    int n = cut * (int)std::max(1.0, floor((left - ufix(q)) / (pcost(q) * cut)));
+                    n = std::min(n, a1 - a);
+                    pcs.push_back(make_int4(u, a, a + n, 0));
+                    pseg.push_back(sg);
+                    left -= ufix(q) + pcost(q) * n;
+                    a += n;
+                } while (a < a1);
+                const int np = (int)(pcs.size() - first);
+                for (int k = 0; k < np; k++) pcs[first + k].w = k | (np << 16);
+            }
+            return true;
+        };
+        /* the smallest T that nseg segments hold */
+        double lo = 0, hi = 0;
         for (int u = 0; u < nunit; u++) {
             const int r = u / s->nchunk, q = u - r * s->nchunk;
-            const int a0 = s->h_pair_ptr[r], a1 = s->h_pair_ptr[r + 1];
-            const size_t first = pcs.size();
-            if (a0 == a1) { pcs.push_back(make_int4(u, a0, a0, 0)); pseg.push_back(seg_of(pos + 0.5 * ufix(q))); }
-            pos += ufix(q);
-            int cur = -1, b0 = a0;
-            for (int a = a0; a < a1; a += cut) {
-                const double c = pcost(q) * std::min(cut, a1 - a);
-                const int sg = seg_of(pos + 0.5 * c);
-                pos += c;
-                if (sg != cur) {
-                    if (cur >= 0) { pcs.push_back(make_int4(u, b0, a, 0)); pseg.push_back(cur); }
-                    cur = sg;
-                    b0 = a;
-                }
+            hi += ufix(q) + pcost(q) * (s->h_pair_ptr[r + 1] - s->h_pair_ptr[r]);
+        }
+        lo = hi / nseg / 2;
+        for (int it = 0; it < 30; it++) {
+            const double T = 0.5 * (lo + hi);
+            if (cut_at(T)) hi = T; else lo = T;
+        }
+        cut_at(hi);
+        if (f == 0 && cls % 2 == 0) {
+            /* the plain partition's end: units in order, each to the first free slot */
+            std::priority_queue<double, std::vector<double>, std::greater<double>> slot;
+            double end = 0, stream = 0, fixed = 0;
+            for (int k = 0; k < nseg; k++) slot.push(0.0);
+            for (int u = 0; u < nunit; u++) {
+                const int r = u / s->nchunk, q = u - r * s->nchunk;
+                const double t = slot.top() + ufix(q) + pcost(q) * (s->h_pair_ptr[r + 1] - s->h_pair_ptr[r]);
+                slot.pop();
+                slot.push(t);
+                end = std::max(end, t);
+                stream += pcost(q) * (s->h_pair_ptr[r + 1] - s->h_pair_ptr[r]);
+                fixed = std::max(fixed, ufix(q));
             }
-            if (a1 > a0) { pcs.push_back(make_int4(u, b0, a1, 0)); pseg.push_back(cur); }
-            const int np = (int)(pcs.size() - first);
-            for (int k = 0; k < np; k++) pcs[first + k].w = k | (np << 16);
+            /* too little per CTA: the times are latencies that the model does not know */
+            s->asm_bal_gain = stream < 2.0 * fixed * nseg ? 0.0 : end / hi;
         }
         std::vector<int> seg((size_t)nseg + 1, 0);
         for (int sg : pseg) seg[sg + 1]++;
@@ -4704,7 +4743,11 @@ static int choose_operator(gade_solver *s)
     }
     if (!rc) rc = time_step_tables(s, &tab_asm);
     if (rc) { s->use_asm = 0; return rc; }
-    s->asm_part = s->asm_ms[1] < s->asm_ms[0] ? 1 : 0;
+    /* by the cost model, not by the two times: where these are close the choice,
+       and with it the order of the sums, would differ between solvers of one
+       problem.  Measured (plain, balanced): N = 8,400 21 and 22 us (2 pairs per
+       CTA), N = 53,040 88 and 81 us, N = 244,000 510 and 503 us. */
+    s->asm_part = s->asm_bal_gain > 1.03 ? 1 : 0;
     const float best = s->asm_ms[s->asm_part];
     s->tab_ms[0] = tab_mf;
     s->tab_ms[1] = tab_asm;
