@@ -17,8 +17,9 @@ import os
 import numpy as np
 import pytest
 
-from dirac_hydrogen_code_gb300.cn import run
+from dirac_hydrogen_code_gb300.cn import pulse, run
 from dirac_hydrogen_code_gb300.gen import generate
+from dirac_hydrogen_code_gb300.native import Batch, Problem
 from tests.golden.cases import CASES, sketch
 
 pytestmark = pytest.mark.gpu
@@ -148,3 +149,31 @@ def test_fp64_apply_after_double_float_steps(golden_case, native_lib):
     y_after_step = sol.apply(x)
     sol.set_time(fts[-1])
     assert np.array_equal(y_after_step, sol.apply(x))
+
+
+@pytest.mark.parametrize("op", [0, 1])
+def test_adaptive_sweeps_match_one_iteration_per_launch(workdirs, native_lib, op):
+    """The sweeps and iterations that a step launches at once follow the last
+    steps; states, sweeps and iterations are those of one iteration per
+    launch, while tolerances take the counts up and down."""
+    d, params, info = workdirs["tiny_nondipole"]
+    prob = Problem(d, info["lmax"])
+    psi, _ = prob.psi0()
+    dt = params["Cycles"] * 2 * math.pi / params["Omega"] / params["Ntime"]
+    steps = [(1e-4, 500)] * 10 + [(1e-10, 500)] * 3 + [(1e-6, 500)] * 10 + [(1e-11, 500), (1e-2, 500), (1e-10, 500)]
+    out = []
+    for per_launch in (0, 1):
+        b = Batch(prob, [dt], precision="mixed", chunk_splines=16, iters_per_launch=per_launch)
+        b.set_operator(op)
+        b.set_x(0, psi)
+        rec = []
+        for k, (tol, maxit) in enumerate(steps):
+            ft = pulse(params["Intensity"], params["Omega"], params["Cycles"], (k + 0.5) * dt)
+            st = b.step(ft.reshape(1, 6), maxit=maxit, tol=tol)[0]
+            rec.append((st["inner_iters"], st["refinements"], b.get_x(0)))
+        b.close()
+        out.append(rec)
+    assert len({r[:2] for r in out[0]}) > 1
+    for a, c in zip(*out):
+        assert a[:2] == c[:2]
+        assert np.array_equal(a[2], c[2])
