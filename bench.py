@@ -478,7 +478,8 @@ def run_ours(args):
                    else "k_apply (matrix-free S + H(t) apply)"),
         "note": ("achieved = CSR-equivalent bytes of the reference assembled complex128 SpMV "
                  "(20 nnz + 4(N+1) + 32N) / average operator apply time over the sampled steps; the kernel "
-                 "stores real coupling values (8 B) and is bound by the FP64 pipe, see fp64" if assembled else
+                 "streams real coupling values (8 B fixed point) and multiplies them on the integer units; it is "
+                 "bound by HBM and the latencies around the stream, see compulsory_bytes" if assembled else
                  "achieved = CSR-equivalent bytes of the reference assembled complex128 SpMV "
                  "(20 nnz + 4(N+1) + 32N) / average k_apply time over the sampled steps; the matrix-free "
                  "kernel moves far fewer bytes and is bound by the FP64 pipe, see fp64"),
@@ -486,12 +487,15 @@ def run_ours(args):
         "assembly_per_step": {"kernel": "k_assemble", "flops": asm_flops, "bytes": asm_bytes} if assembled else None,
         "fp64": {"achieved_tflops": mf_flops / (apply_ms * 1e-3) / 1e12, "peak_tflops": fp64_peak,
                  "frac": mf_flops / (apply_ms * 1e-3) / 1e12 / fp64_peak, "flops_per_launch": mf_flops,
-                 "peak_kind": "measured (own FP64 FMA kernel)"},
+                 "peak_kind": "measured (own FP64 FMA kernel)",
+                 "note": ("multiply-adds counted as FP64 ones; the couplings' run on the integer units, so the "
+                          "fraction is no bound" if assembled else "")},
         "compulsory_bytes": {"per_launch": mf_bytes,
                              "achieved_gbs": mf_bytes / (apply_ms * 1e-3) / 1e9,
                              "frac": mf_bytes / (apply_ms * 1e-3) / 1e9 / hbm_peak,
-                             "formula": ("stored coupling values pairs x W x B x 8 B + diagonal blocks "
-                                         "nk x W x B x 16 B + 48 N (x, r0 in; v out)" if assembled else
+                             "formula": ("stored coupling values pairs x W x padded rows x 8 B, exponents "
+                                         "pairs x padded rows x 2 B, diagonal blocks nk x W x B x 16 B, "
+                                         "48 N (x, r0 in; v out)" if assembled else
                                          "table slabs of the used (order, kappa) pairs x W x B x 32 B + "
                                          "diagonal blocks nk x W x B x 16 B + angular terms x 36 B + "
                                          "slot maps + 48 N (x, r0 in; v out)")},
