@@ -2936,7 +2936,7 @@ struct gade_solver {
     int2 *d_K, *d_A;            /* fixed-point limbs of K (per table set) and of A (per pulse), see AsmLay */
     unsigned short *d_Ke, *d_Ae;   /* row exponents: [table set][pairs][3][Bp], [pulse][pairs][Bp] */
     int rdiag;                  /* S(k) is real and i h dt/2 h0(k) imaginary */
-    int dsym;                   /* the diagonal blocks are symmetric to rounding: the block-LU solves invert them */
+    int dsym;                   /* the diagonal blocks are symmetric to rounding and the block-LU solves invert them (check_diag_known) */
     int halves;                 /* the ELL slots are laid out by column half and spline offset */
     int APp, RMA;               /* row positions of the assembled layout (Bp of AsmLay), most of one chunk */
     int *d_pad, *d_off, *d_prow, *d_pq;
@@ -3545,9 +3545,12 @@ static int solver_create(const gade_problem *p, int npulse, const double *dts, c
         cudaFuncSetAttribute(k_precond_tma<double, 32, 8>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm64);
         /* k_precond_fx is written for 16 chain columns (half-bandwidth <= 16,
            both bases' own ordering) and must fit an SM (Bp <= 4,500); wider
-           bands and larger blocks keep the FP64 kernel */
+           bands and larger blocks keep the FP64 kernel, and so do batches whose
+           second copy of the factors would take a tenth of the free memory */
         const size_t smx = pf_smem(s->Bp, s->nch);
-        if (s->bwp == PF_BW && smx <= 220 * 1024) {
+        size_t fr = 0, tot = 0;
+        if (cudaMemGetInfo(&fr, &tot) != cudaSuccess) fr = 0;
+        if (s->bwp == PF_BW && smx <= 220 * 1024 && 2 * sizeof(int4) * NP * s->fstride < fr / 10) {
             cudaFuncSetAttribute(k_precond_fx, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smx);
             UP(s->d_XL, (const int4 *)nullptr, NP * s->fstride);
             UP(s->d_XU, (const int4 *)nullptr, NP * s->fstride);
@@ -4731,6 +4734,44 @@ static float step_cost(const gade_solver *s, float tables_ms, float apply_ms)
     return tables_ms + (s->prec == GADE_PREC_MIXED ? 1.0f : 3.0f) * apply_ms;
 }
 
+/* Whether BiCGSTAB may take p for D M^-1 p (batch_seq_iters): the blocks are
+   symmetric, and the solves invert them to 2e-13 of a random right-hand side,
+   a fifth of the tightest tolerance in use (measured: 2e-14 to 3e-14 on every
+   configuration, 1e-15 for a state; without pivoting the LU of other blocks
+   could be worse).  One solve and one apply with zero couplings per pulse. */
+static int check_diag_known(gade_solver *s)
+{
+    if (!s->dsym || s->prec != GADE_PREC_FP64) return GADE_OK;
+    const size_t n = (size_t)s->n;
+    std::vector<double2> p(n), v(n);
+    unsigned long long seed = 88172645463325252ull;
+    auto rnd = [&] {
+        seed ^= seed << 13; seed ^= seed >> 7; seed ^= seed << 17;
+        return (double)(seed >> 11) * 0x1p-52 - 1.0;
+    };
+    double pp = 0;
+    for (double2 &e : p) { e.x = rnd(); e.y = rnd(); pp += e.x * e.x + e.y * e.y; }
+    for (int k = 0; k < s->npulse; k++)
+        CK(cudaMemcpyAsync(s->s + k * n, p.data(), n * sizeof(double2), cudaMemcpyHostToDevice, s->stream));
+    CK(cudaMemsetAsync(s->d_coef, 0, sizeof(double2) * (size_t)s->npulse * s->lmax * 3, s->stream));
+    int rc = launch_assemble(s, s->stream);
+    if (rc || (rc = launch_precond(s, PC_PLAIN, s->s, nullptr, nullptr, s->z, s->stream))) return rc;
+    VecP V = {}; V.out0 = s->tmp1; V.in0 = s->r0;
+    if ((rc = launch_apply(s, s->z, AX_R0V, V, RED_R0V, s->stream))) return rc;
+    for (int k = 0; k < s->npulse && s->dsym; k++) {
+        CK(cudaMemcpyAsync(v.data(), s->tmp1 + k * n, n * sizeof(double2), cudaMemcpyDeviceToHost, s->stream));
+        CK(cudaStreamSynchronize(s->stream));
+        double rr = 0;
+        for (size_t i = 0; i < n; i++) {
+            const double a = v[i].x - p[i].x, b = v[i].y - p[i].y;
+            rr += a * a + b * b;
+        }
+        if (!(rr <= 2e-13 * 2e-13 * pp)) s->dsym = 0;
+    }
+    s->has_time = 0;
+    return GADE_OK;
+}
+
 static int choose_operator(gade_solver *s)
 {
     s->mf_ms = s->split_ms[s->nsplit >= 1 && s->nsplit <= 4 ? s->nsplit : 0];
@@ -4746,6 +4787,7 @@ static int choose_operator(gade_solver *s)
         rc = time_fp64_apply(s, &s->asm_ms[part]);
     }
     if (!rc) rc = time_step_tables(s, &tab_asm);
+    if (!rc) rc = check_diag_known(s);
     if (rc) { s->use_asm = 0; return rc; }
     /* by the cost model, not by the two times: where these are close the choice,
        and with it the order of the sums, would differ between solvers of one
@@ -5400,7 +5442,10 @@ static int batch_choose_operator(gade_batch *b)
     if ((rc = time_fp64_apply(s, &mf)) || (rc = time_step_tables(s, &tmf))) return rc;
     s->use_asm = 1;
     s->asm_part = 0;
-    if ((rc = time_fp64_apply(s, &am)) || (rc = time_step_tables(s, &tam))) { s->use_asm = 0; return rc; }
+    if ((rc = time_fp64_apply(s, &am)) || (rc = time_step_tables(s, &tam)) || (rc = check_diag_known(s))) {
+        s->use_asm = 0;
+        return rc;
+    }
     s->mf_ms = mf;
     s->asm_ms[0] = am;
     s->asm_ms[1] = 0.f;
