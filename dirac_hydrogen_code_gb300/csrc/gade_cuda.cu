@@ -1375,8 +1375,8 @@ __host__ __device__ __forceinline__ unsigned asm_smem(int XS, int W, int RM, boo
  * entries of x that are as much smaller: products of the window's common
  * exponent would lose them).
  * N = 53,040 (41.7M values, 0.33 GB): 188 us with FP64 products (FP64 pipe
- * bound), 81 us now (4.1 TB/s; each CTA's staging, exchange and epilogue do not
- * overlap its stream); N = 244,000 (2.8 GB): 1.36 ms, now 0.50 ms (5.6 TB/s).
+ * bound), 76 us now (4.3 TB/s; each CTA's staging, exchange and epilogue do not
+ * overlap its stream); N = 244,000 (2.8 GB): 1.36 ms, now 0.48 ms (5.8 TB/s).
  * HL: the halves layout (slot 15 h + t of a row of spline s is spline
  * s - 7 + t of half h); otherwise the slots' columns come from a table.
  */
