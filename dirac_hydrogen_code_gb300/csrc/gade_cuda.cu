@@ -1405,8 +1405,6 @@ __global__ void __launch_bounds__(256, 3)
     const int RMA = P.RMA, NPR = RMA >> 1, NG = nt / NPR;        /* row pairs of a chunk, thread groups */
     const int grp = tid / NPR, rp = tid - grp * NPR;
     const int half = tid / RMA, trow = tid - half * RMA;   /* diagonal blocks and output: two threads per row */
-    /* AX_R0V, AX_TS: D x where the caller knows it (NULL: formed here) */
-    const C *dx = !SEP && (mode == AX_R0V || mode == AX_TS) ? (const C *)V.in1 : nullptr;
     __shared__ int s_pc, s_pw, s_ex[ASM_GB];
     for (int pc = P.seg_ptr[blockIdx.y]; pc < P.seg_ptr[blockIdx.y + 1]; pc = *(volatile int *)&s_pc + 1) {
     const int4 pd = P.pieces[pc];
@@ -1426,7 +1424,7 @@ __global__ void __launch_bounds__(256, 3)
     };
     __syncthreads();                          /* the previous piece is done with shared memory */
     if (tid == 0) { s_pc = pc; s_pw = pd.w; } /* read back after the next barrier */
-    const bool diag = (pd.w & 0xffff) == 0 && !dx;   /* the unit's first piece has the diagonal blocks */
+    const bool diag = (pd.w & 0xffff) == 0;   /* the unit's first piece has the diagonal blocks */
     if (diag) {
         const size_t vo = (size_t)pulse * P.vstride + (size_t)r * B;
         const C *xb = x + (size_t)r * B;
@@ -1647,7 +1645,6 @@ __global__ void __launch_bounds__(256, 3)
     double v[NRED] = {0, 0, 0, 0};
     if (half == 0 && i >= 0) {
         const size_t gi = (size_t)pulse * P.vstride + (size_t)r * B + i;
-        if (dx) accH = cadd(accH, dx[gi]);
         apply_epilogue<C, SEP>(mode, V, gi, accS, accH, accD, v);
     }
     if (red.kind != RED_NONE) reduce_part(red, v, shred, (unsigned)u);
@@ -2936,7 +2933,6 @@ struct gade_solver {
     int2 *d_K, *d_A;            /* fixed-point limbs of K (per table set) and of A (per pulse), see AsmLay */
     unsigned short *d_Ke, *d_Ae;   /* row exponents: [table set][pairs][3][Bp], [pulse][pairs][Bp] */
     int rdiag;                  /* S(k) is real and i h dt/2 h0(k) imaginary */
-    int dsym;                   /* the diagonal blocks are symmetric to rounding and the block-LU solves invert them (check_diag_known) */
     int halves;                 /* the ELL slots are laid out by column half and spline offset */
     int APp, RMA;               /* row positions of the assembled layout (Bp of AsmLay), most of one chunk */
     int *d_pad, *d_off, *d_prow, *d_pq;
@@ -3280,46 +3276,6 @@ static void pack_factors(const gade_setup *su, int nk, int nch, int bw, int bwp,
     }
 }
 
-/* Whether the diagonal blocks S(k) and i h dt/2 h0(k) are symmetric up to their
-   quadrature's rounding, |M_ij - M_ji| <= 1e-13 sqrt(|M_ii M_jj|).  The
-   preconditioner holds the exact LU of D^T (tools/superlu.c:142-152), so its
-   solves then also invert D: D (M^-1 p) is p up to the solve's rounding, which
-   is relative to p, a vector of the residual's size, and the FP64 BiCGSTAB
-   products need no diagonal blocks.  check_diag_known measures what the
-   asymmetry and the rounding leave; a limit of 8 2^-53 here refused the blocks
-   of N = 53,040 (8 steps 6.40 ms, without their products 6.12) and N = 244,000
-   (2 steps 9.14, 8.95), whose measured residuals are those of exactly symmetric
-   ones. */
-static int diag_symmetric(const gade_setup *su, int B)
-{
-    const size_t WB = (size_t)su->W * B;
-    std::vector<gc64> row((size_t)B * B), dg(B);
-    for (int m = 0; m < 2; m++) {
-        const gc64 *src = m ? su->Hst_ell : su->S_ell;
-        for (int k = 0; k < su->nk; k++) {
-            const gc64 *M = src + k * WB;
-            for (int i = 0; i < B; i++) dg[i] = gc64{0, 0};
-            for (int j = 0; j < su->W; j++)
-                for (int i = 0; i < B; i++) {
-                    const int c = su->ell_col[(size_t)j * B + i];
-                    if (c < 0) continue;
-                    row[(size_t)i * B + c] = M[(size_t)j * B + i];
-                    if (c == i) dg[i] = M[(size_t)j * B + i];
-                }
-            for (int j = 0; j < su->W; j++)
-                for (int i = 0; i < B; i++) {
-                    const int c = su->ell_col[(size_t)j * B + i];
-                    if (c <= i) continue;      /* every entry above the diagonal against its mirror (symmetric pattern) */
-                    const gc64 a = row[(size_t)i * B + c], b = row[(size_t)c * B + i];
-                    const double lim = 1e-13 *
-                                       sqrt(hypot(dg[i].re, dg[i].im)) * sqrt(hypot(dg[c].re, dg[c].im));
-                    if (!(fabs(a.re - b.re) <= lim && fabs(a.im - b.im) <= lim)) return 0;
-                }
-        }
-    }
-    return 1;
-}
-
 /*
  * Shared by gade_solver_create (one pulse) and gade_batch_create (npulse
  * pulses on one set of angular tables, h0 and S).  Pulse k has its own time
@@ -3423,7 +3379,6 @@ static int solver_create(const gade_problem *p, int npulse, const double *dts, c
         for (int k = 0; k < npulse && s->zskip; k++)
             if (!gade_dkb_zero(p, (const gc64 *)(gext + 2 * per * k))) s->zskip = 0;
     }
-    s->dsym = diag_symmetric(su, p->blkdim);
     s->rdiag = 1;
     for (size_t e = 0; e < (size_t)su->nk * su->W * p->blkdim && s->rdiag; e++)
         if (su->S_ell[e].im != 0.0 || su->Hst_ell[e].re != 0.0) s->rdiag = 0;
@@ -4738,44 +4693,6 @@ static float step_cost(const gade_solver *s, float tables_ms, float apply_ms)
     return tables_ms + (s->prec == GADE_PREC_MIXED ? 1.0f : 3.0f) * apply_ms;
 }
 
-/* Whether BiCGSTAB may take p for D M^-1 p (batch_seq_iters): the blocks are
-   symmetric, and the solves invert them to 2e-13 of a random right-hand side,
-   a fifth of the tightest tolerance in use (measured: 2e-14 to 3e-14 on every
-   configuration, 1e-15 for a state; without pivoting the LU of other blocks
-   could be worse).  One solve and one apply with zero couplings per pulse. */
-static int check_diag_known(gade_solver *s)
-{
-    if (!s->dsym || s->prec != GADE_PREC_FP64) return GADE_OK;
-    const size_t n = (size_t)s->n;
-    std::vector<double2> p(n), v(n);
-    unsigned long long seed = 88172645463325252ull;
-    auto rnd = [&] {
-        seed ^= seed << 13; seed ^= seed >> 7; seed ^= seed << 17;
-        return (double)(seed >> 11) * 0x1p-52 - 1.0;
-    };
-    double pp = 0;
-    for (double2 &e : p) { e.x = rnd(); e.y = rnd(); pp += e.x * e.x + e.y * e.y; }
-    for (int k = 0; k < s->npulse; k++)
-        CK(cudaMemcpyAsync(s->s + k * n, p.data(), n * sizeof(double2), cudaMemcpyHostToDevice, s->stream));
-    CK(cudaMemsetAsync(s->d_coef, 0, sizeof(double2) * (size_t)s->npulse * s->lmax * 3, s->stream));
-    int rc = launch_assemble(s, s->stream);
-    if (rc || (rc = launch_precond(s, PC_PLAIN, s->s, nullptr, nullptr, s->z, s->stream))) return rc;
-    VecP V = {}; V.out0 = s->tmp1; V.in0 = s->r0;
-    if ((rc = launch_apply(s, s->z, AX_R0V, V, RED_R0V, s->stream))) return rc;
-    for (int k = 0; k < s->npulse && s->dsym; k++) {
-        CK(cudaMemcpyAsync(v.data(), s->tmp1 + k * n, n * sizeof(double2), cudaMemcpyDeviceToHost, s->stream));
-        CK(cudaStreamSynchronize(s->stream));
-        double rr = 0;
-        for (size_t i = 0; i < n; i++) {
-            const double a = v[i].x - p[i].x, b = v[i].y - p[i].y;
-            rr += a * a + b * b;
-        }
-        if (!(rr <= 2e-13 * 2e-13 * pp)) s->dsym = 0;
-    }
-    s->has_time = 0;
-    return GADE_OK;
-}
-
 static int choose_operator(gade_solver *s)
 {
     s->mf_ms = s->split_ms[s->nsplit >= 1 && s->nsplit <= 4 ? s->nsplit : 0];
@@ -4791,7 +4708,6 @@ static int choose_operator(gade_solver *s)
         rc = time_fp64_apply(s, &s->asm_ms[part]);
     }
     if (!rc) rc = time_step_tables(s, &tab_asm);
-    if (!rc) rc = check_diag_known(s);
     if (rc) { s->use_asm = 0; return rc; }
     /* by the cost model, not by the two times: where these are close the choice,
        and with it the order of the sums, would differ between solvers of one
@@ -5207,13 +5123,10 @@ static int batch_seq_iters(gade_batch *b, int K, cudaStream_t st)
     const size_t rsm = sizeof(double) * NRED * s->upd_block;
     for (int it = 0; it < K; it++) {
         if ((rc = launch_precond(s, PC_P, s->r, s->v, s->p, s->y, st, PRED_RUN))) return rc;
-        /* y = M^-1 p with M = D^T = D: the diagonal blocks' part D y of A y is p
-           itself (and D z is s) */
-        const bool dknown = s->dsym && s->use_asm;
-        VecP A1 = {}; A1.out0 = s->v; A1.in0 = s->r0; A1.in1 = dknown ? s->p : nullptr;
+        VecP A1 = {}; A1.out0 = s->v; A1.in0 = s->r0;
         if ((rc = launch_apply(s, s->y, AX_R0V, A1, RED_R0V, st, PRED_RUN))) return rc;
         if ((rc = launch_precond(s, PC_S, s->r, s->v, s->s, s->z, st, PRED_RUN))) return rc;
-        VecP A2 = {}; A2.out0 = s->t; A2.in0 = s->s; A2.in1 = dknown ? s->s : nullptr;
+        VecP A2 = {}; A2.out0 = s->t; A2.in0 = s->s;
         if ((rc = launch_apply(s, s->z, AX_TS, A2, RED_TS, st, PRED_RUN))) return rc;
         RedP red = make_red(s, s->d_sc, RED_UPDATE, PRED_RUN);
         launch_pdl(k_update<double>, dim3(s->upd_grid, s->nslot), dim3(s->upd_block), rsm, st,
@@ -5446,10 +5359,7 @@ static int batch_choose_operator(gade_batch *b)
     if ((rc = time_fp64_apply(s, &mf)) || (rc = time_step_tables(s, &tmf))) return rc;
     s->use_asm = 1;
     s->asm_part = 0;
-    if ((rc = time_fp64_apply(s, &am)) || (rc = time_step_tables(s, &tam)) || (rc = check_diag_known(s))) {
-        s->use_asm = 0;
-        return rc;
-    }
+    if ((rc = time_fp64_apply(s, &am)) || (rc = time_step_tables(s, &tam))) { s->use_asm = 0; return rc; }
     s->mf_ms = mf;
     s->asm_ms[0] = am;
     s->asm_ms[1] = 0.f;
