@@ -379,11 +379,11 @@ struct OpP {
     /* assembled operator (k_apply_asm): this step's coupling values
        A[pair][W][B] and the coupled block of every (block row, block) pair;
        a piece's order range is then a pair range */
-    const void *A;                 /* fixed-point limbs (int2), or float for the complex64 instance */
-    const unsigned short *Ae;      /* [pair][Bp] biased exponent of a row's values (fixed point) */
+    const void *A;                 /* words (gade_fx.cuh), or float for the complex64 instance */
+    const unsigned short *Ae;      /* [pair][Bp] exponent of a row's words */
     const int *pair_c;
     size_t astride, aestride;      /* values per pulse of A and of Ae */
-    const int *pad, *off, *prow;   /* row positions of the fixed-point values (AsmLay) */
+    const int *pad, *off, *prow;   /* row positions of the words (AsmLay) */
     int Bp, npairs, RMA;           /* row positions; pairs; most row positions of one chunk (even) */
 };
 
@@ -1141,10 +1141,11 @@ __global__ void __launch_bounds__(256, std::is_same<R, dd>::value ? GADE_DD_MINB
  * of the chunk's splines to an even count, so that two neighbouring rows make
  * one aligned 16-byte load), at row positions off[q] .. off[q] + RMq - 1:
  *   A [off[q] npairs W + (p W + slot) RMq + row], K with 3 factors per pair.
- * K and A are fixed-point limbs (int2) with one exponent per (pair, factor,
- * row position) and (pair, row position).  Ke holds the upper 16 bits of a
- * bound of the row's largest |K| (its exponent field is the row's exponent),
- * Ae the biased exponent of the step's values.
+ * K and A are words with an exponent of their own each (gade_fx.cuh), as
+ * offsets from one exponent per (pair, factor, row position) and (pair, row
+ * position).  Ke holds the upper 16 bits of a bound of the row's largest |K|
+ * (its exponent field is the row's exponent), Ae the exponent of the step's
+ * values (0: the row has none, ASM_NAN: not finite).
  */
 struct AsmLay {
     const int *pad, *off;          /* [nchunk] padded rows, first row position */
@@ -1175,7 +1176,7 @@ __global__ void k_build_K(int2 *__restrict__ K, unsigned short *__restrict__ Ke,
     const int ia = (a - base) / 2;
     const int kk = row_kidx[pair_r[p]];
     double acc[30];
-    double mx = 0.0;
+    unsigned long long mx = 0;                   /* bits of the largest |value|: a NaN stays the largest */
     for (int t = 0; t < W; t++) {
         double v = 0.0;
         for (int k = le_ptr[p]; k < le_ptr[p + 1]; k++) {
@@ -1187,14 +1188,14 @@ __global__ void k_build_K(int2 *__restrict__ K, unsigned short *__restrict__ Ke,
             v = fma(m.d, a1k[e], v);
         }
         acc[t] = v;
-        mx = fmax(mx, fabs(v));
+        mx = max(mx, (unsigned long long)__double_as_longlong(v) & 0x7FFFFFFFFFFFFFFFull);
     }
-    const unsigned short u = fx_bound16(mx);
+    const unsigned short u = fx_bound16_bits(mx);
     const int em = u >> 4 ? u >> 4 : 1;
     Ke[((size_t)p * 3 + ia) * L.Bp + g] = u;
     const int q = L.pq[g] >> 16, RMq = L.pad[q];
     int2 *Kq = K + (size_t)L.off[q] * L.npairs * 3 * W + ((size_t)p * 3 + ia) * W * RMq + (g - L.off[q]);
-    for (int t = 0; t < W; t++) Kq[(size_t)t * RMq] = fx_split(fx_from(acc[t], em, FX_UPA));
+    for (int t = 0; t < W; t++) Kq[(size_t)t * RMq] = fx_word(acc[t], em);
 }
 
 /* complex64 copies of the step's values in the layout of k_apply_asm32
@@ -1212,17 +1213,20 @@ struct A32Map {
  * One thread per (pair, two rows) and nsl of the W slots in sequence; grid
  * (chunk, groups of blockDim / (RMA/2) pairs, groups of PT pulses x slot
  * groups).  The rows' exponents are known before
- * their values are: |A| <= sum_ia |w_ia| max|K_ia|.  Each w_ia is scaled once
- * per row to a fixed-point factor with A = (sum_ia w_ia K_ia) >> 58, so a
- * value costs nine integer multiply-adds and the kernel runs at the memory
- * rate (24 bytes in per value and pulse group, 8 out per pulse): 190 us at
- * 41.7M values, 6.9 TB/s (209 us with three FP64 DFMA per value, which bound it).  With PT > 1 the pulses of a group share the
- * reads of K (batches whose pulses share the radial tables: 8 pulses 1.64 ms,
- * now 0.69 ms).
+ * their values are: |A| <= sum_ia |w_ia| max|K_ia|.  The three products of a
+ * value are aligned to their largest and summed on the integer units, to
+ * 2^-53 of that product, so every value is as accurate as in FP64.  One pulse
+ * runs at the memory rate (24 bytes in per value and pulse group, 8 out per
+ * pulse): 196 us at 41.7M values, 6.8 TB/s (209 us with three FP64 DFMA per
+ * value, which bound it).  With PT = 2 the pulses of a group share the reads
+ * of K (batches whose pulses share the radial tables), and the integer units
+ * bind: 8 pulses 1.23 ms (one pulse at a time 1.44, four 1.39; three FP64 DFMA
+ * 1.64).
  */
+#define ASM_NAN 0xFFFF    /* row exponent where a factor or a value is not finite */
 #define ASB_PF 1    /* slots prefetched ahead of the five being loaded (5: 204 us, 10: 238 us against 190 us at 41.7M values) */
 template <int PT>
-__global__ void __launch_bounds__(128) k_assemble(int2 *__restrict__ A, unsigned short *__restrict__ Ae, A32Map F,
+__global__ void __launch_bounds__(128, 6) k_assemble(int2 *__restrict__ A, unsigned short *__restrict__ Ae, A32Map F,
                                                   const int2 *__restrict__ K, const unsigned short *__restrict__ Ke,
                                                   AsmLay L, const int *__restrict__ pair_par,
                                                   const double2 *__restrict__ coef, int2 lpar,
@@ -1257,9 +1261,8 @@ __global__ void __launch_bounds__(128) k_assemble(int2 *__restrict__ A, unsigned
     ushort2 ke[3];
 #pragma unroll
     for (int ia = 0; ia < 3; ia++) ke[ia] = *(const ushort2 *)(Ke + (size_t)ia * L.Bp);
-    int2 w[PT][3][2];
-    int pulse[PT];
-    float f0[PT][2], f1[PT][2];
+    int2 w[PT][3];
+    int ew[PT][3], ea[PT][2], pulse[PT];
 #pragma unroll
     for (int j = 0; j < PT; j++) {
         pulse[j] = -1;
@@ -1267,38 +1270,35 @@ __global__ void __launch_bounds__(128) k_assemble(int2 *__restrict__ A, unsigned
         pulse[j] = plist ? plist[s0 + j] : 0;
         const double2 *cp = coef + (size_t)pulse[j] * lmax * 3 + cb;
         const double wv[3] = {cp[0].y, cp[1].y, cp[2].y};
+#pragma unroll
+        for (int ia = 0; ia < 3; ia++) {
+            /* w = W 2^(ew - 1079) */
+            const unsigned long long bits = (unsigned long long)__double_as_longlong(wv[ia]);
+            int e = (int)((bits >> 52) & 0x7FF);
+            long long m = (long long)(bits & 0xFFFFFFFFFFFFFull);
+            if (e) m |= 1ll << 52; else e = 1;
+            ew[j][ia] = m ? e : FX_ZERO;
+            w[j][ia] = fx_limbs((long long)bits < 0 ? -(m << 4) : m << 4);
+        }
         unsigned short em2[2];
 #pragma unroll
         for (int rr = 0; rr < 2; rr++) {
             double b = 0.0;
 #pragma unroll
             for (int ia = 0; ia < 3; ia++) b = fma(fabs(wv[ia]), fx_bound_to(rr ? ke[ia].y : ke[ia].x), b);
-            int em = fx_exp((unsigned)__double2hiint(b));     /* 2047: a coefficient is not finite */
-            if (em == 0) em = 1;
-#pragma unroll
-            for (int ia = 0; ia < 3; ia++) {
-                /* w 2^(ek - em + 58) */
-                const int u = (rr ? ke[ia].y : ke[ia].x) >> 4, ek = u ? u : 1;
-                const unsigned long long bits = (unsigned long long)__double_as_longlong(wv[ia]);
-                int ew = (int)((bits >> 52) & 0x7FF);
-                unsigned long long m = bits & 0xFFFFFFFFFFFFFull;
-                if (ew) m |= 1ull << 52; else ew = 1;
-                const int sh = ew + ek - em - 1017;
-                m = sh >= 0 ? (sh > 6 ? 0ull : m << sh) : (sh < -63 ? 0ull : m >> -sh);
-                w[j][ia][rr] = fx_split((long long)bits < 0 ? -(long long)m : (long long)m);
-            }
-            em2[rr] = (unsigned short)em;
-            if (F.A32) {
-                /* N 2^(em - 1079) as a float in two factors */
-                const int k = em - 1079, k1 = k < -126 ? -126 : (k > 127 ? 127 : k);
-                const int k2 = k - k1 < -126 ? -126 : (k - k1 > 127 ? 127 : k - k1);
-                f0[j][rr] = em == 2047 ? __int_as_float(0x7FC00000) : __int_as_float((k1 + 127) << 23);
-                f1[j][rr] = __int_as_float((k2 + 127) << 23);
-            }
+            const int em = fx_exp((unsigned)__double2hiint(b));     /* 2047: a factor or a value is not finite */
+            ea[j][rr] = em + 1;
+            em2[rr] = em == 2047 ? ASM_NAN : b == 0.0 ? 0 : em + 1;
         }
         if (t0 == 0) *(ushort2 *)(Ae + (size_t)pulse[j] * aestride) = make_ushort2(em2[0], em2[1]);
     }
     float *A32 = F.A32 ? F.A32 + ((size_t)q * L.npairs + p) * W * F.RMp : nullptr;
+    int ek[3][2];                                  /* the exponents of the rows of K */
+#pragma unroll
+    for (int ia = 0; ia < 3; ia++) {
+        ek[ia][0] = max(ke[ia].x >> 4, 1);
+        ek[ia][1] = max(ke[ia].y >> 4, 1);
+    }
 #pragma unroll 5
     for (int t = t0; t < t1; t++) {
         if ((t - t0) % 5 == 0) prefetch(t + ASB_PF, t + ASB_PF + 5);
@@ -1308,30 +1308,50 @@ __global__ void __launch_bounds__(128) k_assemble(int2 *__restrict__ A, unsigned
 #pragma unroll
         for (int j = 0; j < PT; j++) {
             if (PT > 1 && pulse[j] < 0) continue;
-            long long N[2];
+            int2 v[2];
 #pragma unroll
             for (int rr = 0; rr < 2; rr++) {
+                int key[3];
+#pragma unroll
+                for (int ia = 0; ia < 3; ia++) key[ia] = ew[j][ia] + ek[ia][rr] - ((rr ? k[ia].z : k[ia].x) & FX_OFF);
+                const int C = max(max(key[0], key[1]), key[2]);
                 long long h = 0, m = 0;
 #pragma unroll
                 for (int ia = 0; ia < 3; ia++) {
-                    const int kh = rr ? k[ia].z : k[ia].x, kl = rr ? k[ia].w : k[ia].y;
-                    h += (long long)kh * w[j][ia][rr].x;
-                    m += (long long)kh * w[j][ia][rr].y;
-                    m += (long long)kl * w[j][ia][rr].x;
+                    int kh, kl;
+                    fx_take(rr ? k[ia].z : k[ia].x, rr ? k[ia].w : k[ia].y, C - key[ia], kh, kl);
+                    fx_mad(h, kh, w[j][ia].x);
+                    fx_mad(m, kh, w[j][ia].y);
+                    fx_mad(m, kl, w[j][ia].x);
                 }
-                N[rr] = h + ((m + (1ll << (FX_LB - 1))) >> FX_LB);
+                /* the value is S 2^(C - 2103), |S| < 2^61; its word: S shifted up to bit 62 */
+                const long long S = (h << 5) + (m >> (FX_WB - 5)), sg = S ^ (S >> 63);
+                int z = __clz((int)(sg >> 32));
+                if (z == 32) z += __clz((int)sg);
+                int off = ea[j][rr] + 1017 - C + z;
+                /* below 2^-183 of the row nothing is left of it */
+                const long long T = S == 0 || off >= FX_OFF + 56 ? 0 : fx_shr(S << (z - 1), max(off - FX_OFF, 0));
+                off = T == 0 ? FX_OFF : min(off, FX_OFF);
+                v[rr] = fx_word_of(T, off);
+                if (F.A32) {
+                    const int c = rr ? q1 & 0xffff : q0 & 0xffff;
+                    if (c != 0xffff) {
+                        /* T 2^(ea - off - 1085) as a float, from its upper 31 bits, in two factors */
+                        const int e = ea[j][rr] - off - 1053, e1 = max(-126, min(e, 127)), e2 = max(-126, min(e - e1, 127));
+                        const float f = (float)(int)(T >> 32) * __int_as_float((e1 + 127) << 23) * __int_as_float((e2 + 127) << 23);
+                        A32[(size_t)pulse[j] * F.astride + (size_t)t * F.RMp + c] =
+                            ea[j][rr] == 2048 ? __int_as_float(0x7FC00000) : f;
+                    }
+                }
             }
-            const int2 v0 = fx_split(N[0]), v1 = fx_split(N[1]);
-            *(int4 *)(A + (size_t)pulse[j] * astride + (size_t)t * RMq) = make_int4(v0.x, v0.y, v1.x, v1.y);
-            if (F.A32) {
-                float *d = A32 + (size_t)pulse[j] * F.astride + (size_t)t * F.RMp;
-                if ((q0 & 0xffff) != 0xffff) d[q0 & 0xffff] = __ll2float_rn(N[0]) * f0[j][0] * f1[j][0];
-                if ((q1 & 0xffff) != 0xffff) d[q1 & 0xffff] = __ll2float_rn(N[1]) * f0[j][1] * f1[j][1];
-            }
+            *(int4 *)(A + (size_t)pulse[j] * astride + (size_t)t * RMq) = make_int4(v[0].x, v[0].y, v[1].x, v[1].y);
         }
     }
 }
 
+#define ASM_GS 8                       /* slots of a row summed with one alignment */
+#define ASM_GPH ((15 + ASM_GS - 1) / ASM_GS)
+#define ASM_XZERO (-20000) /* exponent of a zero entry of x: no product of it is a row's largest */
 #define ASM_GB 16   /* coupled blocks staged per phase: two per warp */
 /* what a piece costs beyond its pairs, in pairs: staging, exchange, the arrival
    count and the next piece's descriptor, 8-12 us of latencies under load where a
@@ -1343,19 +1363,21 @@ __global__ void __launch_bounds__(128) k_assemble(int2 *__restrict__ A, unsigned
 #endif
 
 /* shared memory of k_apply_asm: x windows of the block row (x, x_n, delta;
-   FP64), the staged fixed-point windows of ASM_GB coupled blocks, the slot
-   columns (general layout only), the exchange / reduction buffer.  XS:
+   FP64), the staged windows of ASM_GB coupled blocks as limbs, the slot columns
+   (general layout only), the exchange / reduction buffer, the diagonal blocks'
+   sums, the staged entries' exponents.  XS:
    entries of a window: two halves of RM/2 + 16 columns each (halves layout)
    or the chunk's columns and a zero column */
 __host__ __device__ __forceinline__ int asm_xs(int RM, int CM, bool halves) { return halves ? RM + 32 : (CM + 2) & ~1; }
 __host__ __device__ __forceinline__ unsigned asm_smem(int XS, int W, int RM, bool halves, int nt, unsigned *o_xw,
-                                                      unsigned *o_lc, unsigned *o_red, unsigned *o_xd)
+                                                      unsigned *o_lc, unsigned *o_red, unsigned *o_xd, unsigned *o_xe)
 {
     unsigned o = up32(3u * 16u * XS);
     *o_xw = o;  o = up32(o + 16u * ASM_GB * XS);
     *o_lc = o;  o = up32(o + (halves ? 0u : 2u * W * RM));
     *o_red = o; o = up32(o + 8u * NRED * nt);
     *o_xd = o;  o = up32(o + 3u * 16u * RM);
+    *o_xe = o;  o = up32(o + 2u * ASM_GB * XS);
     return o;
 }
 
@@ -1363,37 +1385,44 @@ __host__ __device__ __forceinline__ unsigned asm_smem(int XS, int W, int RM, boo
  * y = (S + H(t)) x with the assembled couplings: grid (pulse slot, segment)
  * over the same units and pieces as k_apply (a piece's range is a range of
  * (block row, coupled block) pairs).  Per phase of ASM_GB coupled blocks each
- * warp stages windows of x in shared memory as fixed-point limbs with the
- * window's largest exponent.  Then a thread takes two neighbouring rows (one
- * 16-byte load per slot) of every NG-th staged block, all W slots: with the
- * halves layout the slots of a row are consecutive window entries, so the
- * two rows share all but one of the entries they read and no column index is
- * needed.  The products run on the integer units (see above) with one FP64
- * addition per pair, row and component.  The NG partial sums of a row meet in
- * shared memory, where two threads per row add the diagonal blocks in FP64 (their
- * entries near the origin are orders of magnitude above the rest and meet
- * entries of x that are as much smaller: products of the window's common
- * exponent would lose them).
+ * warp stages windows of x in shared memory as limbs with an exponent per
+ * entry.  Then a thread takes two neighbouring rows (one 16-byte load per
+ * slot) of every NG-th staged block, all W slots: with the halves layout the
+ * slots of a row are consecutive window entries, so the two rows share all but
+ * one of the entries they read and no column index is needed.  The products
+ * run on the integer units, ASM_GS slots at a time: the group's largest
+ * product (exponents only) fixes the alignment, then each value is shifted
+ * into place and multiplied.  Near the origin the entries of x and of A rise
+ * over many orders of magnitude within a row's 15 columns; with one exponent
+ * per window and per row instead (76 us below) rows there were off by up to
+ * 1e-13 of their own terms where x starts as r^7, and by 1e-2 where x spans
+ * 24 orders of magnitude.  One FP64 addition per pair, row and component.  The
+ * NG partial sums of a row meet in shared memory, where two threads per row
+ * add the diagonal blocks in FP64.
  * N = 53,040 (41.7M values, 0.33 GB): 188 us with FP64 products (FP64 pipe
- * bound), 76 us now (4.3 TB/s; each CTA's staging, exchange and epilogue do not
- * overlap its stream); N = 244,000 (2.8 GB): 1.36 ms, now 0.48 ms (5.8 TB/s).
+ * bound), 110 us now (3.0 TB/s; some 30 instructions per value and the
+ * staging, exchange and epilogue of each CTA, which do not overlap its
+ * stream); N = 244,000 (2.8 GB): 1.36 ms, now 0.75 ms.  At N = 53,040 two
+ * CTAs with 128 registers and every load of a pair in flight take 110 us,
+ * three with 80 registers (spills) 129-137.
  * HL: the halves layout (slot 15 h + t of a row of spline s is spline
  * s - 7 + t of half h); otherwise the slots' columns come from a table.
  */
 template <bool SEP, bool HL>
-__global__ void __launch_bounds__(256, 3)
+__global__ void __launch_bounds__(256, 2)
     k_apply_asm(OpP P, const double2 *__restrict__ x, int mode, VecP V, RedP red)
 {
     constexpr int HJ = 15;
     typedef double2 C;
     extern __shared__ __align__(32) unsigned char smem_raw[];
     const int XS = asm_xs(P.RMA, P.CM, HL);
-    unsigned oxw, olc, ored, oxd;
-    asm_smem(XS, P.W, P.RMA, HL, blockDim.x, &oxw, &olc, &ored, &oxd);
+    unsigned oxw, olc, ored, oxd, oxe;
+    asm_smem(XS, P.W, P.RMA, HL, blockDim.x, &oxw, &olc, &ored, &oxd, &oxe);
     C *xr = (C *)smem_raw, *xs = xr + XS, *ds = xs + XS;   /* windows of the block row itself: x, x_n, delta (FP64) */
     int4 *xw = (int4 *)(smem_raw + oxw);      /* [ASM_GB][XS] re hi, re lo, im hi, im lo */
     unsigned short *lc = (unsigned short *)(smem_raw + olc);   /* [W][RM] window entry of a slot (general layout) */
     double *shred = (double *)(smem_raw + ored);
+    short *xe = (short *)(smem_raw + oxe);    /* [ASM_GB][XS] exponents of the staged entries */
     C *xd = (C *)(smem_raw + oxd);            /* [row][3] the diagonal blocks' sums: S, H (or D), S delta */
 
     pdl_enter();
@@ -1497,82 +1526,104 @@ __global__ void __launch_bounds__(256, 3)
         const int ng = pd.z - pg < ASM_GB ? pd.z - pg : ASM_GB;
         __syncthreads();     /* staging done / previous group's products done */
         for (int g = wid; g < ng; g += nt >> 5) {
-            /* the window of one coupled block: the largest exponent over the
-               warp, then the limbs (the second read of x hits L1) */
+            /* the window of one coupled block: every entry with the larger exponent
+               of its two parts, v = X 2^(e - 1080) */
             const C *xc = x + (size_t)P.pair_c[pg + g] * B;
             int4 *win = xw + g * XS;
-            unsigned mx = 0;
+            short *we = xe + g * XS;
+            bool bad = false;
 #pragma unroll 5
             for (int c = lane; c < ncols; c += 32) {
                 const int cc = column(c);
                 const C v = cc >= 0 ? xc[cc] : mk<C>(0, 0);
-                mx = max(mx, max((unsigned)__double2hiint(v.x) & 0x7FFFFFFFu,
-                                 (unsigned)__double2hiint(v.y) & 0x7FFFFFFFu));
-            }
-            int em = fx_exp(__reduce_max_sync(0xffffffffu, mx));
-            if (em == 0) em = 1;
-            if (lane == 0) s_ex[g] = em;
-#pragma unroll 5
-            for (int c = lane; c < ncols; c += 32) {
-                const int cc = column(c);
-                const C v = cc >= 0 ? xc[cc] : mk<C>(0, 0);
-                const int2 re = fx_split(fx_from(v.x, em, FX_UPX)), im = fx_split(fx_from(v.y, em, FX_UPX));
+                const unsigned hi = max((unsigned)__double2hiint(v.x) & 0x7FFFFFFFu, (unsigned)__double2hiint(v.y) & 0x7FFFFFFFu);
+                const int em = max(fx_exp(hi), 1);
+                bad |= em == 2047;
+                const int2 re = fx_limbs(fx_from(v.x, em, FX_UPX)), im = fx_limbs(fx_from(v.y, em, FX_UPX));
                 win[c] = make_int4(re.x, re.y, im.x, im.y);
+                we[c] = (v.x == 0.0 && v.y == 0.0) ? (short)ASM_XZERO : (short)em;
             }
+            bad = __any_sync(0xffffffffu, bad);
+            if (lane == 0) s_ex[g] = bad;
         }
         __syncthreads();
         if (act) {
             for (int g = grp; g < ng; g += NG) {
                 const ushort2 ea = *(const ushort2 *)(P.Ae + (size_t)pulse * P.aestride + (size_t)(pg + g) * P.Bp + off +
                                                       2 * rp);
-                const int ex = s_ex[g];
                 const int2 *Av = Aq + (size_t)(pg + g) * W * RMq;
-                if (ex != 2047) {
-                    const int4 *xg = xw + g * XS + (HL ? 2 * rp - hb : 0);
-                    long long h0r = 0, m0r = 0, h0i = 0, m0i = 0, h1r = 0, m1r = 0, h1i = 0, m1i = 0;
+                if (!s_ex[g]) {
+                    const int w0 = HL ? 2 * rp - hb : 0;
+                    const int4 *xg = xw + g * XS + w0;
+                    const short *eg = xe + g * XS + w0;
+                    /* sums of the rows' (re, im), S 2^C, over the groups of slots so far */
+                    long long S0r = 0, S0i = 0, S1r = 0, S1i = 0;
+                    int E0 = 2 * ASM_XZERO, E1 = E0;
 #pragma unroll
-                    for (int hh = 0; hh < 2; hh++) {
-                        int4 b1 = HL ? xg[hh * HW] : make_int4(0, 0, 0, 0);
-                        int4 av[HJ];           /* 15 loads in flight */
+                    for (int gs = 0; gs < 2 * ASM_GPH; gs++) {
+                        const int hh = gs / ASM_GPH, ts = gs % ASM_GPH * ASM_GS;
+                        const int nsl = min(ASM_GS, HJ - ts), sl = hh * HJ + ts;
+                        const int ws = hh * HW + ts;
+                        int4 av[ASM_GS];       /* the group's loads in flight */
 #pragma unroll
-                        for (int t = 0; t < HJ; t++)
-                            av[t] = HL || hh * HJ + t < W ? __ldcs((const int4 *)(Av + (size_t)(hh * HJ + t) * RMq))
-                                                          : make_int4(0, 0, 0, 0);
+                        for (int t = 0; t < ASM_GS; t++)
+                            av[t] = t < nsl && (HL || sl + t < W) ? __ldcs((const int4 *)(Av + (size_t)(sl + t) * RMq))
+                                                                  : make_int4(FX_OFF, 0, FX_OFF, 0);
+                        /* window entry of slot t for the first row; the second row's is one on (halves layout) */
+                        auto at = [&](int t, int rr) {
+                            return HL ? ws + t + rr : (int)lc[min(sl + t, W - 1) * RMA + 2 * rp + rr];
+                        };
+                        int C0 = 2 * ASM_XZERO, C1 = C0;       /* the rows' largest products */
 #pragma unroll
-                        for (int t = 0; t < HJ; t++) {
-                            if (!HL && hh * HJ + t >= W) break;
-                            const int4 a = av[t];
+                        for (int t = 0; t < ASM_GS; t++) {
+                            C0 = max(C0, eg[at(t, 0)] - (av[t].x & FX_OFF));
+                            C1 = max(C1, eg[at(t, 1)] - (av[t].z & FX_OFF));
+                        }
+                        long long h0r = 0, m0r = 0, h0i = 0, m0i = 0, h1r = 0, m1r = 0, h1i = 0, m1i = 0;
+                        int4 b1 = HL ? xg[ws] : make_int4(0, 0, 0, 0);
+#pragma unroll
+                        for (int t = 0; t < ASM_GS; t++) {
                             int4 b0 = b1;
                             if (HL) {
-                                b1 = xg[hh * HW + t + 1];
+                                b1 = xg[ws + t + 1];
                             } else {
-                                b0 = xg[lc[(hh * HJ + t) * RMA + 2 * rp]];
-                                b1 = xg[lc[(hh * HJ + t) * RMA + 2 * rp + 1]];
+                                b0 = xg[at(t, 0)];
+                                b1 = xg[at(t, 1)];
                             }
-                            h0r += (long long)a.x * b0.x;
-                            m0r += (long long)a.x * b0.y;
-                            m0r += (long long)a.y * b0.x;
-                            h0i += (long long)a.x * b0.z;
-                            m0i += (long long)a.x * b0.w;
-                            m0i += (long long)a.y * b0.z;
-                            h1r += (long long)a.z * b1.x;
-                            m1r += (long long)a.z * b1.y;
-                            m1r += (long long)a.w * b1.x;
-                            h1i += (long long)a.z * b1.z;
-                            m1i += (long long)a.z * b1.w;
-                            m1i += (long long)a.w * b1.z;
+                            int h, l;
+                            fx_take(av[t].x, av[t].y, C0 - eg[at(t, 0)] + (av[t].x & FX_OFF), h, l);
+                            fx_mad(h0r, h, b0.x);
+                            fx_mad(m0r, h, b0.y);
+                            fx_mad(m0r, l, b0.x);
+                            fx_mad(h0i, h, b0.z);
+                            fx_mad(m0i, h, b0.w);
+                            fx_mad(m0i, l, b0.z);
+                            fx_take(av[t].z, av[t].w, C1 - eg[at(t, 1)] + (av[t].z & FX_OFF), h, l);
+                            fx_mad(h1r, h, b1.x);
+                            fx_mad(m1r, h, b1.y);
+                            fx_mad(m1r, l, b1.x);
+                            fx_mad(h1i, h, b1.z);
+                            fx_mad(m1i, h, b1.w);
+                            fx_mad(m1i, l, b1.z);
                         }
+                        fx_join(S0r, E0, fx_sum(h0r, m0r), C0);
+                        fx_join(S0i, E0, fx_sum(h0i, m0i), C0);
+                        fx_join(S1r, E1, fx_sum(h1r, m1r), C1);
+                        fx_join(S1i, E1, fx_sum(h1i, m1i), C1);
+                        E0 = max(E0, C0);
+                        E1 = max(E1, C1);
                     }
-                    const long long rnd = 1ll << (FX_LB - 1);
-                    if (ea.x == 2047 || ea.y == 2047) {
+                    if (ea.x == 0) S0r = S0i = 0;          /* a row without values */
+                    if (ea.y == 0) S1r = S1i = 0;
+                    if (ea.x == ASM_NAN || ea.y == ASM_NAN) {
                         acc0 = mk<C>(__longlong_as_double(0x7FF8000000000000ll), __longlong_as_double(0x7FF8000000000000ll));
                         acc1 = acc0;
                     } else {
-                        const int e0 = ea.x + ex - 2101, e1 = ea.y + ex - 2101;
-                        acc0.x = fx_add(acc0.x, h0r + ((m0r + rnd) >> FX_LB), e0);
-                        acc0.y = fx_add(acc0.y, h0i + ((m0i + rnd) >> FX_LB), e0);
-                        acc1.x = fx_add(acc1.x, h1r + ((m1r + rnd) >> FX_LB), e1);
-                        acc1.y = fx_add(acc1.y, h1i + ((m1i + rnd) >> FX_LB), e1);
+                        const int e0 = ea.x + E0 - 2101, e1 = ea.y + E1 - 2101;
+                        acc0.x = fx_add(acc0.x, S0r, e0);
+                        acc0.y = fx_add(acc0.y, S0i, e0);
+                        acc1.x = fx_add(acc1.x, S1r, e1);
+                        acc1.y = fx_add(acc1.y, S1i, e1);
                     }
                 } else {
                     /* an infinity or NaN in the window: products in FP64, so that it
@@ -1581,14 +1632,13 @@ __global__ void __launch_bounds__(256, 3)
                     for (int rr = 0; rr < 2; rr++) {
                         const int row = P.prow[off + 2 * rp + rr], e = rr ? ea.y : ea.x;
                         if (row < 0) continue;
-                        const double sc = e == 2047 ? __longlong_as_double(0x7FF8000000000000ll)
-                                                    : pow2d(e - 1079 < -1022 ? -1022 : e - 1079);
                         for (int t = 0; t < W; t++) {
                             const int w = HL ? (t / HJ) * HW + 2 * rp + rr - hb + t % HJ : lc[t * RMA + 2 * rp + rr];
                             const int cc = column(w);
                             if (cc < 0) continue;
-                            const int2 a = Av[(size_t)t * RMq + rr];
-                            rfma(rr ? acc1 : acc0, ((double)a.x * 536870912.0 + (double)a.y) * sc, xc[cc]);
+                            const double a = e == ASM_NAN ? __longlong_as_double(0x7FF8000000000000ll)
+                                                          : fx_value(Av[(size_t)t * RMq + rr], e);
+                            rfma(rr ? acc1 : acc0, a, xc[cc]);
                         }
                     }
                 }
@@ -2930,7 +2980,7 @@ struct gade_solver {
     double asm_bal_gain;        /* modelled time of the plain partition over the balanced one's */
     int npairs;                 /* (block row, coupled block) pairs */
     int *d_pair_c;
-    int2 *d_K, *d_A;            /* fixed-point limbs of K (per table set) and of A (per pulse), see AsmLay */
+    int2 *d_K, *d_A;            /* words of K (per table set) and of A (per pulse), see AsmLay */
     unsigned short *d_Ke, *d_Ae;   /* row exponents: [table set][pairs][3][Bp], [pulse][pairs][Bp] */
     int rdiag;                  /* S(k) is real and i h dt/2 h0(k) imaginary */
     int halves;                 /* the ELL slots are laid out by column half and spline offset */
@@ -4051,8 +4101,8 @@ static int asm_partitions(gade_solver *s)
 
 static size_t asm_smem_bytes(const gade_solver *s)
 {
-    unsigned a, b, c, d;
-    return asm_smem(asm_xs(s->RMA, s->CM, s->halves), s->W, s->RMA, s->halves, 256, &a, &b, &c, &d);
+    unsigned a, b, c, d, e;
+    return asm_smem(asm_xs(s->RMA, s->CM, s->halves), s->W, s->RMA, s->halves, 256, &a, &b, &c, &d, &e);
 }
 
 /* dynamic shared memory of k_apply_asm32 */
@@ -4205,8 +4255,8 @@ static int launch_assemble(gade_solver *s, cudaStream_t st)
 {
     prof_begin(s, st);
     A32Map F = {(float *)s->d_A32, s->RMp, s->a32_stride};
-    /* pulses that share K read it together, four to a group */
-    const int pt = s->asm_kstride == 0 && s->nslot > 1 ? 4 : 1;
+    /* pulses that share K read it together, two to a group */
+        const int pt = s->asm_kstride == 0 && s->nslot > 1 ? 2 : 1;
     const int ppb = 128 / (s->RMA / 2);                        /* pairs per CTA */
     const int gy = (s->npairs + ppb - 1) / ppb, gz = (s->nslot + pt - 1) / pt;
     /* all slots to a thread where the pairs alone give every SM its CTAs (the
@@ -4218,7 +4268,7 @@ static int launch_assemble(gade_solver *s, cudaStream_t st)
 #define AS(PT_) k_assemble<PT_><<<grid, 128, 0, st>>>(s->d_A, s->d_Ae, F, s->d_K, s->d_Ke, asm_lay(s), s->d_pair_par, \
         s->d_coef, make_int2(s->lpar[0], s->lpar[1]), s->d_plist, s->nslot, s->asm_kstride, \
         s->asm_kstride / s->W, s->lmax, nsl)
-    if (pt == 4) AS(4); else AS(1);
+    if (pt == 2) AS(2); else AS(1);
 #undef AS
     prof_end(s, st, 2);
     CKL();
