@@ -1730,7 +1730,7 @@ struct PcT {
     int pred;                      /* PRED_* */
     unsigned spin_limit;           /* polls of a stage wait before the kernel gives up */
     int withhold;                  /* failure injection: stage whose copy is not issued (-1: none) */
-    const int *ex, *scale;         /* fixed point: [pulse][nk][2][2][nch] exponents, [pulse][nk][Bp] row scales */
+    const int *bad;                /* k_precond_fx: [pulse][nk], factors not finite */
 };
 
 __device__ __forceinline__ unsigned smem_u32(const void *p)
@@ -2019,119 +2019,78 @@ __global__ void __launch_bounds__(NW * 32) k_precond_tma(PcT Q, int mode, const 
 }
 
 /* ------------------------------------------------------------------ */
-/* block-LU preconditioner in fixed point                               */
+/* block-LU preconditioner on the integer units                         */
 /* ------------------------------------------------------------------ */
 /*
  * The FP64 solves above need 129k DFMA per block row of 510 and were bound by
  * the FP64 pipe of the SM that holds the row (58 us at N = 53,040).  Here the
- * same sweeps run on the integer units (gade_fx.cuh).  D^T is scaled to a
- * unit diagonal first, E D^T E with E = diag(2^-s), s_i = round(log2 |D_ii| /
- * 2), so that the factors' entries and the vectors are of one size within a
- * chunk: L' = E L E^-1, U' = E U E, b' = E b, x' = L'^-1 b', y = E U'^-1 x'.
- * Factor entries are 57-bit integers with one exponent per chunk (triangle
- * and chain block apart), vector entries 57-bit integers with one exponent
- * per chunk; sums are exact 64-bit integers, rescaled once per chunk and
- * sweep step.  An entry's error is ~2^-57 of the chunk's largest, where the
- * FP64 sweeps round 33 products and sums to 2^-53 of theirs; measured against
- * 64-bit-mantissa solves, rms over block rows, both are the same to 1% (the
- * factors' own rounding): 4.0e-14 for a state, 2.3e-14 for random entries.
- * What bounds it at 16 chunks: the chains' 32 dependent steps (34,000 of some
- * 62,000 cycles), then the triangles' integer multiply-adds (21,000).  31.8 us
- * for 104 block rows of 510 (FP64: 58), 118 us for 832 (330).
+ * same sweeps run on the integer units (gade_fx.cuh): a factor entry is two
+ * words of 57 bits with the exponent of its larger part, a vector entry two
+ * 58-bit integers with the exponent of its larger part, and every sum of
+ * products (a lane's 8 or 9 of a triangle, 4 or 8 of a chain block) is aligned
+ * to its largest product.  Sums are 64-bit integers S 2^(E - 2100) until the
+ * result is stored: a row's error is a few 2^-54 of the sum of its terms, where
+ * the FP64 sweeps round every product and sum to 2^-53.  (With one exponent
+ * per 32 rows of a factor and of the vector, 31.8 us, rows were off by up to
+ * 30 x 2^-53 of their terms for vectors that fall by 24 orders of magnitude.)
+ * What bounds it at 16 chunks: the chains' 32 dependent steps, then the
+ * triangles' multiply-adds.  41.5 us for 104 block rows of 510 (FP64: 58), 171
+ * us for 832 (330), 21.7 us for 40 of 210 (30).
  * An infinity or NaN in a block row or its factors makes its whole result NaN.
  */
 #define PF_BW 16                       /* band padding it is written for (the B-spline bases' half-width is 15) */
 #define PF_PPS 2                       /* triangle pairs per stage */
 #define PF_GCH 4                       /* chain blocks per stage */
-#define PF_NAN 1000000                 /* exponent of a factor chunk that is not finite */
+#define PF_UP 3                        /* bits of a word below a 53-bit value */
+#define PF_EX 2100                     /* a sum is S 2^(E - PF_EX) */
+#define PF_LOW (-20000)                /* exponent of a zero entry of the vector */
 #define PF_STAGE (PF_PPS * PC_TP > PF_GCH * 32 * PF_BW ? PF_PPS * PC_TP : PF_GCH * 32 * PF_BW)
-/* dynamic shared memory: two stages, x (int64 re, im) and its limbs per row,
-   partial sums, exponents (triangles and chains of both sweeps, vector) */
-__host__ __device__ __forceinline__ size_t pf_smem(int Bp, int nch)
+/* dynamic shared memory: two stages, sums (int64 re, im) and limbs per row,
+   partial sums and their exponents, exponents of the rows' sums and limbs */
+__host__ __device__ __forceinline__ size_t pf_smem(int Bp)
 {
-    return (size_t)16 * (2 * PF_STAGE + 2 * Bp) + 8 * 1024 + 4 * (size_t)(7 * nch);
+    return (size_t)16 * (2 * PF_STAGE + 2 * Bp) + 8 * 1024 + 4 * (512 + 2 * (size_t)Bp);
 }
 
-/* v 2^-sh to nearest, sh >= 1, |v| < 2^62 */
-__device__ __forceinline__ long long fx_rshift(long long v, int sh) { return ((v >> (min(sh, 63) - 1)) + 1) >> 1; }
-/* N = X 2^-sh with |N| <= 2^57 for a group whose largest |X| has high word mh; returns sh */
-__device__ __forceinline__ int fx_norm_shift(unsigned mh) { return 7 - __clz((int)mh); }
-__device__ __forceinline__ long long fx_norm(long long X, int sh) { return sh > 0 ? fx_rshift(X, sh) : X << -sh; }
-__device__ __forceinline__ unsigned fx_abs_hi(long long X)
+/* the words of a factor entry: the exponent e of its larger part is split over
+   their lowest 7 bits, part = N 2^(e - 1078) */
+__device__ __forceinline__ int4 pf_pack(double2 v, bool &bad)
 {
-    const int h = (int)(X >> 32);
-    return (unsigned)(h ^ (h >> 31));
+    const unsigned h = max((unsigned)__double2hiint(v.x) & 0x7FFFFFFFu, (unsigned)__double2hiint(v.y) & 0x7FFFFFFFu);
+    int e = max(fx_exp(h), 1);
+    if (e == 2047) { bad = true; return make_int4(0, 0, 0, 0); }
+    if (v.x == 0.0 && v.y == 0.0) e = 0;
+    const int2 a = fx_word_of(e ? fx_from(v.x, e, PF_UP) << 7 : 0, e & FX_OFF);
+    const int2 b = fx_word_of(e ? fx_from(v.y, e, PF_UP) << 7 : 0, e >> 7);
+    return make_int4(a.x, a.y, b.x, b.y);
 }
+__device__ __forceinline__ int pf_exp(int4 d) { return (d.x & FX_OFF) | ((d.z & FX_OFF) << 7); }
 
-/* scales and converts the factors of one (pulse, kappa): grid (triangle pairs
-   then chunks, sweep, pulse x kappa), one warp */
+/* the factors of all pulses as words; bad[pulse x kappa]: not finite */
 __global__ void k_fix_factors(const double2 *__restrict__ FL, const double2 *__restrict__ FU, int4 *__restrict__ XL,
-                              int4 *__restrict__ XU, const int *__restrict__ scale, int *__restrict__ ex, int nch,
-                              int bwp, int Bp, size_t per)
+                              int4 *__restrict__ XU, int *__restrict__ bad, size_t per)
 {
-    const int npair = (nch + 1) / 2, lane = threadIdx.x, up = blockIdx.y, pk = blockIdx.z;
-    const double2 *F = (up ? FU : FL) + (size_t)pk * per;
-    int4 *X = (up ? XU : XL) + (size_t)pk * per;
-    const int *s = scale + (size_t)pk * Bp;
-    int *eT = ex + ((size_t)pk * 2 + up) * 2 * nch, *eG = eT + nch;
-    /* value of an entry (row r, column c) after scaling */
-    auto scaled = [&](double2 v, int r, int c) {
-        const int k = up ? s[r] + s[c] : s[c] - s[r];
-        return make_double2(scalbn(v.x, k), scalbn(v.y, k));
-    };
-    auto gscaled = [&](double2 v, int r, int c) {
-        const int k = up ? s[r] - s[c] : s[c] - s[r];
-        return make_double2(scalbn(v.x, k), scalbn(v.y, k));
-    };
-    /* value = N 2^(em - 1075 - FX_UPA); PF_NAN where a factor is not finite */
-    auto exponent = [](int em) { return em == 2047 ? PF_NAN : em - 1075 - FX_UPA; };
-    auto hi = [](double2 v) {
-        return max((unsigned)__double2hiint(v.x) & 0x7FFFFFFFu, (unsigned)__double2hiint(v.y) & 0x7FFFFFFFu);
-    };
-    auto put = [](double2 v, int em) {
-        const int2 a = fx_split(fx_from(v.x, em, FX_UPA)), b = fx_split(fx_from(v.y, em, FX_UPA));
-        return make_int4(a.x, a.y, b.x, b.y);
-    };
-    if (blockIdx.x < npair) {
-        const int p = blockIdx.x, c0 = 2 * p, c1 = 2 * p + 1;
-        const bool has1 = c1 < nch;
-        const int sw = up ? 31 - lane : lane;
-        unsigned m0 = 0, m1 = 0;
-        for (int pass = 0; pass < 2; pass++) {
-            const int e0 = max(fx_exp(__reduce_max_sync(0xffffffffu, m0)), 1),
-                      e1 = max(fx_exp(__reduce_max_sync(0xffffffffu, m1)), 1);
-            for (int q = 0; q < 33; q++) {
-                const size_t o = (size_t)p * PC_TP + q * 32 + lane;
-                const bool first = q <= sw;
-                if (!first && !has1) { if (pass) X[o] = make_int4(0, 0, 0, 0); continue; }
-                const int r = first ? 32 * c0 + lane : 32 * c1 + 31 - lane;
-                const int c = up ? (first ? 32 * c0 + lane + q : 32 * c1 + q - 1)
-                                 : (first ? 32 * c0 + q : 32 * c1 + q - lane - 1);
-                const double2 v = scaled(F[o], r, c);
-                if (!pass) { if (first) m0 = max(m0, hi(v)); else m1 = max(m1, hi(v)); }
-                else X[o] = put(v, first ? e0 : e1);
-            }
-            if (pass && lane == 0) {
-                eT[c0] = exponent(e0);
-                if (has1) eT[c1] = exponent(e1);
-            }
-        }
-    } else {
-        const int c = blockIdx.x - npair;
-        const size_t o0 = (size_t)npair * PC_TP + (size_t)c * 32 * bwp;
-        unsigned m = 0;
-        for (int pass = 0; pass < 2; pass++) {
-            const int em = max(fx_exp(__reduce_max_sync(0xffffffffu, m)), 1);
-            for (int col = 0; col < bwp; col++) {
-                const int r = 32 * c + lane, cc = up ? 32 * (c + 1) + col : 32 * c - bwp + col;
-                double2 v = make_double2(0.0, 0.0);
-                if (cc >= 0 && cc < Bp) v = gscaled(F[o0 + col * 32 + lane], r, cc);
-                if (!pass) m = max(m, hi(v));
-                else X[o0 + col * 32 + lane] = put(v, em);
-            }
-            if (pass && lane == 0) eG[c] = exponent(em);
-        }
-    }
+    const size_t o = (size_t)blockIdx.y * per, e = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (e >= per) return;
+    bool b = false;
+    XL[o + e] = pf_pack(FL[o + e], b);
+    XU[o + e] = pf_pack(FU[o + e], b);
+    if (b) atomicOr(&bad[blockIdx.y], 1);
+}
+
+/* the complex value (re, im) S 2^(E - PF_EX) as limbs of a vector entry with the
+   exponent c of its larger part; bits: 64 less the leading zeros of the larger |S| */
+__device__ __forceinline__ int pf_bits(long long S) { return 64 - __clzll(S ^ (S >> 63)); }
+__device__ __forceinline__ long long pf_norm(long long S, int bits)
+{
+    const int sh = 58 - bits;
+    return sh >= 0 ? S << sh : (fx_shr(S, -sh - 1) + 1) >> 1;
+}
+__device__ __forceinline__ int pf_cexp(int E, int bits) { return bits ? E - (PF_EX - 1080) - (58 - bits) : PF_LOW; }
+/* h 2^60 + m 2^30 in units of 2^59, to nearest */
+__device__ __forceinline__ long long pf_sum(long long h, long long m)
+{
+    return 2 * h + ((m + (1ll << (FX_WB - 2))) >> (FX_WB - 1));
 }
 
 /*
@@ -2139,11 +2098,12 @@ __global__ void k_fix_factors(const double2 *__restrict__ FL, const double2 *__r
  * triangles, L chain, U triangles, U chain) with two triangle pairs or four
  * chain blocks each, so that two CTAs fit an SM.
  * Triangle stage: a pair's 33 products per lane are split over four warps,
- * whose sums (rows of chunk c0 and of chunk c1 apart) meet in shared memory.
+ * whose sums (rows of chunk c0 and of chunk c1 apart, each with its own
+ * alignment) meet in shared memory.
  * Chain: the next step needs only 16 of a chunk's rows, so four warps walk the
  * chain on those alone (lane = row and component, four of the 16 columns per
- * warp) and leave each chunk's normalised limbs in shared memory; another warp
- * forms the chunk's other 16 rows from them as soon as they are there.
+ * warp) and leave each chunk's limbs in shared memory; another warp forms the
+ * chunk's other 16 rows from them as soon as they are there.
  */
 __global__ void __launch_bounds__(256, 2) k_precond_fx(PcT Q, int mode, const double2 *__restrict__ in0,
                                                        const double2 *__restrict__ in1, double2 *io,
@@ -2152,12 +2112,12 @@ __global__ void __launch_bounds__(256, 2) k_precond_fx(PcT Q, int mode, const do
     constexpr int BWP = PF_BW, GC = 32 * BWP, GCH = PF_GCH, SB = PF_STAGE;
     extern __shared__ __align__(128) unsigned char smem_tma[];
     int4 *stg = (int4 *)smem_tma;                          /* [2][SB] */
-    longlong2 *tx = (longlong2 *)(stg + 2 * SB);           /* [Bp] x as integers (re, im) */
+    longlong2 *tx = (longlong2 *)(stg + 2 * SB);           /* [Bp] sums (re, im) */
     int4 *xq = (int4 *)(tx + Q.Bp);                        /* [Bp] limbs */
     long long *pt = (long long *)(xq + Q.Bp);              /* [2][4][4][32] partial sums of a triangle stage */
-    int *sexp = (int *)(pt + 1024);
+    int *pe = (int *)(pt + 1024);                          /* [2][4][2][32] their exponents (chain: [2][4][32]) */
+    int *tE = pe + 512, *xe = tE + Q.Bp;                   /* [Bp] exponents of the sums and of the limbs */
     const int nch = Q.nch;
-    int *sE = sexp + 4 * nch, *sEt = sE + nch, *sX = sEt + nch;   /* [4 nch] factors; x, triangle result, limbs */
     __shared__ __align__(8) uint64_t bar[2];
     __shared__ int all_ok, bad, s_prog;                    /* s_prog: chunks the chain has passed in this sweep */
     __shared__ double2 s_c[2];                             /* beta, -w (PC_P) or -alpha (PC_S) */
@@ -2186,7 +2146,6 @@ __global__ void __launch_bounds__(256, 2) k_precond_fx(PcT Q, int mode, const do
     const size_t per = pc_sweep_elems(nch, BWP);
     const size_t pk = (size_t)pulse * Q.fstride / per + kk;    /* (pulse, kappa) */
     const int4 *FL = (const int4 *)Q.FL + pk * per, *FU = (const int4 *)Q.FU + pk * per;
-    const int *scale = Q.scale + pk * Bp;
     auto stage = [&](int k, const int4 **src, int *cnt) {
         const int4 *F = k < nps ? FL : FU;
         const int j = k < nps ? k : k - nps;
@@ -2209,20 +2168,18 @@ __global__ void __launch_bounds__(256, 2) k_precond_fx(PcT Q, int mode, const do
         const unsigned bytes = stage(0, &src, &cnt);
         if (Q.withhold != 0) tma_bulk_load(stg, src, bytes, &bar[0]);
         all_ok = 1;
-        bad = 0;
+        bad = Q.bad[pk];
         s_prog = 0;
     }
     /* the vectors' entries are fetched while one thread forms the scalars (the
        divisions of eight warps took 11,000 of the kernel's 90,000 cycles) */
     constexpr int NL = 3;
     double2 f0[NL], f1[NL], f2[NL];
-    int fs[NL], fg[NL];
+    int fg[NL];
     auto fetch = [&](int n, int o) {
-        fs[n] = 0;
         f0[n] = f1[n] = f2[n] = make_double2(0, 0);
         if (o >= B) return;
         fg[n] = Q.ord[o];
-        fs[n] = scale[o];
         const size_t gi = off + fg[n];
         f0[n] = in0[gi];
         if (mode != PC_PLAIN) f1[n] = in1[gi];
@@ -2238,14 +2195,11 @@ __global__ void __launch_bounds__(256, 2) k_precond_fx(PcT Q, int mode, const do
             s_c[1] = make_double2(-sc->alpha.x, -sc->alpha.y);
         }
     }
-    for (int e = tid; e < 4 * nch; e += 256) sexp[e] = Q.ex[pk * 4 * nch + e];
     __syncthreads();
     {
         const double2 beta = s_c[0], negw = s_c[1], nega = s_c[1];
-        /* a warp's 32 entries are one chunk */
         auto enter = [&](int n, int o) {
             double2 val = f0[n];
-            const int so = fs[n];
             if (o < B && mode != PC_PLAIN) {
                 if (mode == PC_P) {
                     double2 t = f2[n];
@@ -2256,37 +2210,18 @@ __global__ void __launch_bounds__(256, 2) k_precond_fx(PcT Q, int mode, const do
                 }
                 io[off + fg[n]] = val;
             }
-            /* the largest |b'|'s exponent: the entries' less the row scales */
-            const unsigned h = max((unsigned)__double2hiint(val.x) & 0x7FFFFFFFu, (unsigned)__double2hiint(val.y) & 0x7FFFFFFFu);
-            const int e = fx_exp(h), es = e ? e - so : -5000;
-            const int em = __reduce_max_sync(0xffffffffu, es);
+            const int e = max(fx_exp(max((unsigned)__double2hiint(val.x) & 0x7FFFFFFFu, (unsigned)__double2hiint(val.y) & 0x7FFFFFFFu)), 1);
             if (e == 2047) bad = 1;
-            /* N = b' 2^-(em - 1079): the mantissa with 4 bits more, down by em - (e - so) */
-            long long N[2];
-#pragma unroll
-            for (int c = 0; c < 2; c++) {
-                const unsigned long long b = (unsigned long long)__double_as_longlong(c ? val.y : val.x);
-                const int ev = (int)((b >> 52) & 0x7FF);
-                unsigned long long m = ev ? (b & 0xFFFFFFFFFFFFFull) | 1ull << 52 : 0ull;
-                m = fx_shift(m << 4, ev ? min(64, em - (ev - so)) : 0);
-                N[c] = (long long)b < 0 ? -(long long)m : (long long)m;
-            }
-            const int2 re = fx_split(N[0]), im = fx_split(N[1]);
+            const int2 re = fx_limbs(fx_from(val.x, e, FX_UPX)), im = fx_limbs(fx_from(val.y, e, FX_UPX));
             xq[o] = make_int4(re.x, re.y, im.x, im.y);
-            /* a chunk of zeros: an exponent below all others, so that it moves no sum */
-            if (lane == 0) sX[o >> 5] = em - 1079;
+            xe[o] = (val.x == 0.0 && val.y == 0.0) ? PF_LOW : e;
         };
 #pragma unroll
         for (int n = 0; n < NL; n++)
             if (tid + 256 * n < Bp) enter(n, tid + 256 * n);
         for (int o = tid + 256 * NL; o < Bp; o += 256) { fetch(0, o); enter(0, o); }
     }
-    __syncthreads();
-    for (int c = tid; c < nch; c += 256) sEt[c] = sexp[c] + sX[c] + 2 * FX_LB;
-    for (int e = tid; e < 4 * nch; e += 256)
-        if (sexp[e] == PF_NAN) bad = 1;
 
-    const long long rnd = 1ll << (FX_LB - 1);
     int k = 0;
     for (; k < ns; k++) {
         if (tid == 0 && k + 1 < ns && k + 1 != Q.withhold) {
@@ -2307,13 +2242,13 @@ __global__ void __launch_bounds__(256, 2) k_precond_fx(PcT Q, int mode, const do
         const int up = k >= nps;                   /* U sweep */
         const int j = up ? k - nps : k;
         if (k == nps) {
-            /* x of the L sweep as limbs, normalised per chunk (a warp per chunk) */
-            for (int c = wid; c < nch; c += 8) {
-                const longlong2 X = tx[32 * c + lane];
-                const int sh = fx_norm_shift(__reduce_max_sync(0xffffffffu, max(fx_abs_hi(X.x), fx_abs_hi(X.y))));
-                const int2 re = fx_split(fx_norm(X.x, sh)), im = fx_split(fx_norm(X.y, sh));
-                xq[32 * c + lane] = make_int4(re.x, re.y, im.x, im.y);
-                if (lane == 0) sEt[c] = sexp[2 * nch + c] + sE[c] + sh + 2 * FX_LB;
+            /* x of the L sweep as limbs */
+            for (int o = tid; o < Bp; o += 256) {
+                const longlong2 X = tx[o];
+                const int b = max(pf_bits(X.x), pf_bits(X.y));
+                const int2 re = fx_limbs(pf_norm(X.x, b)), im = fx_limbs(pf_norm(X.y, b));
+                xq[o] = make_int4(re.x, re.y, im.x, im.y);
+                xe[o] = X.x == 0 && X.y == 0 ? PF_LOW : pf_cexp(tE[o], b);
             }
             __syncthreads();
         }
@@ -2330,46 +2265,68 @@ __global__ void __launch_bounds__(256, 2) k_precond_fx(PcT Q, int mode, const do
                 const int4 *T = S + pr * PC_TP + lane;
                 /* entry of x: q + b0 up to the switch, q + b1 after it (no chunk c1: any entry, T is zero) */
                 const int b0 = up ? 32 * c0 + lane : 32 * c0, b1 = !has1 ? -1 : (up ? 32 * c1 - 1 : 32 * c1 - lane - 1);
+                int4 d[9];
+                int key[9];
+                int C0 = 2 * PF_LOW, C1 = C0;          /* the rows' largest products */
+#pragma unroll
+                for (int n = 0; n < 9; n++) {
+                    /* only the first part has a ninth product (the others' is left out below) */
+                    const int q = n == 8 ? min(Q0 + 8, 32) : Q0 + n;
+                    d[n] = T[q * 32];
+                    key[n] = n == 8 && part > 0 ? 2 * PF_LOW : pf_exp(d[n]) + xe[q + (q <= sw ? b0 : b1)];
+                    C0 = q <= sw ? max(C0, key[n]) : C0;
+                    C1 = q <= sw ? C1 : max(C1, key[n]);
+                }
                 long long hr = 0, mr = 0, hi = 0, mi = 0, hr0 = 0, mr0 = 0, hi0 = 0, mi0 = 0;
 #pragma unroll
                 for (int n = 0; n < 9; n++) {
-                    /* only the first part has a ninth product (the others' is made zero) */
                     const int q = n == 8 ? min(Q0 + 8, 32) : Q0 + n;
-                    int4 d = T[q * 32];
-                    const int4 b = xq[q + (q <= sw ? b0 : b1)];
-                    if (n == 8 && part > 0) d = make_int4(0, 0, 0, 0);
+                    int4 b = xq[q + (q <= sw ? b0 : b1)];
+                    if (n == 8 && part > 0) b = make_int4(0, 0, 0, 0);
+                    const int s = (q <= sw ? C0 : C1) - key[n];
+                    int ah, al, gh, gl;
+                    fx_take(d[n].x, d[n].y, s, ah, al);
+                    fx_take(d[n].z, d[n].w, s, gh, gl);
                     const int nz = -b.z, nw = -b.w;
-                    hr += (long long)d.x * b.x;
-                    hr += (long long)d.z * nz;
-                    mr += (long long)d.x * b.y;
-                    mr += (long long)d.y * b.x;
-                    mr += (long long)d.z * nw;
-                    mr += (long long)d.w * nz;
-                    hi += (long long)d.x * b.z;
-                    hi += (long long)d.z * b.x;
-                    mi += (long long)d.x * b.w;
-                    mi += (long long)d.y * b.z;
-                    mi += (long long)d.z * b.y;
-                    mi += (long long)d.w * b.x;
+                    fx_mad(hr, ah, b.x);
+                    fx_mad(hr, gh, nz);
+                    fx_mad(mr, ah, b.y);
+                    fx_mad(mr, al, b.x);
+                    fx_mad(mr, gh, nw);
+                    fx_mad(mr, gl, nz);
+                    fx_mad(hi, ah, b.z);
+                    fx_mad(hi, gh, b.x);
+                    fx_mad(mi, ah, b.w);
+                    fx_mad(mi, al, b.z);
+                    fx_mad(mi, gh, b.y);
+                    fx_mad(mi, gl, b.x);
                     /* the products up to sw belong to the row of c0 */
                     const bool last = q == sw && (n < 8 || part == 0);
                     hr0 = last ? hr : hr0; mr0 = last ? mr : mr0;
                     hi0 = last ? hi : hi0; mi0 = last ? mi : mi0;
                 }
                 if (sw >= Q1) { hr0 = hr; mr0 = mr; hi0 = hi; mi0 = mi; }
-                long long *d = pt + (size_t)wid * 4 * 32 + lane;
-                d[0] = hr0 + ((mr0 + rnd) >> FX_LB);
-                d[32] = hi0 + ((mi0 + rnd) >> FX_LB);
-                d[64] = (hr - hr0) + ((mr - mr0 + rnd) >> FX_LB);
-                d[96] = (hi - hi0) + ((mi - mi0 + rnd) >> FX_LB);
+                long long *ds = pt + (size_t)wid * 4 * 32 + lane;
+                ds[0] = pf_sum(hr0, mr0);
+                ds[32] = pf_sum(hi0, mi0);
+                ds[64] = pf_sum(hr - hr0, mr - mr0);
+                ds[96] = pf_sum(hi - hi0, mi - mi0);
+                pe[wid * 64 + lane] = C0;
+                pe[wid * 64 + 32 + lane] = C1;
             }
             __syncthreads();
             if (act) {
                 /* warp (pair, component): re, im of the row lane of c0, then of the row 31 - lane of c1 */
-                const long long *d = pt + ((size_t)pr * 16 + part) * 32 + lane;
-                const long long v = d[0] + d[4 * 32] + d[8 * 32] + d[12 * 32];
+                const long long *ds = pt + ((size_t)pr * 16 + part) * 32 + lane;
+                const int *de = pe + pr * 256 + (part >> 1) * 32 + lane;
+                const int e0 = de[0], e1 = de[64], e2 = de[128], e3 = de[192], E = max(max(e0, e1), max(e2, e3));
+                const long long v = fx_shr(ds[0], E - e0) + fx_shr(ds[4 * 32], E - e1) + fx_shr(ds[8 * 32], E - e2) +
+                                    fx_shr(ds[12 * 32], E - e3);
                 const int row = part < 2 ? 32 * c0 + lane : 32 * c1 + 31 - lane;
-                if (part < 2 || has1) ((long long *)tx)[2 * row + (part & 1)] = v;
+                if (part < 2 || has1) {
+                    ((long long *)tx)[2 * row + (part & 1)] = v;
+                    if ((part & 1) == 0) tE[row] = E;
+                }
             }
             __syncthreads();
         } else {
@@ -2384,54 +2341,80 @@ __global__ void __launch_bounds__(256, 2) k_precond_fx(PcT Q, int mode, const do
                 la[comp] = comp ? make_int2(-l.x, -l.y) : l;
                 lb[comp ^ 1] = l;
             };
-            auto products = [&](const int4 *G, const int4 *xl, int n) {
+            /* the sum of the products of n columns' words and the entries xl (exponents
+               ex), aligned to the largest, 2^C */
+            auto products = [&](const int4 *d, const int4 *xl, const int *ex, auto n_, int &C) {
+                constexpr int n = decltype(n_)::value;
+                int key[n];
+                C = 2 * PF_LOW;
+#pragma unroll
+                for (int q = 0; q < n; q++) {
+                    key[q] = pf_exp(d[q]) + ex[q];
+                    C = max(C, key[q]);
+                }
                 long long h = 0, h2 = 0, m = 0, m2 = 0;
 #pragma unroll
                 for (int q = 0; q < n; q++) {
-                    const int4 d = G[q * 32], b = xl[q];
-                    h += (long long)d.x * b.x;
-                    m += (long long)d.x * b.y;
-                    m2 += (long long)d.y * b.x;
-                    h2 += (long long)d.z * b.z;
-                    m += (long long)d.z * b.w;
-                    m2 += (long long)d.w * b.z;
+                    const int4 b = xl[q];
+                    int ah, al, gh, gl;
+                    fx_take(d[q].x, d[q].y, C - key[q], ah, al);
+                    fx_take(d[q].z, d[q].w, C - key[q], gh, gl);
+                    fx_mad(h, ah, b.x);
+                    fx_mad(m, ah, b.y);
+                    fx_mad(m2, al, b.x);
+                    fx_mad(h2, gh, b.z);
+                    fx_mad(m, gh, b.w);
+                    fx_mad(m2, gl, b.z);
                 }
-                return h + h2 + ((m + m2 + rnd) >> FX_LB);
-            };
-            /* aligned sum of the triangle result t and the chain part v of chunk c */
-            auto join = [&](long long t, long long v, int c, int cp, int &E) {
-                const int Et = sEt[c], Eg = sexp[(2 * up + 1) * nch + c] + sX[cp] + 2 * FX_LB;
-                E = max(Et, Eg) + 1;
-                return fx_rshift(t, E - Et) + fx_rshift(v, E - Eg);
+                return pf_sum(h + h2, m + m2);
             };
             if (wid < 4) {
                 /* four columns per warp; the four sums of a row meet in shared memory
                    (two buffers, one barrier of these warps per step) and every warp
                    carries the whole x on, so that nothing is handed back */
+                int4 d[4];
+                auto load = [&](int e) {                     /* the columns of step e, a step ahead of their use */
+                    const int4 *G = S + (up ? cnt - 1 - e : e) * GC + (up ? row16 : 16 + row16) + 4 * wid * 32;
+#pragma unroll
+                    for (int q = 0; q < 4; q++) d[q] = G[q * 32];
+                };
+                load(0);
                 for (int e = 0; e < cnt; e++) {
                     const int ci = up ? cnt - 1 - e : e;     /* U: last chunk first */
                     const int c = g * GCH + ci, cp = up ? c + 1 : c - 1;
                     const int rr = up ? row16 : 16 + row16;
                     long long *tp = (long long *)tx + 2 * (32 * c + rr) + comp;
-                    const long long t = *tp;
-                    long long X = t;
-                    int E = sEt[c];
+                    long long X = *tp;
+                    int E = tE[32 * c + rr];
                     if (cp >= 0 && cp < nch) {               /* the first chunk has no neighbour: the triangle result stands */
-                        long long *ps = pt + (c & 1) * 128;
-                        ps[wid * 32 + lane] = products(S + ci * GC + rr + 4 * wid * 32, xq + 32 * cp + 16 * comp + 4 * wid, 4);
+                        long long *ps = pt + (c & 1) * 128 + lane;
+                        int *pq = pe + (c & 1) * 128 + lane, C;
+                        ps[wid * 32] = products(d, xq + 32 * cp + 16 * comp + 4 * wid, xe + 32 * cp + 4 * wid,
+                                                std::integral_constant<int, 4>(), C);
+                        pq[wid * 32] = C;
+                        if (e + 1 < cnt) load(e + 1);
                         asm volatile("bar.sync 1, 128;" ::: "memory");
-                        X = join(t, (ps[lane] + ps[32 + lane]) + (ps[64 + lane] + ps[96 + lane]), c, cp, E);
+                        const int e0 = pq[0], e1 = pq[32], e2 = pq[64], e3 = pq[96];
+                        const int Ev = max(max(e0, e1), max(e2, e3)), En = max(E, Ev);
+                        X = fx_shr(X, En - E) + fx_shr(ps[0], En - e0) + fx_shr(ps[32], En - e1) + fx_shr(ps[64], En - e2) +
+                            fx_shr(ps[96], En - e3);
+                        E = En;
+                    } else if (e + 1 < cnt) {
+                        load(e + 1);
                     }
-                    const int sh = fx_norm_shift(__reduce_max_sync(0xffffffffu, fx_abs_hi(X)));
-                    const int2 l = fx_split(fx_norm(X, sh));
+                    int b = pf_bits(X);
+                    b = max(b, __shfl_xor_sync(0xffffffffu, b, 1));
+                    const int2 l = fx_limbs(pf_norm(X, b));
                     /* every warp writes the same values: the next step reads what its own warp wrote */
                     put_limbs(xq + 32 * c, l);
-                    if (lane == 0) sX[c] = E + sh;
+                    const bool zero = __shfl_xor_sync(0xffffffffu, X == 0, 1) && X == 0;
+                    if (comp == 0) xe[32 * c + row16] = zero ? PF_LOW : pf_cexp(E, b);
                     __syncwarp();
                     if (wid == 0) {
                         *tp = X;
-                        if (lane == 0) sE[c] = E;
+                        if (comp == 0) tE[32 * c + rr] = E;
                         __threadfence_block();
+                        __syncwarp();
                         if (lane == 0) *(volatile int *)&s_prog = (up ? nch - 1 - c : c) + 1;
                     }
                 }
@@ -2439,15 +2422,29 @@ __global__ void __launch_bounds__(256, 2) k_precond_fx(PcT Q, int mode, const do
                 const int ci = wid - 4, c = g * GCH + ci, cp = up ? c + 1 : c - 1;
                 const int need = up ? nch - 1 - c : c;       /* chunks passed when cp's limbs are there */
                 if (need > 0) {
+                    const int rr = up ? 16 + row16 : row16;
+                    int4 d[16];
+#pragma unroll
+                    for (int q = 0; q < 16; q++) d[q] = S[ci * GC + rr + q * 32];
                     unsigned spins = 0;
                     while (*(volatile int *)&s_prog < need && ++spins < MBAR_SPIN_LIMIT) {
                     }
                     if (spins >= MBAR_SPIN_LIMIT) all_ok = 0;
                     __threadfence_block();
-                    const int rr = up ? 16 + row16 : row16;
                     long long *tp = (long long *)tx + 2 * (32 * c + rr) + comp;
-                    int E;
-                    *tp = join(*tp, products(S + ci * GC + rr, xq + 32 * cp + 16 * comp, BWP), c, cp, E);
+                    long long X = *tp;
+                    int E = tE[32 * c + rr];
+                    __syncwarp();
+#pragma unroll
+                    for (int hf = 0; hf < 2; hf++) {
+                        int C;
+                        const long long v = products(d + 8 * hf, xq + 32 * cp + 16 * comp + 8 * hf, xe + 32 * cp + 8 * hf,
+                                                     std::integral_constant<int, 8>(), C);
+                        fx_join(X, E, v, C);
+                        E = max(E, C);
+                    }
+                    *tp = X;
+                    if (comp == 0) tE[32 * c + rr] = E;
                 }
             }
             __syncthreads();
@@ -2472,7 +2469,7 @@ __global__ void __launch_bounds__(256, 2) k_precond_fx(PcT Q, int mode, const do
     const bool nan = bad != 0;
     for (int o = tid; o < B; o += 256) {
         const longlong2 X = tx[o];
-        const int e = sE[o >> 5] - scale[o];
+        const int e = tE[o] - PF_EX;
         double2 y = make_double2(fx_add(0.0, X.x, e), fx_add(0.0, X.y, e));
         if (nan) y.x = y.y = __longlong_as_double(0x7FF8000000000000ll);
         out[off + Q.ord[o]] = y;
@@ -2922,8 +2919,8 @@ struct gade_solver {
     int *d_ord;
     double2 *d_FL, *d_FU;       /* chunk-packed factors for the TMA kernel */
     int bwp;
-    int4 *d_XL, *d_XU;          /* the factors in fixed point (NULL: not used) */
-    int *d_pex, *d_pscale;      /* their exponents and the row scales (PcT) */
+    int4 *d_XL, *d_XU;          /* the factors as words for k_precond_fx (NULL: not used) */
+    int *d_pbad;                /* [pulse][nk] factors not finite */
     /* vectors */
     double2 *x, *rhs, *r, *r0, *p, *v, *y, *z, *s, *t, *tmp0, *tmp1;
     /* reductions */
@@ -3012,7 +3009,7 @@ struct gade_solver {
     void *d_ang_dd[4], *d_Sdd, *d_Hdd, *d_Mdd;
     cdd *xdd, *ddd, *wdd;
     int pc_withhold;            /* failure injection: preconditioner stage whose copy is withheld (-1: none) */
-    int pc_nw;                  /* warps per block row of the complex128 preconditioner solves (4: FP64; 8: fixed point, or FP64 without d_XL) */
+    int pc_nw;                  /* warps per block row of the complex128 preconditioner solves (4: FP64; 8: integer units, or FP64 without d_XL) */
 };
 
 /* dynamic shared memory of k_precond_tma: two stage buffers, the block
@@ -3556,15 +3553,14 @@ static int solver_create(const gade_problem *p, int npulse, const double *dts, c
            both bases' own ordering) and must fit an SM (Bp <= 4,500); wider
            bands and larger blocks keep the FP64 kernel, and so do batches whose
            second copy of the factors would take a tenth of the free memory */
-        const size_t smx = pf_smem(s->Bp, s->nch);
+        const size_t smx = pf_smem(s->Bp);
         size_t fr = 0, tot = 0;
         if (cudaMemGetInfo(&fr, &tot) != cudaSuccess) fr = 0;
         if (s->bwp == PF_BW && smx <= 220 * 1024 && 2 * sizeof(int4) * NP * s->fstride < fr / 10) {
             cudaFuncSetAttribute(k_precond_fx, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smx);
             UP(s->d_XL, (const int4 *)nullptr, NP * s->fstride);
             UP(s->d_XU, (const int4 *)nullptr, NP * s->fstride);
-            UP(s->d_pex, (const int *)nullptr, NP * s->nk * 4 * s->nch);
-            UP(s->d_pscale, (const int *)nullptr, NP * s->nk * s->Bp);
+            UP(s->d_pbad, (const int *)nullptr, NP * s->nk);
         }
         cudaFuncSetAttribute(k_precond_tma<float, 16, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm32);
         cudaFuncSetAttribute(k_precond_tma<float, 32, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm32);
@@ -3622,23 +3618,10 @@ static int solver_create(const gade_problem *p, int npulse, const double *dts, c
                 if (ce == cudaSuccess) ce = cudaMemcpy((float2 *)s->d_FU32 + k * s->fstride, FUf.data(), sizeof(float2) * s->fstride, cudaMemcpyHostToDevice);
             }
             if (ce == cudaSuccess && s->d_XL) {
-                /* row scales: half the binary exponent of the diagonal, in the factors' ordering */
-                std::vector<int> sc((size_t)s->nk * s->Bp, 0);
-                for (int kk = 0; kk < s->nk; kk++)
-                    for (int o = 0; o < s->B; o++) {
-                        const int i = su->ord[o];
-                        for (int t = 0; t < s->W; t++)
-                            if (su->ell_col[(size_t)t * s->B + i] == i) {
-                                const double2 d = D[((size_t)kk * s->W + t) * s->B + i];
-                                const double m = hypot(d.x, d.y);
-                                if (m > 0 && std::isfinite(m)) sc[(size_t)kk * s->Bp + o] = (int)lrint(0.5 * log2(m));
-                            }
-                    }
-                ce = cudaMemcpy(s->d_pscale + (size_t)k * s->nk * s->Bp, sc.data(), sizeof(int) * sc.size(), cudaMemcpyHostToDevice);
-                k_fix_factors<<<dim3((s->nch + 1) / 2 + s->nch, 2, s->nk), 32>>>(
+                const size_t per = pc_sweep_elems(s->nch, s->bwp);
+                k_fix_factors<<<dim3((unsigned)((per + 255) / 256), s->nk), 256>>>(
                     s->d_FL + k * s->fstride, s->d_FU + k * s->fstride, s->d_XL + k * s->fstride, s->d_XU + k * s->fstride,
-                    s->d_pscale + (size_t)k * s->nk * s->Bp, s->d_pex + (size_t)k * s->nk * 4 * s->nch, s->nch, s->bwp, s->Bp,
-                    pc_sweep_elems(s->nch, s->bwp));
+                    s->d_pbad + (size_t)k * s->nk, per);
                 if (ce == cudaSuccess) ce = cudaGetLastError();
                 if (ce == cudaSuccess) ce = cudaDeviceSynchronize();
             }
@@ -4352,21 +4335,21 @@ static PcT pc_params(const gade_solver *s, const void *FL, const void *FU, int p
     Q.plist = s->d_plist; Q.vstride = s->n; Q.fstride = s->fstride; Q.pred = pred;
     Q.spin_limit = s->pc_wait ? s->pc_wait : MBAR_SPIN_LIMIT;
     Q.withhold = s->pc_withhold;
-    Q.ex = s->d_pex; Q.scale = s->d_pscale;
+    Q.bad = s->d_pbad;
     return Q;
 }
 
 static int launch_precond(gade_solver *s, int mode, const double2 *in0, const double2 *in1, double2 *io,
                           double2 *out, cudaStream_t st, int pred = PRED_NONE)
 {
-    /* 8 warps: fixed point where the factors have that form (see solver_create):
-       31.8 us a solve at N = 53,040 and 118 us for 8 pulses, where
-       k_precond_tma's 8 FP64 warps take 58 and 330 */
+    /* 8 warps: on the integer units where the factors have that form (see
+       solver_create): 41.5 us a solve at N = 53,040 and 171 us for 8 pulses,
+       where k_precond_tma's 8 FP64 warps take 58 and 330 */
     if (s->pc_nw == 8 && s->d_XL) {
         PcT Q = pc_params(s, s->d_XL, s->d_XU, pred);
         const dim3 grid(s->nslot, s->nblk);
         prof_begin(s, st);
-        launch_pdl(k_precond_fx, grid, dim3(256), pf_smem(s->Bp, s->nch), st, Q, mode, in0, in1, io, out, s->d_sc);
+        launch_pdl(k_precond_fx, grid, dim3(256), pf_smem(s->Bp), st, Q, mode, in0, in1, io, out, s->d_sc);
         prof_end(s, st, 1);
         CKL();
         return GADE_OK;

@@ -208,9 +208,13 @@ int gade_solver_operator(const gade_solver *s, int32_t *assembled, float *ms);
 
 /* Flops (2 per multiply-add) of one operator apply and one preconditioner
  * solve, counted exactly from the set-up structure.  The assembled operator
- * and the preconditioner form theirs (but the diagonal blocks') as
- * fixed-point products on the integer units (at least 56 x 57 bits, error no
- * larger than FP64's). */
+ * and the preconditioner form theirs (but the diagonal blocks') on the integer
+ * units: every value has an exponent of its own (57 x 58 bits) and every sum
+ * of products is aligned to its largest, so that a row's error is, as with
+ * FP64 products, a few 2^-53 of the sum of its terms' magnitudes.  Magnitudes
+ * are those of complex numbers: the two parts of a vector entry or of a factor
+ * share an exponent.  A coupling value below 2^-127 of the largest of its row
+ * of a block loses bits. */
 int gade_solver_flops(const gade_solver *s, double *apply_flops, double *precond_flops);
 /* Compulsory DRAM bytes of one FP64 BiCGSTAB operator apply (no reference
  * counterpart).  Matrix-free: the radial-table slabs of the distinct (order,
@@ -273,10 +277,10 @@ int gade_solver_residual_precision(const gade_solver *s, int32_t *mode, int32_t 
 int gade_solver_set_wait_limit(gade_solver *s, uint32_t polls);
 /* Warps per block row of the complex128 block-LU solves (replacing the
  * cuSPARSE triangular solves of tools/gpu_sparse.c:235-263): 8 (the
- * default: products in fixed point on the integer units, 57 x 57 bits with
- * exact sums, where the blocks' half-bandwidth is at most 16; FP64 with the
- * triangle products of a chunk pair split over two warps otherwise) or 4
- * (FP64).  The results differ by rounding.
+ * default: products on the integer units where the blocks' half-bandwidth is
+ * at most 16, see gade_solver_flops; FP64 with the triangle products of a
+ * chunk pair split over two warps otherwise) or 4 (FP64).  The results differ
+ * by rounding.
  * The complex64 solves of the mixed-precision inner iterations always use
  * 4.  Takes effect at the next step. */
 int gade_solver_set_precond_warps(gade_solver *s, int32_t warps);

@@ -63,3 +63,73 @@ def test_operator_rows(tmp_path, native_lib, ns):
             for y, M, A in zip(s.apply(x, parts=True)[1:], (S, H), (Sa, Ha)):
                 err, mag = np.abs(y - M @ x), A @ np.abs(x)
                 assert (err <= 1e-14 * mag).all(), (name, op, float((err / mag).max()))
+
+
+def _factors(A):
+    """Block-LU sweeps' factors of A (in the factors' order): inverse triangles
+    and the 16 chain columns of each 32-row chunk."""
+    B = len(A)
+    nch = (B + 31) // 32
+    L, U = np.eye(32 * nch, dtype=complex), np.eye(32 * nch, dtype=complex)
+    U[:B, :B] = A
+    for k in range(B):
+        e = min(B, k + 17)
+        m = U[k + 1:e, k] / U[k, k]
+        L[k + 1:e, k] = m
+        U[k + 1:e, k:e] -= np.outer(m, U[k, k:e])
+        U[k + 1:e, k] = 0
+    out = []
+    for c in range(nch):
+        s, lo, hi = slice(32 * c, 32 * c + 32), slice(32 * c - 16, 32 * c), slice(32 * c + 32, 32 * c + 48)
+        TL, TU = np.linalg.inv(L[s, s]), np.linalg.inv(U[s, s])
+        out.append((TL, -TL @ L[s, lo] if c else None, TU, -TU @ U[s, hi] if c + 1 < nch else None))
+    return out
+
+
+def _sweeps(F, b, dtype):
+    """M^-1 b by the two sweeps, in the arithmetic of dtype."""
+    nch = len(F)
+    F = [[t if t is None else t.astype(dtype) for t in f] for f in F]
+    x = np.zeros(32 * nch, dtype)
+    x[:len(b)] = b
+    for c in range(nch):
+        s = slice(32 * c, 32 * c + 32)
+        x[s] = F[c][0] @ x[s]
+        if c:
+            x[s] += F[c][1] @ x[32 * c - 16:32 * c]
+    for c in range(nch - 1, -1, -1):
+        s = slice(32 * c, 32 * c + 32)
+        x[s] = F[c][2] @ x[s]
+        if c + 1 < nch:
+            x[s] += F[c][3] @ x[32 * c + 32:32 * c + 48]
+    return x[:len(b)]
+
+
+@pytest.mark.parametrize("ns", [27, 60, 124, 250])
+def test_preconditioner_rows(tmp_path, native_lib, ns):
+    """The block solves with 8 warps per block row against the FP64 ones with
+    4, row by row relative to the row's value.  What FP64 sweeps leave there is
+    measured on the same factors, in double against extended precision; the
+    two kernels may differ by 8 times the worst row's (two errors of that kind,
+    the largest of a few hundred rows each)."""
+    prob, p = _problem(tmp_path, ns)
+    B = 2 * (ns + 5)
+    order = np.arange(B).reshape(2, -1).T.reshape(-1)      # a spline's two functions side by side
+    S, Hst = O.stationary(p, DT)
+    PT = (S + Hst).T.tocsr()
+    s = Solver(prob, DT)
+    seen = {}
+    for r in range(prob.n // B):
+        seen.setdefault(int(p.kappa[r]), r)                # one block row per kappa
+    fac = {r: _factors(PT[r * B + order][:, r * B + order].toarray()) for r in seen.values()}
+    for name, b in _vectors(prob.n // B, B, np.random.default_rng(ns)).items():
+        y = {}
+        for warps in (4, 8):
+            s.set_precond_warps(warps)
+            y[warps] = s.precond(b)
+        for r, F in fac.items():
+            rows = r * B + order
+            ext = _sweeps(F, b[rows], np.clongdouble)
+            e64 = (np.abs(_sweeps(F, b[rows], complex) - ext) / np.abs(ext)).max()
+            err = (np.abs(y[8][rows] - y[4][rows]) / np.abs(y[4][rows])).max()
+            assert err <= 8 * e64, (name, r, float(err), float(e64))
