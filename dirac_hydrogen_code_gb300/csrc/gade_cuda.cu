@@ -2087,11 +2087,6 @@ __device__ __forceinline__ long long pf_norm(long long S, int bits)
     return sh >= 0 ? S << sh : (fx_shr(S, -sh - 1) + 1) >> 1;
 }
 __device__ __forceinline__ int pf_cexp(int E, int bits) { return bits ? E - (PF_EX - 1080) - (58 - bits) : PF_LOW; }
-/* h 2^60 + m 2^30 in units of 2^59, to nearest */
-__device__ __forceinline__ long long pf_sum(long long h, long long m)
-{
-    return 2 * h + ((m + (1ll << (FX_WB - 2))) >> (FX_WB - 1));
-}
 
 /*
  * grid (pulse slot, block row), 8 warps; stages as in k_precond_tma (L
@@ -2307,10 +2302,10 @@ __global__ void __launch_bounds__(256, 2) k_precond_fx(PcT Q, int mode, const do
                 }
                 if (sw >= Q1) { hr0 = hr; mr0 = mr; hi0 = hi; mi0 = mi; }
                 long long *ds = pt + (size_t)wid * 4 * 32 + lane;
-                ds[0] = pf_sum(hr0, mr0);
-                ds[32] = pf_sum(hi0, mi0);
-                ds[64] = pf_sum(hr - hr0, mr - mr0);
-                ds[96] = pf_sum(hi - hi0, mi - mi0);
+                ds[0] = fx_sum59(hr0, mr0);
+                ds[32] = fx_sum59(hi0, mi0);
+                ds[64] = fx_sum59(hr - hr0, mr - mr0);
+                ds[96] = fx_sum59(hi - hi0, mi - mi0);
                 pe[wid * 64 + lane] = C0;
                 pe[wid * 64 + 32 + lane] = C1;
             }
@@ -2366,7 +2361,7 @@ __global__ void __launch_bounds__(256, 2) k_precond_fx(PcT Q, int mode, const do
                     fx_mad(m, gh, b.w);
                     fx_mad(m2, gl, b.z);
                 }
-                return pf_sum(h + h2, m + m2);
+                return fx_sum59(h + h2, m + m2);
             };
             if (wid < 4) {
                 /* four columns per warp; the four sums of a row meet in shared memory

@@ -46,17 +46,6 @@ __device__ __forceinline__ long long fx_from(double v, int em, int up)
     m = fx_shift(m << up, em - ev);
     return (long long)b < 0 ? -(long long)m : (long long)m;
 }
-/* the same for a float, |N| <= 2^57, in a group whose largest biased float
-   exponent is em: v = N 2^(em - 183) */
-__device__ __forceinline__ long long fx_from_float(float v, int em)
-{
-    const unsigned b = __float_as_uint(v);
-    int ev = (int)((b >> 23) & 0xFF);
-    unsigned long long m = b & 0x7FFFFFu;
-    if (ev) m |= 1ull << 23; else ev = 1;
-    m = fx_shift(m << 33, em - ev);
-    return (int)b < 0 ? -(long long)m : (long long)m;
-}
 /* two signed limbs of N */
 __device__ __forceinline__ int2 fx_split(long long N)
 {
@@ -156,6 +145,12 @@ __device__ __forceinline__ int2 fx_limbs(long long X)
 __device__ __forceinline__ long long fx_sum(long long h, long long m)
 {
     return (h << 2) + (m >> (FX_WB - 2));
+}
+/* the same in units of 2^59, to nearest: S 2^(e + C - 2100); sums of 66 products
+   stay below 2^63 */
+__device__ __forceinline__ long long fx_sum59(long long h, long long m)
+{
+    return 2 * h + ((m + (1ll << (FX_WB - 2))) >> (FX_WB - 1));
 }
 /* the value of a word in a group of exponent e */
 __device__ __forceinline__ double fx_value(int2 w, int e)

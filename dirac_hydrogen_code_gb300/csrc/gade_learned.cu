@@ -901,32 +901,42 @@ static cudaError_t launch_pod_partial(int n, int R, const float2 *U, const doubl
     return cudaGetLastError();
 }
 
-/* Stages NP vectors of len complex values as fixed-point limbs (re hi, re lo,
-   im hi, im lo), x_p = x + p ldx into q[p][stride]; every RL entries share an
-   exponent, s_ex[p][nrun].  Warps take runs; ends with a barrier. */
-template <int NP, int RL>
-__device__ __forceinline__ void l_stage_fx(const double2 *__restrict__ x, long long ldx, int np, int len, int stride,
-                                           int4 *q, int *s_ex, int nrun)
+/* Stages NP vectors of len complex values as limbs (gade_fx.cuh), x_p = x + p ldx
+   into q[p][PJ_L], with the exponent of each entry's larger part in ex[p][PJ_L];
+   bad[p]: an entry is not finite.  Ends with a barrier. */
+#define L_LOW (-20000)                 /* exponent of a zero */
+template <int NP>
+__device__ __forceinline__ void l_stage_fx(const double2 *__restrict__ x, long long ldx, int np, int len, int4 *q,
+                                           short *ex, int *bad)
 {
-    const int lane = threadIdx.x & 31;
-    for (int t = threadIdx.x >> 5; t < NP * nrun; t += 8) {
-        const int p = t / nrun, e0 = (t - p * nrun) * RL, e1 = min(len, e0 + RL);
-        unsigned mx = 0;
-#pragma unroll 8
-        for (int e = e0 + lane; e < e1; e += 32) {
-            const double2 v = p < np ? x[(size_t)p * ldx + e] : make_double2(0.0, 0.0);
-            mx = max(mx, max((unsigned)__double2hiint(v.x) & 0x7FFFFFFFu, (unsigned)__double2hiint(v.y) & 0x7FFFFFFFu));
-        }
-        const int em = max(fx_exp(__reduce_max_sync(0xffffffffu, mx)), 1);
-        if (lane == 0) s_ex[t] = em;
-#pragma unroll 4
-        for (int e = e0 + lane; e < e1; e += 32) {
-            const double2 v = p < np ? x[(size_t)p * ldx + e] : make_double2(0.0, 0.0);
-            const int2 re = fx_split(fx_from(v.x, em, FX_UPX)), im = fx_split(fx_from(v.y, em, FX_UPX));
-            q[p * stride + e] = make_int4(re.x, re.y, im.x, im.y);
+    if (threadIdx.x < NP) bad[threadIdx.x] = 0;
+    __syncthreads();
+    for (int e = threadIdx.x; e < len; e += 256) {
+        double2 v[NP];
+#pragma unroll
+        for (int p = 0; p < NP; p++) v[p] = p < np ? x[(size_t)p * ldx + e] : make_double2(0.0, 0.0);
+#pragma unroll
+        for (int p = 0; p < NP; p++) {
+            const int em = max(fx_exp(max((unsigned)__double2hiint(v[p].x) & 0x7FFFFFFFu,
+                                          (unsigned)__double2hiint(v[p].y) & 0x7FFFFFFFu)), 1);
+            if (em == 2047) bad[p] = 1;
+            const int2 re = fx_limbs(fx_from(v[p].x, em, FX_UPX)), im = fx_limbs(fx_from(v[p].y, em, FX_UPX));
+            q[p * PJ_L + e] = make_int4(re.x, re.y, im.x, im.y);
+            ex[p * PJ_L + e] = (short)(v[p].x == 0.0 && v[p].y == 0.0 ? L_LOW : em);
         }
     }
     __syncthreads();
+}
+
+/* N of a part of a basis entry whose larger part has the biased float exponent
+   e, v = N 2^(e - 182), as a word without an offset */
+__device__ __forceinline__ int2 l_word(float v, int e)
+{
+    const unsigned b = __float_as_uint(v);
+    const int ev = (int)((b >> 23) & 0xFF);
+    const long long m = (long long)(ev ? (b & 0x7FFFFFu) | 1u << 23 : b & 0x7FFFFFu) << 39;
+    const long long t = fx_shr(m, e - max(ev, 1));
+    return fx_word_of((int)b < 0 ? -t : t, 0);
 }
 
 /* sums NV (a power of two up to 32) doubles per lane over the warp, the values
@@ -958,81 +968,102 @@ __device__ __forceinline__ double l_warp_split_sum(double (&v)[NV])
 /* the same partial projections to FP64 accuracy (training targets are second
    differences of projections, which cancel).  The 8 n R npulse flops would be
    bound by the FP64 pipe (1.83 ms at n = 53,040, R = 128, 16 pulses, float to
-   double conversions included), so the products run in fixed point: 512
-   entries of a state share an exponent and so do a lane's 16 basis entries
-   among them, 32 real products are summed exactly, one FP64 addition per sum. */
-#define PD_B 16
+   double conversions included), so the products run on the integer units:
+   every entry of a state and of the basis has the exponent of its larger part,
+   8 of a lane's complex products are aligned to the largest and summed, the
+   sums of a chunk meet in 64-bit integers (a few 2^-54 of the sum of the
+   products' magnitudes).  356 us there for the whole call, bound by the integer
+   multiply-adds. */
+#define PD_B 8
 template <int NP>
 __global__ void __launch_bounds__(256, 2) k_pod_partial64(int n, int R, const float2 *__restrict__ U,
                                                           const double2 *__restrict__ x, long long ldx,
                                                           double2 *__restrict__ part, int npulse, int rows)
 {
-    extern __shared__ __align__(16) int4 xq[];       /* [NP][PJ_L] */
-    constexpr int RL = 32 * PD_B, NR = PJ_L / RL;
-    __shared__ int s_ex[NP * NR];
+    extern __shared__ __align__(16) int4 xq[];       /* [NP][PJ_L] limbs, [NP][PJ_L] exponents */
+    short *const xe = (short *)(xq + NP * PJ_L);
+    __shared__ int s_bad[NP];
     const int ch = blockIdx.x, p0 = blockIdx.y * NP;
     const int np = npulse - p0 < NP ? npulse - p0 : NP;
     const int i0 = ch * PJ_L;
     const int len = n - i0 < PJ_L ? n - i0 : PJ_L;
     const double2 *xc = x + (size_t)p0 * ldx + i0;
-    l_stage_fx<NP, RL>(xc, ldx, np, len, PJ_L, xq, s_ex, NR);
+    l_stage_fx<NP>(xc, ldx, np, len, xq, xe, s_bad);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int re = min(R, (int)(blockIdx.z + 1) * rows);
     for (int r = blockIdx.z * rows + warp; r < re; r += 8) {
         const float2 *u = U + (size_t)r * n + i0;
-        double v[2 * NP];
+        /* the lane's sums so far, S 2^(E - 1204); 4 groups of 16 real products stay below 2^63 */
+        static_assert(PJ_L == 4 * 32 * PD_B, "groups of a lane");
+        long long Sr[NP], Si[NP];
+        int E[NP];
 #pragma unroll
-        for (int j = 0; j < 2 * NP; j++) v[j] = 0.0;
+        for (int p = 0; p < NP; p++) { Sr[p] = Si[p] = 0; E[p] = 2 * L_LOW; }
+        bool ubad = false;
         for (int e0 = lane; e0 < len; e0 += 32 * PD_B) {
-            float2 uv[PD_B];
-            unsigned mx = 0;
-#pragma unroll
-            for (int k = 0; k < PD_B; k++) {
-                uv[k] = e0 + 32 * k < len ? __ldcs(&u[e0 + 32 * k]) : make_float2(0.f, 0.f);
-                mx = max(mx, max(__float_as_uint(uv[k].x) & 0x7FFFFFFFu, __float_as_uint(uv[k].y) & 0x7FFFFFFFu));
-            }
-            const int em = max((int)(mx >> 23), 1);
             int4 uq[PD_B];
+            int ue[PD_B];
 #pragma unroll
             for (int k = 0; k < PD_B; k++) {
-                const int2 a = fx_split(fx_from_float(uv[k].x, em)), b = fx_split(fx_from_float(uv[k].y, em));
+                const float2 w = e0 + 32 * k < len ? __ldcs(&u[e0 + 32 * k]) : make_float2(0.f, 0.f);
+                const unsigned mx = max(__float_as_uint(w.x) & 0x7FFFFFFFu, __float_as_uint(w.y) & 0x7FFFFFFFu);
+                const int em = max((int)(mx >> 23), 1);
+                ubad |= em == 255;
+                const int2 a = l_word(w.x, em), b = l_word(w.y, em);
                 uq[k] = make_int4(a.x, a.y, b.x, b.y);
+                ue[k] = mx ? em : L_LOW;
             }
 #pragma unroll
             for (int p = 0; p < NP; p++) {
-                const int ex = s_ex[p * NR + e0 / RL];
-                if (em != 255 && ex != 2047) {
-                    const int4 *xp = xq + p * PJ_L + e0;
-                    long long hr = 0, mr = 0, hi = 0, mi = 0;
+                const int4 *xp = xq + p * PJ_L + e0;
+                const short *ep = xe + p * PJ_L + e0;
+                int C = 2 * L_LOW, key[PD_B];
 #pragma unroll
-                    for (int k = 0; k < PD_B; k++) {
-                        /* past the chunk: u = 0 (the entry read belongs to this CTA's buffer) */
-                        const int4 b = xp[e0 + 32 * k < len ? 32 * k : 0];
-                        const int4 a = uq[k];
-                        hr += (long long)a.x * b.x;      /* conj(u) x */
-                        hr += (long long)a.z * b.z;
-                        mr += (long long)a.x * b.y;
-                        mr += (long long)a.y * b.x;
-                        mr += (long long)a.z * b.w;
-                        mr += (long long)a.w * b.z;
-                        hi += (long long)a.x * b.z;
-                        hi -= (long long)a.z * b.x;
-                        mi += (long long)a.x * b.w;
-                        mi += (long long)a.y * b.z;
-                        mi -= (long long)a.z * b.y;
-                        mi -= (long long)a.w * b.x;
-                    }
-                    const long long rnd = 1ll << (FX_LB - 1);
-                    v[2 * p] = fx_add(v[2 * p], hr + ((mr + rnd) >> FX_LB), em + ex - 1205);
-                    v[2 * p + 1] = fx_add(v[2 * p + 1], hi + ((mi + rnd) >> FX_LB), em + ex - 1205);
-                } else if (p < np) {
-                    /* an infinity or NaN: FP64 products */
-                    for (int e = e0; e < len && e < e0 + 32 * PD_B; e += 32) {
-                        const float2 a = u[e];
-                        const double2 b = xc[(size_t)p * ldx + e];
-                        v[2 * p] += (double)a.x * b.x + (double)a.y * b.y;
-                        v[2 * p + 1] += (double)a.x * b.y - (double)a.y * b.x;
-                    }
+                for (int k = 0; k < PD_B; k++) {
+                    /* past the chunk: u = 0 (the entry read belongs to this CTA's buffer) */
+                    key[k] = ue[k] + ep[e0 + 32 * k < len ? 32 * k : 0];
+                    C = max(C, key[k]);
+                }
+                long long hr = 0, mr = 0, hi = 0, mi = 0;
+#pragma unroll
+                for (int k = 0; k < PD_B; k++) {
+                    const int4 b = xp[e0 + 32 * k < len ? 32 * k : 0];
+                    int ah, al, gh, gl;
+                    fx_take(uq[k].x, uq[k].y, C - key[k], ah, al);
+                    fx_take(uq[k].z, uq[k].w, C - key[k], gh, gl);
+                    const int nx = -b.x, ny = -b.y;
+                    fx_mad(hr, ah, b.x);             /* conj(u) x */
+                    fx_mad(hr, gh, b.z);
+                    fx_mad(mr, ah, b.y);
+                    fx_mad(mr, al, b.x);
+                    fx_mad(mr, gh, b.w);
+                    fx_mad(mr, gl, b.z);
+                    fx_mad(hi, ah, b.z);
+                    fx_mad(hi, gh, nx);
+                    fx_mad(mi, ah, b.w);
+                    fx_mad(mi, al, b.z);
+                    fx_mad(mi, gh, ny);
+                    fx_mad(mi, gl, nx);
+                }
+                fx_join(Sr[p], E[p], fx_sum59(hr, mr), C);
+                fx_join(Si[p], E[p], fx_sum59(hi, mi), C);
+                E[p] = max(E[p], C);
+            }
+        }
+        ubad = __any_sync(0xffffffffu, ubad);
+        double v[2 * NP];
+#pragma unroll
+        for (int p = 0; p < NP; p++) {
+            v[2 * p] = fx_add(0.0, Sr[p], E[p] - 1204);
+            v[2 * p + 1] = fx_add(0.0, Si[p], E[p] - 1204);
+            if ((ubad || s_bad[p]) && p < np) {
+                /* an infinity or NaN: FP64 products */
+                v[2 * p] = v[2 * p + 1] = 0.0;
+                for (int e = lane; e < len; e += 32) {
+                    const float2 a = u[e];
+                    const double2 b = xc[(size_t)p * ldx + e];
+                    v[2 * p] += (double)a.x * b.x + (double)a.y * b.y;
+                    v[2 * p + 1] += (double)a.x * b.y - (double)a.y * b.x;
                 }
             }
         }
@@ -1048,7 +1079,7 @@ template <int NP>
 static cudaError_t launch_pod_partial64(int n, int R, const float2 *U, const double2 *x, long long ldx, double2 *part,
                                         int npulse, int nch, cudaStream_t st)
 {
-    const int smem = (int)sizeof(int4) * PJ_L * NP, rows = 32;
+    const int smem = (int)(sizeof(int4) + sizeof(short)) * PJ_L * NP, rows = 32;
     cudaError_t e = l_allow_smem<k_pod_partial64<NP>>(smem);
     if (e != cudaSuccess) return e;
     k_pod_partial64<NP><<<dim3(nch, (npulse + NP - 1) / NP, (R + rows - 1) / rows), 256, smem, st>>>(

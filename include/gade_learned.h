@@ -79,8 +79,10 @@ int gade_to_bf16(int64_t n, const float *x, void *y, void *stream);
 int gade_pod_project(int64_t n, int32_t R, const void *U, const void *x, int64_t ldx, int32_t npulse,
                      void *coef, void *scratch, int64_t scratch_bytes, void *stream);
 int64_t gade_pod_project_scratch(int64_t n, int32_t R, int32_t npulse);
-/* The same with FP64 products and sums in a fixed order (relative error
- * ~1e-15): for training targets, second differences of projections. */
+/* The same to FP64 accuracy, in a fixed order (error a few 2^-53 of
+ * sum |U_i x_i|, however the entries are spread; products on the integer
+ * units, every entry with an exponent of its own): for training targets,
+ * second differences of projections. */
 int gade_pod_project_fp64(int64_t n, int32_t R, const void *U, const void *x, int64_t ldx, int32_t npulse,
                           void *coef, void *scratch, int64_t scratch_bytes, void *stream);
 

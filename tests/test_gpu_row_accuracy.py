@@ -133,3 +133,40 @@ def test_preconditioner_rows(tmp_path, native_lib, ns):
             e64 = (np.abs(_sweeps(F, b[rows], complex) - ext) / np.abs(ext)).max()
             err = (np.abs(y[8][rows] - y[4][rows]) / np.abs(y[4][rows])).max()
             assert err <= 8 * e64, (name, r, float(err), float(e64))
+
+
+@pytest.mark.parametrize("n", [37, 1024, 3000])
+@pytest.mark.parametrize("R,P", [(1, 1), (5, 2), (33, 4), (9, 7)])
+def test_projection_of_spread_entries(native_lib, n, R, P):
+    """gade_pod_project_fp64 with the entries of the basis and of the states
+    spread over 24 orders of magnitude each, apart, together and opposed (so
+    that every product is of one size): within 2e-15 of sum |U_i x_i|, a chunk's
+    1,024 complex products in FP64 (their random walk is 64 x 2^-53 at most,
+    and a lane sums only 32 of them)."""
+    import torch
+    from dirac_hydrogen_code_gb300 import native
+    rng = np.random.default_rng(n + R + P)
+    t = rng.uniform(-12, 12, n)
+    z = rng.standard_normal((R, n)) + 1j * rng.standard_normal((R, n))
+    w = rng.standard_normal((P, n)) + 1j * rng.standard_normal((P, n))
+    for su, sx in ((t, -t), (t, t), (t, rng.uniform(-12, 12, n)), (0 * t, t)):
+        U = (z * 10.0 ** su).astype(np.complex64)
+        x = w * 10.0 ** sx
+        Ud, xd = torch.from_numpy(U).cuda(), torch.from_numpy(x).cuda()
+        sb = native.call("gade_pod_project_scratch", n, R, P)
+        scratch = torch.empty(sb, dtype=torch.uint8, device="cuda")
+        coef = torch.empty(P, R, dtype=torch.complex128, device="cuda")
+        native.call("gade_pod_project_fp64", n, R, Ud.data_ptr(), xd.data_ptr(), n, P, coef.data_ptr(),
+                    scratch.data_ptr(), sb, 0)
+        torch.cuda.synchronize()
+        U64 = U.astype(np.clongdouble)
+        ref, mag = x @ U64.conj().T, np.abs(x) @ np.abs(U64).T
+        assert np.all(np.abs(coef.cpu().numpy() - ref) <= 2e-15 * mag)
+        # a NaN reaches its own coefficients only
+        xd[P - 1, n // 2] = float("nan")
+        native.call("gade_pod_project_fp64", n, R, Ud.data_ptr(), xd.data_ptr(), n, P, coef.data_ptr(),
+                    scratch.data_ptr(), sb, 0)
+        torch.cuda.synchronize()
+        c = coef.cpu().numpy()
+        assert np.isnan(c[P - 1]).all()
+        assert np.all(np.abs(c[:P - 1] - ref[:P - 1]) <= 2e-15 * mag[:P - 1])
