@@ -3545,13 +3545,16 @@ static int solver_create(const gade_problem *p, int npulse, const double *dts, c
         cudaFuncSetAttribute(k_precond_tma<double, 16, 8>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm64);
         cudaFuncSetAttribute(k_precond_tma<double, 32, 8>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm64);
         /* k_precond_fx is written for 16 chain columns (half-bandwidth <= 16,
-           both bases' own ordering) and must fit an SM (Bp <= 4,500); wider
+           both bases' own ordering) and must fit an SM (Bp <= 3,680); wider
            bands and larger blocks keep the FP64 kernel, and so do batches whose
-           second copy of the factors would take a tenth of the free memory */
+           second copy of the factors would take a twentieth of the device's
+           memory (of all of it: by what is free, two solvers of one problem
+           could differ in their last bits).  Mixed precision solves with
+           complex64 factors only, so its complex128 solves (gade_solver_precond)
+           need no copy: FP64. */
         const size_t smx = pf_smem(s->Bp);
-        size_t fr = 0, tot = 0;
-        if (cudaMemGetInfo(&fr, &tot) != cudaSuccess) fr = 0;
-        if (s->bwp == PF_BW && smx <= 220 * 1024 && 2 * sizeof(int4) * NP * s->fstride < fr / 10) {
+        if (s->prec == GADE_PREC_FP64 && s->bwp == PF_BW && smx <= 220 * 1024 &&
+            2 * sizeof(int4) * NP * s->fstride < prop.totalGlobalMem / 20) {
             cudaFuncSetAttribute(k_precond_fx, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smx);
             UP(s->d_XL, (const int4 *)nullptr, NP * s->fstride);
             UP(s->d_XU, (const int4 *)nullptr, NP * s->fstride);
