@@ -1354,10 +1354,9 @@ __global__ void __launch_bounds__(128, 6) k_assemble(int2 *__restrict__ A, unsig
 #define ASM_XZERO (-20000) /* exponent of a zero entry of x: no product of it is a row's largest */
 #define ASM_GB 16   /* coupled blocks staged per phase: two per warp */
 /* what a piece costs beyond its pairs, in pairs: staging, exchange, the arrival
-   count and the next piece's descriptor, 8-12 us of latencies under load where a
-   pair takes 1.4 us.  4: 6,437 us for 8 steps at N = 53,040 and 9,166 us for 2
-   at N = 244,000, 6: 6,411 and 9,158, 8: 6,429 and 9,136; charged once per unit
-   instead of per piece, as 4: 6,469 and 9,240. */
+   count and the next piece's descriptor.  3 and 6 give the same times from
+   N = 21,840 to 244,000 (76 and 77 us to 764 and 763); 6 tells the sizes apart
+   where the partition does not pay (balanced_partition). */
 #ifndef ASM_UFIX
 #define ASM_UFIX 6.0
 #endif
@@ -4000,9 +3999,6 @@ static int asm_partitions(gade_solver *s)
         }
         if ((rc = part_upload(s, s->part_asm[0], seg, pcs))) return rc;
     }
-    /* a pair's and a piece's cost */
-    auto pcost = [&](int q) { return 2.0 * s->h_chunk_nrows[q] * s->W + 2.0 * s->h_chunk_ncols[q]; };
-    auto ufix = [&](int q) { return ASM_UFIX * pcost(q); };
     /* units are cut at multiples of the pairs that k_apply_asm's thread groups take side by side */
     const int cut = std::max(1, std::min(4, 256 / std::max(1, s->RMA / 2)));
     for (int cls = 0; cls < 4; cls++) {
@@ -4010,6 +4006,13 @@ static int asm_partitions(gade_solver *s)
         if (f == 1 && s->prec != GADE_PREC_MIXED) continue;
         if (s->part_asm_bal[o].nseg) continue;
         const int nseg = o * s->nsm;
+        /* A pair's cost in full chunks: k_apply_asm is bound by its threads'
+           instructions, and a short chunk leaves threads idle, so a pair takes as
+           long there as in a full one (with the rows' share the partition was
+           slower than the plain one where the last chunk is short: 133 us at
+           N = 42,640, now 111); the complex64 kernel streams a chunk's rows. */
+        auto pcost = [&](int q) { return f ? (double)s->h_chunk_nrows[q] / s->RM : 1.0; };
+        auto ufix = [&](int q) { return ASM_UFIX * pcost(q); };
         std::vector<int4> pcs;
         std::vector<int> pseg;
         /* units in order, cut where a segment's cost reaches T; false when
@@ -4684,13 +4687,6 @@ static int time_fp64_apply(gade_solver *s, float *ms)
     return rc;
 }
 
-/*
- * Matrix-free or assembled operator for one pulse with real couplings:
- * the assembled values (K_a) are built, both of their partitions timed, and
- * the assembled operator is kept when its apply is clearly faster than the
- * matrix-free one chosen by choose_split (its per-step assembly replaces the
- * radial tables).
- */
 /* ms of the step's tables of the current operator: the matrix-free radial
    tables or the assembly of the coupling values (float copies included in
    mixed precision) */
@@ -4724,6 +4720,23 @@ static float step_cost(const gade_solver *s, float tables_ms, float apply_ms)
     return tables_ms + (s->prec == GADE_PREC_MIXED ? 1.0f : 3.0f) * apply_ms;
 }
 
+/* Whether the assembled operator runs its balanced partition: by the cost model,
+   not by the two timed applies: where these are close the choice, and with it
+   the order of the sums, would differ between solvers of one problem.
+   Measured (model's gain; plain, balanced us): N = 8,400 (too few pairs) 21,
+   21-32; 12,600 (1.08) 45, 48; 18,600 (0.93) 45, 51; 21,840 (1.37) 86, 76;
+   30,600 (1.22) 92, 77; 42,640 (1.38) 135, 111; 53,040 (1.38) 137, 110; 63,440
+   (1.20) 156, 134; 93,480 (1.10) 310, 294; 139,080 (1.11) 383, 369; 244,000
+   (1.05) 750, 764.  The line lies between 1.08 and 1.10. */
+static int balanced_partition(const gade_solver *s) { return s->asm_bal_gain > 1.085 ? 1 : 0; }
+
+/*
+ * Matrix-free or assembled operator for one pulse with real couplings:
+ * the assembled values (K_a) are built, both of their partitions timed, and
+ * the assembled operator is kept when its apply is clearly faster than the
+ * matrix-free one chosen by choose_split (its per-step assembly replaces the
+ * radial tables).
+ */
 static int choose_operator(gade_solver *s)
 {
     s->mf_ms = s->split_ms[s->nsplit >= 1 && s->nsplit <= 4 ? s->nsplit : 0];
@@ -4740,11 +4753,7 @@ static int choose_operator(gade_solver *s)
     }
     if (!rc) rc = time_step_tables(s, &tab_asm);
     if (rc) { s->use_asm = 0; return rc; }
-    /* by the cost model, not by the two times: where these are close the choice,
-       and with it the order of the sums, would differ between solvers of one
-       problem.  Measured (plain, balanced): N = 8,400 21 and 22 us (2 pairs per
-       CTA), N = 53,040 88 and 81 us, N = 244,000 510 and 503 us. */
-    s->asm_part = s->asm_bal_gain > 1.03 ? 1 : 0;
+    s->asm_part = balanced_partition(s);
     const float best = s->asm_ms[s->asm_part];
     s->tab_ms[0] = tab_mf;
     s->tab_ms[1] = tab_asm;
@@ -4766,7 +4775,7 @@ extern "C" int gade_solver_set_operator(gade_solver *s, int32_t assembled)
         if (!s->asm_ok)
             return fail(GADE_ERR_ARG, "gade_solver_set_operator: the assembled operator needs real couplings, "
                                       "each pair coupled by orders of one parity, and device memory for its values");
-        s->asm_part = 1;
+        s->asm_part = balanced_partition(s);
     }
     if (s->engine) batch_drop_graphs(s->engine);
     s->use_asm = assembled;
