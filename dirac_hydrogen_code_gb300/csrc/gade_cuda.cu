@@ -1349,7 +1349,7 @@ __global__ void __launch_bounds__(128, 6) k_assemble(int2 *__restrict__ A, unsig
     }
 }
 
-#define ASM_GS 8                       /* slots of a row summed with one alignment */
+#define ASM_GS 8                       /* slots of a row summed with one alignment (4: 735 us at N = 244,000, 5: 721, 8: 702) */
 #define ASM_GPH ((15 + ASM_GS - 1) / ASM_GS)
 #define ASM_XZERO (-20000) /* exponent of a zero entry of x: no product of it is a row's largest */
 #define ASM_GB 16   /* coupled blocks staged per phase: two per warp */
@@ -1399,11 +1399,11 @@ __host__ __device__ __forceinline__ unsigned asm_smem(int XS, int W, int RM, boo
  * NG partial sums of a row meet in shared memory, where two threads per row
  * add the diagonal blocks in FP64.
  * N = 53,040 (41.7M values, 0.33 GB): 188 us with FP64 products (FP64 pipe
- * bound), 110 us now (3.0 TB/s; some 30 instructions per value and the
- * staging, exchange and epilogue of each CTA, which do not overlap its
- * stream); N = 244,000 (2.8 GB): 1.36 ms, now 0.75 ms.  At N = 53,040 two
- * CTAs with 128 registers and every load of a pair in flight take 110 us,
- * three with 80 registers (spills) 129-137.
+ * bound), 103 us now (3.2 TB/s; some 33 instructions per value at 1.6 per
+ * clock, and the staging, exchange and epilogue of each CTA, which do not
+ * overlap its stream); N = 244,000 (2.8 GB): 1.36 ms, now 0.69 ms.  A group of
+ * slots is loaded while the one before it is multiplied (0.75 ms without); two
+ * CTAs with 128 registers: three with 80 spill (129 us).
  * HL: the halves layout (slot 15 h + t of a row of spline s is spline
  * s - 7 + t of half h); otherwise the slots' columns come from a table.
  */
@@ -1547,10 +1547,20 @@ __global__ void __launch_bounds__(256, 2)
         }
         __syncthreads();
         if (act) {
+            /* a group of slots is loaded while the one before it is multiplied */
+            int4 nx[ASM_GS];
+            auto load = [&](int g, int gs) {
+                const int ts = gs % ASM_GPH * ASM_GS, sl = gs / ASM_GPH * HJ + ts;
+                const int2 *Av = Aq + ((size_t)(pg + g) * W + sl) * RMq;
+#pragma unroll
+                for (int t = 0; t < ASM_GS; t++)
+                    if (ts + t < HJ)
+                        nx[t] = HL || sl + t < W ? __ldcs((const int4 *)(Av + (size_t)t * RMq)) : make_int4(FX_OFF, 0, FX_OFF, 0);
+            };
+            if (grp < ng) load(grp, 0);
             for (int g = grp; g < ng; g += NG) {
                 const ushort2 ea = *(const ushort2 *)(P.Ae + (size_t)pulse * P.aestride + (size_t)(pg + g) * P.Bp + off +
                                                       2 * rp);
-                const int2 *Av = Aq + (size_t)(pg + g) * W * RMq;
                 if (!s_ex[g]) {
                     const int w0 = HL ? 2 * rp - hb : 0;
                     const int4 *xg = xw + g * XS + w0;
@@ -1563,25 +1573,25 @@ __global__ void __launch_bounds__(256, 2)
                         const int hh = gs / ASM_GPH, ts = gs % ASM_GPH * ASM_GS;
                         const int nsl = min(ASM_GS, HJ - ts), sl = hh * HJ + ts;
                         const int ws = hh * HW + ts;
-                        int4 av[ASM_GS];       /* the group's loads in flight */
+                        int4 av[ASM_GS];
 #pragma unroll
-                        for (int t = 0; t < ASM_GS; t++)
-                            av[t] = t < nsl && (HL || sl + t < W) ? __ldcs((const int4 *)(Av + (size_t)(sl + t) * RMq))
-                                                                  : make_int4(FX_OFF, 0, FX_OFF, 0);
+                        for (int t = 0; t < ASM_GS; t++) av[t] = nx[t];
+                        if (gs + 1 < 2 * ASM_GPH) load(g, gs + 1);
+                        else if (g + NG < ng) load(g + NG, 0);
                         /* window entry of slot t for the first row; the second row's is one on (halves layout) */
                         auto at = [&](int t, int rr) {
                             return HL ? ws + t + rr : (int)lc[min(sl + t, W - 1) * RMA + 2 * rp + rr];
                         };
-                        int C0 = 2 * ASM_XZERO, C1 = C0;       /* the rows' largest products */
+                        int k0[ASM_GS], k1[ASM_GS], C0 = 2 * ASM_XZERO, C1 = C0;   /* the rows' products and the largest */
 #pragma unroll
-                        for (int t = 0; t < ASM_GS; t++) {
-                            C0 = max(C0, eg[at(t, 0)] - (av[t].x & FX_OFF));
-                            C1 = max(C1, eg[at(t, 1)] - (av[t].z & FX_OFF));
+                        for (int t = 0; t < nsl; t++) {
+                            C0 = max(C0, k0[t] = eg[at(t, 0)] - (av[t].x & FX_OFF));
+                            C1 = max(C1, k1[t] = eg[at(t, 1)] - (av[t].z & FX_OFF));
                         }
                         long long h0r = 0, m0r = 0, h0i = 0, m0i = 0, h1r = 0, m1r = 0, h1i = 0, m1i = 0;
                         int4 b1 = HL ? xg[ws] : make_int4(0, 0, 0, 0);
 #pragma unroll
-                        for (int t = 0; t < ASM_GS; t++) {
+                        for (int t = 0; t < nsl; t++) {
                             int4 b0 = b1;
                             if (HL) {
                                 b1 = xg[ws + t + 1];
@@ -1590,14 +1600,14 @@ __global__ void __launch_bounds__(256, 2)
                                 b1 = xg[at(t, 1)];
                             }
                             int h, l;
-                            fx_take(av[t].x, av[t].y, C0 - eg[at(t, 0)] + (av[t].x & FX_OFF), h, l);
+                            fx_take(av[t].x, av[t].y, C0 - k0[t], h, l);
                             fx_mad(h0r, h, b0.x);
                             fx_mad(m0r, h, b0.y);
                             fx_mad(m0r, l, b0.x);
                             fx_mad(h0i, h, b0.z);
                             fx_mad(m0i, h, b0.w);
                             fx_mad(m0i, l, b0.z);
-                            fx_take(av[t].z, av[t].w, C1 - eg[at(t, 1)] + (av[t].z & FX_OFF), h, l);
+                            fx_take(av[t].z, av[t].w, C1 - k1[t], h, l);
                             fx_mad(h1r, h, b1.x);
                             fx_mad(m1r, h, b1.y);
                             fx_mad(m1r, l, b1.x);
@@ -1625,6 +1635,7 @@ __global__ void __launch_bounds__(256, 2)
                         acc1.y = fx_add(acc1.y, S1i, e1);
                     }
                 } else {
+                    if (g + NG < ng) load(g + NG, 0);
                     /* an infinity or NaN in the window: products in FP64, so that it
                        reaches the rows that hold it and no others */
                     const C *xc = x + (size_t)P.pair_c[pg + g] * B;
@@ -1636,7 +1647,7 @@ __global__ void __launch_bounds__(256, 2)
                             const int cc = column(w);
                             if (cc < 0) continue;
                             const double a = e == ASM_NAN ? __longlong_as_double(0x7FF8000000000000ll)
-                                                          : fx_value(Av[(size_t)t * RMq + rr], e);
+                                                          : fx_value(Aq[((size_t)(pg + g) * W + t) * RMq + rr], e);
                             rfma(rr ? acc1 : acc0, a, xc[cc]);
                         }
                     }
@@ -4010,7 +4021,7 @@ static int asm_partitions(gade_solver *s)
            instructions, and a short chunk leaves threads idle, so a pair takes as
            long there as in a full one (with the rows' share the partition was
            slower than the plain one where the last chunk is short: 133 us at
-           N = 42,640, now 111); the complex64 kernel streams a chunk's rows. */
+           N = 42,640 where it now took 111); the complex64 kernel streams a chunk's rows. */
         auto pcost = [&](int q) { return f ? (double)s->h_chunk_nrows[q] / s->RM : 1.0; };
         auto ufix = [&](int q) { return ASM_UFIX * pcost(q); };
         std::vector<int4> pcs;
@@ -4724,10 +4735,11 @@ static float step_cost(const gade_solver *s, float tables_ms, float apply_ms)
    not by the two timed applies: where these are close the choice, and with it
    the order of the sums, would differ between solvers of one problem.
    Measured (model's gain; plain, balanced us): N = 8,400 (too few pairs) 21,
-   21-32; 12,600 (1.08) 45, 48; 18,600 (0.93) 45, 51; 21,840 (1.37) 86, 76;
-   30,600 (1.22) 92, 77; 42,640 (1.38) 135, 111; 53,040 (1.38) 137, 110; 63,440
-   (1.20) 156, 134; 93,480 (1.10) 310, 294; 139,080 (1.11) 383, 369; 244,000
-   (1.05) 750, 764.  The line lies between 1.08 and 1.10. */
+   20; 5,880 (too few) 25, 32; 12,600 (1.08) 43, 47; 18,600 (0.93) 43, 50;
+   21,840 (1.37) 81, 71; 30,600 (1.22) 86, 72; 42,640 (1.38) 123, 103; 53,040
+   (1.38) 129, 104; 63,440 (1.20) 142, 127; 93,480 (1.10) 283, 274; 139,080
+   (1.11) 350, 341; 244,000 (1.05) 693, 704.  The line lies between 1.08 and
+   1.10. */
 static int balanced_partition(const gade_solver *s) { return s->asm_bal_gain > 1.085 ? 1 : 0; }
 
 /*
