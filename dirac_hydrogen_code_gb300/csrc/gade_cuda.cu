@@ -2229,12 +2229,6 @@ __global__ void __launch_bounds__(256, 2) k_precond_fx(PcT Q, int mode, const do
 
     int k = 0;
     for (; k < ns; k++) {
-        if (tid == 0 && k + 1 < ns && k + 1 != Q.withhold) {
-            const int4 *src;
-            int cnt;
-            const unsigned bytes = stage(k + 1, &src, &cnt);
-            tma_bulk_load(stg + ((k + 1) & 1) * SB, src, bytes, &bar[(k + 1) & 1]);
-        }
         unsigned spins = 0;
         bool ok = true;
         while (!mbar_try_wait(&bar[k & 1], (k >> 1) & 1)) {
@@ -2243,6 +2237,15 @@ __global__ void __launch_bounds__(256, 2) k_precond_fx(PcT Q, int mode, const do
         if (!ok) all_ok = 0;
         __syncthreads();
         if (!all_ok) break;
+        /* the next stage, into the buffer that the last one left: issued by a warp
+           with slack in both kinds of stages, while the others start (by the
+           first thread before the barrier it took 500 cycles a stage) */
+        if (tid == 224 && k + 1 < ns && k + 1 != Q.withhold) {
+            const int4 *src;
+            int cnt;
+            const unsigned bytes = stage(k + 1, &src, &cnt);
+            tma_bulk_load(stg + ((k + 1) & 1) * SB, src, bytes, &bar[(k + 1) & 1]);
+        }
         const int4 *S = stg + (k & 1) * SB;
         const int up = k >= nps;                   /* U sweep */
         const int j = up ? k - nps : k;
@@ -2253,7 +2256,7 @@ __global__ void __launch_bounds__(256, 2) k_precond_fx(PcT Q, int mode, const do
                 const int b = max(pf_bits(X.x), pf_bits(X.y));
                 const int2 re = fx_limbs(pf_norm(X.x, b)), im = fx_limbs(pf_norm(X.y, b));
                 xq[o] = make_int4(re.x, re.y, im.x, im.y);
-                xe[o] = X.x == 0 && X.y == 0 ? PF_LOW : pf_cexp(tE[o], b);
+                xe[o] = pf_cexp(tE[o], b);
             }
             __syncthreads();
         }
@@ -2273,21 +2276,17 @@ __global__ void __launch_bounds__(256, 2) k_precond_fx(PcT Q, int mode, const do
                 int4 d[9];
                 int key[9];
                 int C0 = 2 * PF_LOW, C1 = C0;          /* the rows' largest products */
-#pragma unroll
-                for (int n = 0; n < 9; n++) {
-                    /* only the first part has a ninth product (the others' is left out below) */
-                    const int q = n == 8 ? min(Q0 + 8, 32) : Q0 + n;
+                auto exponent = [&](int n) {
+                    const int q = Q0 + n;
                     d[n] = T[q * 32];
-                    key[n] = n == 8 && part > 0 ? 2 * PF_LOW : pf_exp(d[n]) + xe[q + (q <= sw ? b0 : b1)];
+                    key[n] = pf_exp(d[n]) + xe[q + (q <= sw ? b0 : b1)];
                     C0 = q <= sw ? max(C0, key[n]) : C0;
                     C1 = q <= sw ? C1 : max(C1, key[n]);
-                }
+                };
                 long long hr = 0, mr = 0, hi = 0, mi = 0, hr0 = 0, mr0 = 0, hi0 = 0, mi0 = 0;
-#pragma unroll
-                for (int n = 0; n < 9; n++) {
-                    const int q = n == 8 ? min(Q0 + 8, 32) : Q0 + n;
-                    int4 b = xq[q + (q <= sw ? b0 : b1)];
-                    if (n == 8 && part > 0) b = make_int4(0, 0, 0, 0);
+                auto product = [&](int n) {
+                    const int q = Q0 + n;
+                    const int4 b = xq[q + (q <= sw ? b0 : b1)];
                     const int s = (q <= sw ? C0 : C1) - key[n];
                     int ah, al, gh, gl;
                     fx_take(d[n].x, d[n].y, s, ah, al);
@@ -2306,10 +2305,16 @@ __global__ void __launch_bounds__(256, 2) k_precond_fx(PcT Q, int mode, const do
                     fx_mad(mi, gh, b.y);
                     fx_mad(mi, gl, b.x);
                     /* the products up to sw belong to the row of c0 */
-                    const bool last = q == sw && (n < 8 || part == 0);
+                    const bool last = q == sw;
                     hr0 = last ? hr : hr0; mr0 = last ? mr : mr0;
                     hi0 = last ? hi : hi0; mi0 = last ? mi : mi0;
-                }
+                };
+#pragma unroll
+                for (int n = 0; n < 8; n++) exponent(n);
+                if (part == 0) exponent(8);            /* only the first part has a ninth product */
+#pragma unroll
+                for (int n = 0; n < 8; n++) product(n);
+                if (part == 0) product(8);
                 if (sw >= Q1) { hr0 = hr; mr0 = mr; hi0 = hi; mi0 = mi; }
                 long long *ds = pt + (size_t)wid * 4 * 32 + lane;
                 ds[0] = fx_sum59(hr0, mr0);
@@ -2354,7 +2359,8 @@ __global__ void __launch_bounds__(256, 2) k_precond_fx(PcT Q, int mode, const do
                 C = 2 * PF_LOW;
 #pragma unroll
                 for (int q = 0; q < n; q++) {
-                    key[q] = pf_exp(d[q]) + ex[q];
+                    const int4 e4 = *(const int4 *)(ex + (q & ~3));
+                    key[q] = pf_exp(d[q]) + ((q & 3) == 0 ? e4.x : (q & 3) == 1 ? e4.y : (q & 3) == 2 ? e4.z : e4.w);
                     C = max(C, key[q]);
                 }
                 long long h = 0, h2 = 0, m = 0, m2 = 0;
@@ -2412,8 +2418,7 @@ __global__ void __launch_bounds__(256, 2) k_precond_fx(PcT Q, int mode, const do
                     const int2 l = fx_limbs(pf_norm(X, b));
                     /* every warp writes the same values: the next step reads what its own warp wrote */
                     put_limbs(xq + 32 * c, l);
-                    const bool zero = __shfl_xor_sync(0xffffffffu, X == 0, 1) && X == 0;
-                    if (comp == 0) xe[32 * c + row16] = zero ? PF_LOW : pf_cexp(E, b);
+                    if (comp == 0) xe[32 * c + row16] = pf_cexp(E, b);
                     __syncwarp();
                     if (wid == 0) {
                         *tp = X;
@@ -2459,12 +2464,11 @@ __global__ void __launch_bounds__(256, 2) k_precond_fx(PcT Q, int mode, const do
     if (!all_ok) {
         if (tid == 0) {
             atomicOr(&sc->err, 1u);
-            /* drain the copies still in flight (bounded) before exiting: the
-               stage that timed out and the next one, both issued unless withheld */
-            for (int k2 = k; k2 < k + 2 && k2 < ns; k2++) {
-                if (k2 == Q.withhold) continue;
+            /* drain the copy still in flight (bounded) before exiting: that of the
+               stage whose wait ran out, unless withheld (the next is not issued) */
+            if (k < ns && k != Q.withhold) {
                 unsigned spins = 0;
-                while (!mbar_try_wait(&bar[k2 & 1], (k2 >> 1) & 1) && ++spins < MBAR_SPIN_LIMIT) {
+                while (!mbar_try_wait(&bar[k & 1], (k >> 1) & 1) && ++spins < MBAR_SPIN_LIMIT) {
                 }
             }
         }
