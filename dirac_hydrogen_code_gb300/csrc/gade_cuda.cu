@@ -1624,16 +1624,12 @@ __global__ void __launch_bounds__(256, 2)
                     }
                     if (ea.x == 0) S0r = S0i = 0;          /* a row without values */
                     if (ea.y == 0) S1r = S1i = 0;
-                    if (ea.x == ASM_NAN || ea.y == ASM_NAN) {
-                        acc0 = mk<C>(__longlong_as_double(0x7FF8000000000000ll), __longlong_as_double(0x7FF8000000000000ll));
-                        acc1 = acc0;
-                    } else {
-                        const int e0 = ea.x + E0 - 2101, e1 = ea.y + E1 - 2101;
-                        acc0.x = fx_add(acc0.x, S0r, e0);
-                        acc0.y = fx_add(acc0.y, S0i, e0);
-                        acc1.x = fx_add(acc1.x, S1r, e1);
-                        acc1.y = fx_add(acc1.y, S1i, e1);
-                    }
+                    /* ASM_NAN: far above any other exponent, a NaN for this row */
+                    const int e0 = ea.x + E0 - 2101, e1 = ea.y + E1 - 2101;
+                    acc0.x = fx_add(acc0.x, S0r, e0);
+                    acc0.y = fx_add(acc0.y, S0i, e0);
+                    acc1.x = fx_add(acc1.x, S1r, e1);
+                    acc1.y = fx_add(acc1.y, S1i, e1);
                 } else {
                     if (g + NG < ng) load(g + NG, 0);
                     /* an infinity or NaN in the window: products in FP64, so that it

@@ -55,12 +55,13 @@ __device__ __forceinline__ int2 fx_split(long long N)
     return r;
 }
 __device__ __forceinline__ double pow2d(int e) { return __hiloint2double((e + 1023) << 20, 0); }   /* -1022 <= e <= 1023 */
+#define FX_NAN 20000                   /* exponents from here on make a sum NaN */
 /* acc += V 2^e; e of any size (below the normal range in two factors) */
 __device__ __forceinline__ double fx_add(double acc, long long V, int e)
 {
     double v = (double)V;
     if (e < -1022) { v *= pow2d(e + 900 < -1022 ? -1022 : e + 900); e = -900; }
-    return fma(v, pow2d(e > 1023 ? 1023 : e), acc);
+    return fma(v, e >= FX_NAN ? __longlong_as_double(0x7FF8000000000000ll) : pow2d(e > 1023 ? 1023 : e), acc);
 }
 /* the upper 16 bits of a double >= v (v >= 0): sign, exponent and 4 mantissa bits, rounded up */
 __device__ __forceinline__ unsigned short fx_bound16(double v)

@@ -111,3 +111,24 @@ def test_mixed_solver_complex128_solves(tmp_path, native_lib, form):
         assert np.linalg.norm(PT @ z - b) <= 1e-13 * np.linalg.norm(abs(PT) @ abs(z) + abs(b))
         y.append(z)
     assert np.linalg.norm(y[0] - y[1]) <= 1e-13 * np.linalg.norm(y[0])
+
+
+def test_nan_in_a_coupling_table(tmp_path, native_lib):
+    """A NaN in one radial table entry reaches the same rows of the assembled
+    operator as of the matrix-free one."""
+    prob, p = _problem(tmp_path, 28, "")
+    d, lmax = str(tmp_path), prob.info["lmax"]
+    path = next(os.path.join(d, f"g{q}a{a}l{l}.csr") for l in range(lmax) for a in range(6) for q in range(4)
+                if a % 2 != l % 2 and np.abs(formats.csr_read(os.path.join(d, f"g{q}a{a}l{l}.csr")).Ax).max() > 0)
+    m = formats.csr_read(path)
+    m.Ax[np.abs(m.Ax).argmax()] = np.nan
+    formats.csr_write(path, m)
+    s = Solver(Problem(d, lmax), DT)
+    rng = np.random.default_rng(2)
+    x = rng.standard_normal(prob.n) + 1j * rng.standard_normal(prob.n)
+    fin = []
+    for op in (0, 1):
+        s.set_operator(op)
+        s.set_time(pulse(10, 50.0, 1, 70 * DT))
+        fin.append(np.isfinite(s.apply(x)))
+    assert np.array_equal(fin[0], fin[1]) and not fin[0].all() and fin[0].any()
