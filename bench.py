@@ -478,8 +478,8 @@ def run_ours(args):
                    else "k_apply (matrix-free S + H(t) apply)"),
         "note": ("achieved = CSR-equivalent bytes of the reference assembled complex128 SpMV "
                  "(20 nnz + 4(N+1) + 32N) / average operator apply time over the sampled steps; the kernel "
-                 "streams real coupling values (8 B fixed point) and multiplies them on the integer units; it is "
-                 "bound by HBM and the latencies around the stream, see compulsory_bytes" if assembled else
+                 "streams real coupling values (8-byte words) and multiplies them on the integer units; it is "
+                 "bound by its integer instructions and the latencies around the stream" if assembled else
                  "achieved = CSR-equivalent bytes of the reference assembled complex128 SpMV "
                  "(20 nnz + 4(N+1) + 32N) / average k_apply time over the sampled steps; the matrix-free "
                  "kernel moves far fewer bytes and is bound by the FP64 pipe, see fp64"),

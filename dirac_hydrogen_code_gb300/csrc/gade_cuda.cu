@@ -1216,8 +1216,8 @@ struct A32Map {
  * their values are: |A| <= sum_ia |w_ia| max|K_ia|.  The three products of a
  * value are aligned to their largest and summed on the integer units, to
  * 2^-53 of that product, so every value is as accurate as in FP64.  One pulse
- * runs at the memory rate (24 bytes in per value and pulse group, 8 out per
- * pulse): 196 us at 41.7M values, 6.8 TB/s (209 us with three FP64 DFMA per
+ * runs near the memory rate (24 bytes in per value and pulse group, 8 out per
+ * pulse): 196 us at 41.7M values, 6.5 TB/s (209 us with three FP64 DFMA per
  * value, which bound it).  With PT = 2 the pulses of a group share the reads
  * of K (batches whose pulses share the radial tables), and the integer units
  * bind: 8 pulses 1.23 ms (one pulse at a time 1.44, four 1.39; three FP64 DFMA
@@ -2040,8 +2040,8 @@ __global__ void __launch_bounds__(NW * 32) k_precond_tma(PcT Q, int mode, const 
  * per 32 rows of a factor and of the vector, 31.8 us, rows were off by up to
  * 30 x 2^-53 of their terms for vectors that fall by 24 orders of magnitude.)
  * What bounds it at 16 chunks: the chains' 32 dependent steps, then the
- * triangles' multiply-adds.  41.5 us for 104 block rows of 510 (FP64: 58), 171
- * us for 832 (330), 21.7 us for 40 of 210 (30).
+ * triangles' multiply-adds.  40.1 us for 104 block rows of 510 (FP64: 58), 163
+ * us for 832 (330), 21.1 us for 40 of 210 (30).
  * An infinity or NaN in a block row or its factors makes its whole result NaN.
  */
 #define PF_BW 16                       /* band padding it is written for (the B-spline bases' half-width is 15) */
@@ -4218,7 +4218,7 @@ static int asm_build(gade_solver *s)
         }
     if ((rc = asm_partitions(s))) return rc;
     /* costs: 2 multiply-adds per stored value of the pairs' nonzero slots
-       (fixed point on the integer units) plus the diagonal blocks (complex,
+       (on the integer units) plus the diagonal blocks (complex,
        4 FP64 FMAs); the values stream once per apply */
     s->asm_flops = 2.0 * (2.0 * (double)s->npairs * s->blk_nnz + 4.0 * (double)s->nblk * s->blk_nnz);
     s->asm_bytes = 8.0 * (double)per + 2.0 * rows + 16.0 * (double)s->nk * WB + 4.0 * s->npairs + 48.0 * (double)s->n;
@@ -4355,7 +4355,7 @@ static int launch_precond(gade_solver *s, int mode, const double2 *in0, const do
                           double2 *out, cudaStream_t st, int pred = PRED_NONE)
 {
     /* 8 warps: on the integer units where the factors have that form (see
-       solver_create): 41.5 us a solve at N = 53,040 and 171 us for 8 pulses,
+       solver_create): 40.1 us a solve at N = 53,040 and 163 us for 8 pulses,
        where k_precond_tma's 8 FP64 warps take 58 and 330 */
     if (s->pc_nw == 8 && s->d_XL) {
         PcT Q = pc_params(s, s->d_XL, s->d_XU, pred);

@@ -1,30 +1,40 @@
 /*
- * gade_fx.cuh - fixed-point products of FP64 values on the integer units
- * (device helpers shared by the operator and the projection kernels).
+ * gade_fx.cuh - sums of products of FP64 values on the integer units (device
+ * helpers shared by the operator, the block solves and the projection).
  */
 #ifndef GADE_FX_CUH
 #define GADE_FX_CUH
 
 /*
- * GB300 retires 2 DFMA per clock and SM but 32 32x32+64-bit integer
- * multiply-adds (measured: 1.6 against 24 per nominal clock), so the long
- * real x real sums of the assembled operator run there.  A vector of FP64
- * values that share a power of two is held as integers N, value = N 2^e:
- *   matrix values     |N| <= 2^57, one e per row or run        (FX_UPA = 4)
- *   vector entries    |N| <= 2^58, one e per staged window     (FX_UPX = 5)
- * each in two signed limbs, N = hi 2^29 + lo, |lo| <= 2^28.  A product is
- * hi hi 2^58 + (hi lo + lo hi) 2^29, three multiply-adds into two 64-bit
- * sums (the lo lo term, below 2^-56 of the largest product, is left out);
- * sums of up to 32 products stay below 2^63 and are exact.  A 53-bit
- * mantissa is held in full down to 2^-4 (2^-5 for vector entries) of its
- * group's largest value and rounded to nearest below that, at 2^-58 (2^-59)
- * of the group's power of two, so a row's sum carries an error of about 2^-57
- * of its largest terms once, where FP64 rounds every product and partial sum
- * to 2^-53 of them.
+ * GB300 retires 2 DFMA per clock and SM but some 27 32x32+64-bit integer
+ * multiply-adds (measured: 1.6 against 24-27 per nominal clock), so long sums
+ * of products run there.
+ *
+ * A matrix value is a word (int2, x the low half): N in its upper 57 bits
+ * (2^55 <= |N| <= 2^56: 53 bits and 3 more) and an offset in its lower 7,
+ * value = N 2^(e - 1078 - offset) with e the exponent of the value's group;
+ * zero is N = 0 with offset 127.  A value below 2^-127 of its group's power of
+ * two loses bits, any other keeps FP64's.  (Factors and basis entries use the
+ * 7 bits for an exponent of their own.)  A vector entry is X 2^(ex - 1080),
+ * |X| <= 2^58, with ex the biased exponent of the larger part of the complex
+ * entry.
+ *
+ * A sum of up to 33 complex or 30 real products aligns its words to its
+ * largest product first, C = max (ex - offset): each N is shifted into place
+ * and multiplied in limbs of 30 bits, 2 N 2^-s = h 2^30 + l with l in
+ * [0, 2^30) and X = h 2^30 + l with |l| <= 2^29, three multiply-adds per
+ * product into two 64-bit sums (l l is left out: below 2^-54 of the largest
+ * product).  The shifts leave 2^-57 of that product, so a sum's error is a few
+ * 2^-54 of its largest product, whichever of its entries is the largest;
+ * FP64 rounds every product and partial sum to 2^-53 of its own.  (With one
+ * exponent per row of values and per window of entries the shift and the
+ * offsets are not needed, and a row whose own products are far below the
+ * largest value times the largest entry loses its digits.)
  */
-#define FX_UPA 4
-#define FX_UPX 5
-#define FX_LB 29                       /* bits of the low limb */
+#define FX_UPX 5                       /* bits of X below a 53-bit value */
+#define FX_OFF 127
+#define FX_ZERO (-100000)              /* exponent of a zero factor: never the largest */
+#define FX_WB 30                       /* bits of the low limb */
 
 /* biased exponent field of a double given by its high word */
 __host__ __device__ __forceinline__ int fx_exp(unsigned hi) { return (int)((hi >> 20) & 0x7FF); }
@@ -46,14 +56,6 @@ __device__ __forceinline__ long long fx_from(double v, int em, int up)
     m = fx_shift(m << up, em - ev);
     return (long long)b < 0 ? -(long long)m : (long long)m;
 }
-/* two signed limbs of N */
-__device__ __forceinline__ int2 fx_split(long long N)
-{
-    int2 r;
-    r.x = (int)((N + (1ll << (FX_LB - 1))) >> FX_LB);
-    r.y = (int)(N - ((long long)r.x << FX_LB));
-    return r;
-}
 __device__ __forceinline__ double pow2d(int e) { return __hiloint2double((e + 1023) << 20, 0); }   /* -1022 <= e <= 1023 */
 #define FX_NAN 20000                   /* exponents from here on make a sum NaN */
 /* acc += V 2^e; e of any size (below the normal range in two factors) */
@@ -63,36 +65,13 @@ __device__ __forceinline__ double fx_add(double acc, long long V, int e)
     if (e < -1022) { v *= pow2d(e + 900 < -1022 ? -1022 : e + 900); e = -900; }
     return fma(v, e >= FX_NAN ? __longlong_as_double(0x7FF8000000000000ll) : pow2d(e > 1023 ? 1023 : e), acc);
 }
-/* the upper 16 bits of a double >= v (v >= 0): sign, exponent and 4 mantissa bits, rounded up */
-__device__ __forceinline__ unsigned short fx_bound16(double v)
-{
-    const unsigned long long b = (unsigned long long)__double_as_longlong(v);
-    return (unsigned short)((b + 0xFFFFFFFFFFFFull) >> 48);
-}
-/* the same from the bits of |v|: an infinity or a NaN gives 0x7FF0 */
+/* the upper 16 bits of a double >= |v|, given the bits of |v|: exponent and 4
+   mantissa bits, rounded up; an infinity or a NaN gives 0x7FF0 */
 __device__ __forceinline__ unsigned short fx_bound16_bits(unsigned long long b)
 {
     return b >= 0x7FF0000000000000ull ? (unsigned short)0x7FF0 : (unsigned short)((b + 0xFFFFFFFFFFFFull) >> 48);
 }
 __device__ __forceinline__ double fx_bound_to(unsigned short u) { return __hiloint2double((int)u << 16, 0); }
-
-/*
- * Values with an exponent of their own.  A word (int2, x the low half) holds
- * N in its upper 57 bits (2^55 <= |N| <= 2^56: 53 bits and 3 more) and in its
- * lower 7 an offset, value = N 2^(e - 1078 - offset) with e the exponent of
- * the value's group; zero is N = 0 with offset 127.  A value below 2^-127 of
- * its group's power of two loses bits, any other keeps FP64's.  A factor of
- * the words is X 2^(ex - 1080), |X| <= 2^58 (the larger part of a complex
- * value has ex for its biased exponent).  A sum of up to 15 products aligns
- * its words to its largest product first, C = max (ex - offset); the shifts
- * leave 2^-57 of that product, so the sum is as accurate as FP64's (5 times
- * more, measured on rows with one large product and on rows of equal ones)
- * whichever of its entries is the largest.  Limbs of 30 bits: N / 2^-1 2^-s
- * as h 2^30 + l, l in [0, 2^30), and X as h 2^30 + l, |l| <= 2^29.
- */
-#define FX_OFF 127
-#define FX_ZERO (-100000)              /* exponent of a zero factor: never the largest */
-#define FX_WB 30                       /* bits of the low limb */
 
 __device__ __forceinline__ int2 fx_word_of(long long T, int off)
 {
