@@ -277,9 +277,9 @@ int gade_solver_residual_precision(const gade_solver *s, int32_t *mode, int32_t 
 int gade_solver_set_wait_limit(gade_solver *s, uint32_t polls);
 /* Warps per block row of the complex128 block-LU solves (replacing the
  * cuSPARSE triangular solves of tools/gpu_sparse.c:235-263): 8 (the
- * default: products on the integer units where the blocks' half-bandwidth is
- * at most 16, see gade_solver_flops; FP64 with the triangle products of a
- * chunk pair split over two warps otherwise) or 4 (FP64).  The results differ
+ * default: products on the integer units, see gade_solver_flops, in FP64
+ * solvers whose blocks' half-bandwidth is at most 16; FP64 with the triangle
+ * products of a chunk pair split over two warps otherwise) or 4 (FP64).  The results differ
  * by rounding.
  * The complex64 solves of the mixed-precision inner iterations always use
  * 4.  Takes effect at the next step. */
